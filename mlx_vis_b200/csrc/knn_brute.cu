@@ -8,9 +8,9 @@
 //            distance (|x~_i|^2 is constant along the row).  The three extra K
 //            columns live in padding the 64-wide K blocks carry anyway.
 // 2. topk:   persistent tcgen05 kernel.  The n x n score matrix is cut into
-//            tiles of 256 points (MMA N) by 256 query rows (L <= 32: a CTA pair
-//            on one TPC, cluster of 2, tcgen05.mma.cta_group::2 with M = 256) or
-//            by 128 rows (L > 32, or pairing switched off: one CTA, M = 128);
+//            tiles of 256 points (MMA N) by 256 query rows (a CTA pair on one TPC,
+//            cluster of 2, tcgen05.mma.cta_group::2 with M = 256) or by 128 rows
+//            (pairing switched off: one CTA, M = 128);
 //            unit u (pair or CTA) owns the contiguous tile range
 //            [u*T/G, (u+1)*T/G) in (row block, column tile) order.  In every CTA
 //            warp 0 streams k-blocks with TMA (128-byte swizzle, zero fill past
@@ -46,37 +46,49 @@ constexpr int BN = 256;  // points per tile = MMA N
 constexpr int BK = 64;   // BF16 elements per 128-byte swizzled row
 constexpr int UK = 16;   // K of one tcgen05.mma kind::f16
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int THREADS = 256;  // warp 0 TMA, warp 1 MMA, warp 2 TMEM owner, warps 4-7 epilogue
+// warp 0 TMA, warp 1 MMA, warp 2 TMEM owner, warp 3 release relay, warps 4-7 epilogue,
+// then four warps per further list of 32
+constexpr int THREADS = 256;
 
-constexpr int STG_PITCH = 36;  // floats per staging row (32 scores + padding)
-
-// LCAP == 32: each thread keeps its row's best 32 (score, column) pairs sorted in
-// registers and appends hits (score below its 32nd best) to a private buffer in
-// shared memory; batches of 16 are merged by data-independent sorting networks,
-// so the 32 rows of a warp merge in lockstep without divergence.
-// LCAP > 32: per-thread sorted lists in shared memory with insertion.
+// Selection of the L best of a row, L <= 32 NL: the row's list is cut into NL sorted
+// lists of 32 (score, column) pairs, each in the registers of one thread.  The epilogue
+// thread of the row (the leader, list 0) appends hits (scores below the row's L-th best)
+// to a private buffer in shared memory and merges it in batches of 16 by
+// data-independent sorting networks, so the 32 rows of a warp merge in lockstep without
+// divergence.  The 16 pairs that a merge pushes out of a list go through a shared-memory
+// mailbox to the follower thread that holds the next 32, which merges them while the
+// leader scans on; the last list yields the admission threshold.
+// What bounds it: the epilogue warps' instruction latency, one warp per scheduler, for
+// small d; the MMAs and their operands from L2 for d in the hundreds.  Sorted registers
+// cost about 3 instructions per hit against 15 for reducing unsorted lists by
+// bisection.  B200, tile kernel: 9999 x 50, k = 30 (two lists) 7842 -> 186 us (one
+// thread inserting into a list in shared memory before); 20000 x 784, k = 100 (four
+// lists) 58.6 -> 1.4 ms; 20000 x 784, k = 15 (one list, appends without a branch) 549 ->
+// 497 us.
 // PAIR: the CTA holds 128 of the tile's 256 points (its half of the pair's B).
-template <int LCAP, bool PAIR>
+template <int NL, bool PAIR>
 struct Cfg {
-  static_assert(!PAIR || LCAP == 32, "CTA pairs run the batched top-32 epilogue only");
-  static constexpr bool kWarpSelect = LCAP == 32;
+  static_assert(NL >= 1 && NL <= 4, "lists of 32, at most 128 candidates");
+  static constexpr int kThreads = THREADS + 128 * (NL - 1);
   static constexpr int kBBytes = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int kStageBytes = A_BYTES + kBBytes;
   static constexpr int kRowsPerBlock = PAIR ? 2 * BM : BM;
-  static constexpr int kStages = PAIR ? 5 : (LCAP <= 64 ? 3 : 2);
-  // batched selection: merge once some row of the warp holds kMergeAt hits; a
-  // 32-column group then adds at most 32 to the kMergeAt - 1 already pending
-  static constexpr int kMergeAt = PAIR ? 12 : 16;
+  static constexpr int kStages = PAIR ? (NL == 1 ? 5 : NL == 4 ? 3 : 4) : (NL == 1 ? 3 : 2);
+  // merge once some row of the warp holds kMergeAt hits; a 32-column group then adds at
+  // most 32 to the kMergeAt - 1 already pending
+  static constexpr int kMergeAt = 16;
   static constexpr int kBuf = kMergeAt + 32;
-  static constexpr int kListBytes = kWarpSelect ? BM * kBuf * 8 + BM * STG_PITCH * 4 : BM * LCAP * 8;
-  static constexpr int kBarBytes = 256;
+  static constexpr int kMailBytes = BM * 16 * 8;  // one mailbox per link: 16 pairs for each row
+  static constexpr int kListBytes = BM * kBuf * 8 + (NL - 1) * kMailBytes + BM * 4;  // ... and the thresholds
+  static constexpr int kBarBytes = 512;
   static constexpr int kSmem = 1024 + kStages * kStageBytes + kListBytes + kBarBytes;
+  static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
 };
 
 struct Plan {
   int64_t n, d, ld;
   int64_t m, r0;  // query rows [r0, r0 + m) against all n rows (m = n, r0 = 0: every row)
-  int k, L, lcap, num_kb, slots;
+  int k, L, lists, num_kb, slots;  // lists: 32-entry lists per row
   bool pair;     // 256-row tiles on CTA pairs (cta_group::2)
   int rb_rows;   // query rows per row block: 256 (pair) or 128
   int64_t row_blocks, col_tiles, tiles, cols_pad;
@@ -108,7 +120,7 @@ static bool pairing_enabled() {
 }
 
 static int make_plan(int64_t n, int64_t d, int k, int extra, void* ws, Plan& p, int64_t r0 = 0,
-                     int64_t m = -1) {
+                     int64_t m = -1, bool pair_ok = true) {
   if (m < 0) m = n;
   if (n < 2) return set_error(UMAPB_ERR_ARG, "knn_brute: need n >= 2 (got %lld)", (long long)n);
   if (r0 < 0 || m < 1 || r0 + m > n)
@@ -133,14 +145,14 @@ static int make_plan(int64_t n, int64_t d, int k, int extra, void* ws, Plan& p, 
     p.status = p.xp.status;
     return s;
   }
-  p.lcap = p.L <= 32 ? 32 : (p.L <= 64 ? 64 : 128);
+  p.lists = (p.L + 31) / 32;
   // features + three norm columns, padded to whole 64-element K blocks so every
   // 128-byte TMA box row starts on a 128-byte boundary
   p.ld = (d + 3 + BK - 1) / BK * BK;
   p.num_kb = (int)ceil_div(p.ld, BK);
   int64_t g = 0;
   p.pair = false;
-  if (p.lcap == 32 && pairing_enabled()) {
+  if (pair_ok && pairing_enabled()) {
     g = resident_pairs();
     p.pair = g > 0;
   }
@@ -233,20 +245,23 @@ __device__ __forceinline__ void sort16(float (&v)[16], int (&x)[16]) {
   }
 }
 
-// list (32, ascending) := smallest 32 of list U batch (16, ascending), ascending.
+// ascending order of 16 pairs that form a bitonic sequence
+__device__ __forceinline__ void clean16(float (&v)[16], int (&x)[16]) {
+#pragma unroll
+  for (int stride = 8; stride > 0; stride >>= 1) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if ((i & stride) == 0) cex(v[i], x[i], v[i + stride], x[i + stride], true);
+  }
+}
+
+// list (32, ascending) := smallest 32 of list U batch (16, ascending), ascending; the
+// batch becomes the 16 largest, a bitonic sequence.
 // [list, +inf x16, reversed batch] is bitonic; its half-cleaner keeps the 32
 // smallest in the lower half, which a bitonic merge then sorts.
-__device__ __forceinline__ void merge_32_16(float (&lv)[32], int (&li)[32], const float (&bv)[16],
-                                            const int (&bx)[16]) {
+__device__ __forceinline__ void merge_32_16(float (&lv)[32], int (&li)[32], float (&bv)[16], int (&bx)[16]) {
 #pragma unroll
-  for (int i = 16; i < 32; ++i) {
-    const float b = bv[31 - i];
-    const int ib = bx[31 - i];
-    if (b < lv[i]) {
-      lv[i] = b;
-      li[i] = ib;
-    }
-  }
+  for (int i = 16; i < 32; ++i) cex(lv[i], li[i], bv[31 - i], bx[31 - i], true);
 #pragma unroll
   for (int stride = 16; stride > 0; stride >>= 1) {
 #pragma unroll
@@ -256,30 +271,76 @@ __device__ __forceinline__ void merge_32_16(float (&lv)[32], int (&li)[32], cons
   }
 }
 
+__device__ __forceinline__ void reset_list(float (&lv)[32], int (&li)[32]) {
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    lv[e] = INFINITY;
+    li[e] = -1;
+  }
+}
+
+// the list's entries [0, m) to the candidate arrays
+__device__ __forceinline__ void store_list(const float (&lv)[32], const int (&li)[32], int m, float* cs, int32_t* ci) {
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    if (e < m) {
+      cs[e] = lv[e];
+      ci[e] = li[e];
+    }
+  }
+}
+
+// entry p of the list (p a run-time value below 32)
+__device__ __forceinline__ float list_at(const float (&lv)[32], int p) {
+  float x = lv[31];
+#pragma unroll
+  for (int e = 0; e < 31; ++e) x = e == p ? lv[e] : x;
+  return x;
+}
+
+// (score, column) pairs in shared memory, 8 bytes each
+__device__ __forceinline__ void lds_pair(uint32_t at, float& s, int& x) {
+  uint32_t u;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(u), "=r"(x) : "r"(at) : "memory");
+  s = __uint_as_float(u);
+}
+__device__ __forceinline__ void sts_pair(uint32_t at, float s, int x) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(s)), "r"(x) : "memory");
+}
+
+enum MailCmd : int { kMailMerge = 0, kMailFlush = 1, kMailExit = 2 };
 
 // ---- 2. tcgen05 distance tiles + fused per-row top-L ------------------------
-template <int LCAP, bool PAIR>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int NL, bool PAIR>
+__global__ void __launch_bounds__(Cfg<NL, PAIR>::kThreads, 1)
     topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 int n, int num_kb, int64_t col_tiles, int64_t tiles, int slots,
                 int L, float* __restrict__ cand_s, int32_t* __restrict__ cand_i, int32_t* __restrict__ status,
                 int m_rows, int r0) {
-  using C = Cfg<LCAP, PAIR>;
+  using C = Cfg<NL, PAIR>;
   constexpr int STAGE_BYTES = C::kStageBytes;
   constexpr int RB = C::kRowsPerBlock;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stages = smem;
-  float* list_s = reinterpret_cast<float*>(smem + C::kStages * STAGE_BYTES);  // [LCAP][BM]
-  int32_t* list_i = reinterpret_cast<int32_t*>(list_s + LCAP * BM);           // [LCAP][BM]
+  // pending hits [kBuf][BM] and mailboxes [NL - 1][16][BM], (score, column) pairs; the
+  // rows' thresholds [BM]
+  float* list_s = reinterpret_cast<float*>(smem + C::kStages * STAGE_BYTES);
+  float* mail_s = list_s + 2 * C::kBuf * BM;
+  volatile float* tau_s = mail_s + (NL - 1) * (C::kMailBytes / 4);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * STAGE_BYTES + C::kListBytes);
   uint64_t* full = bars;
   uint64_t* empty = bars + C::kStages;
   uint64_t* tfull = bars + 2 * C::kStages;
   uint64_t* tempty = tfull + 2;
   uint64_t* relay = tempty + 2;  // pair, rank 1: its epilogue's releases, forwarded to rank 0
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(relay + 2);
+  uint64_t* mfull = relay + 2;              // [NL - 1][4]: mailbox of link l, lane quarter q, is full ...
+  uint64_t* mempty = mfull + 4 * (NL - 1);  // ... has been read
+  uint64_t* flushed = mempty + 4 * (NL - 1);  // [4]: the last list of the quarter is reset
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(flushed + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* mail_cmd = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [NL - 1][4]
+  static_assert((2 * 5 + 2 + 2 + 2 + 8 * 3 + 4) * 8 + (2 + 4 * 3) * 4 <= C::kBarBytes, "barrier area");
 
   if constexpr (PAIR) {
     uint32_t nrank;
@@ -310,9 +371,17 @@ __global__ void __launch_bounds__(THREADS, 1)
       tc::mbar_init(&tempty[a], PAIR ? 129 : 128);
       tc::mbar_init(&relay[a], 128);
     }
+    if constexpr (NL > 1) {
+      for (int l = 0; l < 4 * (NL - 1); ++l) {
+        tc::mbar_init(&mfull[l], 32);
+        tc::mbar_init(&mempty[l], 32);
+      }
+      for (int l = 0; l < 4; ++l) tc::mbar_init(&flushed[l], 32);
+    }
     *abort_flag = 0;
     tc::fence_mbar_init();
   }
+  if (NL > 1 && threadIdx.x < BM) tau_s[threadIdx.x] = INFINITY;
   if (warp == 0 && lane == 0) {
     tc::prefetch_tmap(&tmA);
     tc::prefetch_tmap(&tmB);
@@ -325,13 +394,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == 2) tc::tmem_alloc_pair(tmem_slot, 512);
   } else {
     if (warp == 2) tc::tmem_alloc(tmem_slot, 512);
-  }
-  if (!C::kWarpSelect && warp >= 4) {
-    const int r = threadIdx.x - 128;
-    for (int e = 0; e < LCAP; ++e) {
-      list_s[e * BM + r] = INFINITY;
-      list_i[e * BM + r] = -1;
-    }
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -456,75 +518,79 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (acc == 0) acc_phase ^= 1;
       }
     }
-  } else if (C::kWarpSelect && warp >= 4) {
-    // ---------------- epilogue: batched per-row top-32 (L <= 32) ----------------
+  } else if (warp >= 4 && warp < 8) {
+    // ---------------- epilogue: batched per-row top-L ----------------
     // Thread r of the four epilogue warps owns TMEM lane r, i.e. query row
-    // rb*128 + r.  It keeps the row's best 32 (score, column) pairs sorted in
-    // registers (lv/li; lv[31] is the admission threshold) and appends every hit
-    // to its own kBuf-entry buffer in shared memory (two stores, no loop).  When a
-    // thread of the warp holds kMergeAt hits the whole warp merges its buffers in
-    // batches of 16 with a bitonic sort network and a bitonic 32+16 merge —
-    // data-independent, so the 32 rows of a warp run in lockstep.
+    // rb*RB + r (+ 128 in rank 1), and its list 0.  Every hit is appended to its own
+    // kBuf-entry buffer in shared memory by predicated stores (no branch).  When a
+    // thread of the warp holds kMergeAt hits the whole warp merges in batches of 16.
     const int q = warp & 3;
     const int r = q * 32 + lane;
-    constexpr int BUF = C::kBuf;
-    float* bs = list_s;                                          // [BUF][BM]
-    int32_t* bi = reinterpret_cast<int32_t*>(list_s + BUF * BM);  // [BUF][BM]
-    // per-thread staging row for the chunk being appended; a pitch of 36 floats
-    // keeps each quarter-warp's 16-byte stores on distinct banks
-    float* stg_row = list_s + 2 * BUF * BM + r * STG_PITCH;
+    const uint32_t my_at = tc::smem_u32(list_s) + 8u * (uint32_t)r;  // [kBuf][BM] (score, column)
     float lv[32];
     int li[32];
-#pragma unroll
-    for (int e = 0; e < 32; ++e) {
-      lv[e] = INFINITY;
-      li[e] = 0x7fffffff;
-    }
+    reset_list(lv, li);
+    float tau = INFINITY;  // NL == 1: the row's L-th best score
     int cnt = 0;
     int acc = 0;
     uint32_t acc_phase = 0;
+    uint32_t sent = 0, flushes = 0;  // messages to the first follower, flushes among them
     int64_t cur_rb = -1;
     bool ok = true;
-    auto merge_pending = [&]() {
-      while (__any_sync(0xffffffffu, cnt > 0)) {
-        const int m = cnt < 16 ? cnt : 16;
-        const int base = cnt - m;
-        float bv[16];
-        int bx[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          if (e < m) {
-            bv[e] = bs[(base + e) * BM + r];
-            bx[e] = bi[(base + e) * BM + r];
-          } else {
-            bv[e] = INFINITY;
-            bx[e] = 0x7fffffff;
-          }
+    // hands the 16 pairs pushed out of list 0 (or a command) to the next list
+    auto send = [&](const float (&bv)[16], const int (&bx)[16], int cmd) {
+      if constexpr (NL > 1) {
+        if (!tc::mbar_wait(&mempty[q], (sent & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          return;
         }
-        cnt = base;
-        sort16(bv, bx);
-        merge_32_16(lv, li, bv, bx);
+        if (cmd == kMailMerge) {
+          const uint32_t at = tc::smem_u32(mail_s) + 8u * (uint32_t)r;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) sts_pair(at + (uint32_t)(e * BM * 8), bv[e], bx[e]);
+        }
+        if (lane == 0) mail_cmd[q] = cmd;
+        tc::mbar_arrive(&mfull[q]);
+        ++sent;
       }
     };
-    auto flush = [&](int64_t rb) {
-      merge_pending();
-      const int64_t row = rb * RB + (int64_t)rank * BM + r;
-      const int64_t slot = cta - first_cta(rb * col_tiles, tiles, G);
-      if (row < m_rows) {
-        float* cs = cand_s + (row * slots + slot) * L;
-        int32_t* ci = cand_i + (row * slots + slot) * L;
+    auto merge_batch = [&]() {
+      const int m = cnt < 16 ? cnt : 16;
+      const int base = cnt - m;
+      float bv[16];
+      int bx[16];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          if (e < L) {
-            cs[e] = lv[e];
-            ci[e] = li[e] == 0x7fffffff ? -1 : li[e];
-          }
+      for (int e = 0; e < 16; ++e) {
+        if (e < m) {
+          lds_pair(my_at + (uint32_t)((base + e) * BM * 8), bv[e], bx[e]);
+        } else {
+          bv[e] = INFINITY;
+          bx[e] = -1;
         }
       }
-#pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        lv[e] = INFINITY;
-        li[e] = 0x7fffffff;
+      cnt = base;
+      sort16(bv, bx);
+      merge_32_16(lv, li, bv, bx);
+      if constexpr (NL == 1)
+        tau = list_at(lv, L - 1);
+      else
+        send(bv, bx, kMailMerge);
+    };
+    auto flush = [&](int64_t rb) {
+      while (ok && __any_sync(0xffffffffu, cnt > 0)) merge_batch();
+      const int64_t row = rb * RB + (int64_t)rank * BM + r;
+      const int64_t slot = cta - first_cta(rb * col_tiles, tiles, G);
+      const int64_t e0 = (row * slots + slot) * L;
+      if (row < m_rows) store_list(lv, li, L < 32 ? L : 32, cand_s + e0, cand_i + e0);
+      reset_list(lv, li);
+      tau = INFINITY;
+      if constexpr (NL > 1) {
+        float bv[16];
+        int bx[16];
+        if (ok) send(bv, bx, kMailFlush);
+        // the followers have written their lists and the threshold is infinite again
+        if (ok && !tc::mbar_wait(&flushed[q], flushes & 1u, abort_flag)) ok = false;
+        ++flushes;
       }
     };
     for (int64_t t = t_begin; t < t_end; ++t) {
@@ -535,7 +601,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (cur_rb >= 0) flush(cur_rb);
         cur_rb = rb;
       }
-      if (!tc::mbar_wait(&tfull[acc], acc_phase, abort_flag)) {
+      if (!ok || !tc::mbar_wait(&tfull[acc], acc_phase, abort_flag)) {
         ok = false;
         break;
       }
@@ -545,14 +611,15 @@ __global__ void __launch_bounds__(THREADS, 1)
       const int self_col = row_ok ? (int)(row + r0) : -1;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
       // Admission cap of the first tile of a row block, where the empty list
-      // would admit every column: per 32-column group the 4th smallest valid
-      // score, maximised over the groups.  At least 4 x 8 = 32 valid scores are
-      // <= that value, so the row's 32 best of the tile all are, and admitting
+      // would admit every column: per 32-column group the 4 NL-th smallest valid
+      // score, maximised over the groups.  At least 4 NL x 8 = 32 NL >= L valid scores
+      // are <= that value, so the row's L best of the tile all are, and admitting
       // scores <= cap alone keeps the list exact while cutting the first tile's
-      // hits from 256 to about the best fifth.  A group with fewer than 4 valid
-      // columns leaves the cap infinite.
+      // hits from 256.  A group with fewer than 4 NL valid columns leaves the cap
+      // infinite.
       float cap = INFINITY;
       if (fresh) {
+        constexpr int D = 4 * NL;
         float hi = -INFINITY;
 #pragma unroll 1
         for (int ch = 0; ch < BN / 32; ++ch) {
@@ -560,56 +627,67 @@ __global__ void __launch_bounds__(THREADS, 1)
           __syncwarp();
           tc::tmem_ld32(taddr + ch * 32, v);
           const int col0 = ct * BN + ch * 32;
-          float a0 = INFINITY, a1 = INFINITY, a2 = INFINITY, a3 = INFINITY;  // 4 smallest, sorted
+          float a[D];  // the D smallest, sorted
+#pragma unroll
+          for (int d = 0; d < D; ++d) a[d] = INFINITY;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int col = col0 + j;
             const float x = (col != self_col && col < n) ? v[j] : INFINITY;
-            a3 = fminf(a3, fmaxf(a2, x));
-            a2 = fminf(a2, fmaxf(a1, x));
-            a1 = fminf(a1, fmaxf(a0, x));
-            a0 = fminf(a0, x);
+#pragma unroll
+            for (int d = D - 1; d > 0; --d) a[d] = fminf(a[d], fmaxf(a[d - 1], x));
+            a[0] = fminf(a[0], x);
           }
-          hi = fmaxf(hi, a3);
+          hi = fmaxf(hi, a[D - 1]);
         }
         // v <= hi  <=>  v < next float above hi (hi finite); infinite hi admits all
         cap = hi < INFINITY ? nextafterf(hi, INFINITY) : INFINITY;
       }
+      // columns per step: 16 at 512 threads (128 registers; 672 against 726 us at 20000 x 50,
+      // k = 50); at 640 threads (96 registers) 16 spill as 32 do and cost more steps
+      constexpr int CW = NL == 3 ? 16 : 32;
+      constexpr unsigned kAll = 0xffffffffu >> (32 - CW);
 #pragma unroll 1
-      for (int ch = 0; ch < BN / 32; ++ch) {
-        float v[32];
+      for (int ch = 0; ch < BN / CW; ++ch) {
+        float v[CW];
         __syncwarp();
-        tc::tmem_ld32(taddr + ch * 32, v);
-        const int col0 = ct * BN + ch * 32;
-        // branch-free hit mask of the 32 columns (four independent OR chains);
-        // rows past n never admit
-        const float tau = row_ok ? fminf(lv[31], cap) : -INFINITY;
-        unsigned m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+        if constexpr (CW == 32)
+          tc::tmem_ld32(taddr + ch * CW, v);
+        else
+          tc::tmem_ld16(taddr + ch * CW, v);
+        const int col0 = ct * BN + ch * CW;
+        // rows past the last one never admit
+        const float lim_s = row_ok ? fminf(NL == 1 ? tau : tau_s[r], cap) : -INFINITY;
+        const int self_off = self_col - col0, lim = n - col0;  // the row itself, zero-filled columns past n
+        unsigned valid = kAll;
+        if ((unsigned)self_off < (unsigned)CW) valid &= ~(1u << self_off);
+        if (lim < CW) valid &= lim <= 0 ? 0u : ((1u << lim) - 1u);
+        if (__any_sync(0xffffffffu, valid != kAll)) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          m0 |= (v[j] < tau ? 1u : 0u) << j;
-          m1 |= (v[j + 8] < tau ? 1u : 0u) << j;
-          m2 |= (v[j + 16] < tau ? 1u : 0u) << j;
-          m3 |= (v[j + 24] < tau ? 1u : 0u) << j;
+          for (int j = 0; j < CW; ++j) v[j] = (valid >> j) & 1u ? v[j] : INFINITY;  // never below the threshold
         }
-        unsigned mask = m0 | (m1 << 8) | (m2 << 16) | (m3 << 24);
-        const int self_off = self_col - col0;  // the row itself
-        if ((unsigned)self_off < 32u) mask &= ~(1u << self_off);
-        const int lim = n - col0;  // zero-filled columns past n
-        if (lim < 32) mask &= lim <= 0 ? 0u : ((1u << lim) - 1u);
-        if (mask) {  // stage the chunk, then append the hits in column order
-          float4* st4 = reinterpret_cast<float4*>(stg_row);
+        // a column's slot is computed before any store: a register that a store still
+        // reads cannot be advanced, and waiting for that took 25 cycles a column
+        uint32_t at = my_at + (uint32_t)(cnt * BM * 8);
+        uint32_t slot[CW];
 #pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) st4[j4] = make_float4(v[4 * j4], v[4 * j4 + 1], v[4 * j4 + 2], v[4 * j4 + 3]);
-          while (mask) {
-            const int j = __ffs(mask) - 1;
-            mask &= mask - 1u;
-            bs[cnt * BM + r] = stg_row[j];
-            bi[cnt * BM + r] = col0 + j;
-            ++cnt;
-          }
+        for (int j = 0; j < CW; ++j) {
+          slot[j] = at;
+          at += v[j] < lim_s ? (uint32_t)(BM * 8) : 0u;
         }
-        if (__any_sync(0xffffffffu, cnt >= C::kMergeAt)) merge_pending();
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          asm volatile(
+              "{\n\t.reg .pred p;\n\t"
+              "setp.lt.f32 p, %1, %2;\n\t"
+              "@p st.shared.v2.b32 [%0], {%3, %4};\n\t}"
+              ::"r"(slot[j]), "f"(v[j]), "f"(lim_s), "r"(__float_as_uint(v[j])), "r"(col0 + j)
+              : "memory");
+        cnt = (int)(at - my_at) / (BM * 8);
+        if (__any_sync(0xffffffffu, cnt >= C::kMergeAt)) {
+          do merge_batch();
+          while (ok && __any_sync(0xffffffffu, cnt >= C::kMergeAt));
+        }
       }
       tc::tc_fence_before();
       // CTA-scope arrivals only: a cluster-scope release costs each epilogue
@@ -619,79 +697,67 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (acc == 0) acc_phase ^= 1;
     }
     if (ok && cur_rb >= 0) flush(cur_rb);
-  } else if (!C::kWarpSelect && warp >= 4) {
-    // ---------------- epilogue: per-row top-L ----------------
-    const int q = warp & 3;  // TMEM lane quarter of this warp
-    const int r = q * 32 + lane;
-    float tau = INFINITY;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    int64_t cur_rb = -1;
-    bool ok = true;
-    auto flush = [&](int64_t rb) {
-      const int64_t row = rb * BM + r;
-      const int64_t slot = cta - first_cta(rb * col_tiles, tiles, G);
-      if (row < m_rows) {
-        float* cs = cand_s + (row * slots + slot) * L;
-        int32_t* ci = cand_i + (row * slots + slot) * L;
-        for (int e = 0; e < L; ++e) {
-          cs[e] = list_s[e * BM + r];
-          ci[e] = list_i[e * BM + r];
-        }
-      }
-      for (int e = 0; e < LCAP; ++e) {
-        list_s[e * BM + r] = INFINITY;
-        list_i[e * BM + r] = -1;
-      }
-    };
-    for (int64_t t = t_begin; t < t_end; ++t) {
-      const int64_t rb = t / col_tiles;
-      const int ct = (int)(t % col_tiles);
-      if (rb != cur_rb) {
-        if (cur_rb >= 0) flush(cur_rb);
-        cur_rb = rb;
-        tau = INFINITY;
-      }
-      if (!tc::mbar_wait(&tfull[acc], acc_phase, abort_flag)) {
-        ok = false;
-        break;
-      }
-      tc::tc_fence_after();
-      const int64_t row = rb * BM + r;
-      const bool row_ok = row < m_rows;
-      const int self_col = (int)(row + r0);
-      const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-#pragma unroll 1
-      for (int ch = 0; ch < BN / 32; ++ch) {
-        float v[32];
-        __syncwarp();
-        tc::tmem_ld32(taddr + ch * 32, v);
-        const int col0 = ct * BN + ch * 32;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float s = v[j];
-          const int col = col0 + j;
-          if (s < tau && row_ok && col != self_col && col < n) {
-            int p = L - 1;
-            while (p > 0) {
-              const float prev = list_s[(p - 1) * BM + r];
-              if (prev <= s) break;
-              list_s[p * BM + r] = prev;
-              list_i[p * BM + r] = list_i[(p - 1) * BM + r];
-              --p;
-            }
-            list_s[p * BM + r] = s;
-            list_i[p * BM + r] = col;
-            tau = list_s[(L - 1) * BM + r];
-          }
-        }
-      }
-      tc::tc_fence_before();
-      tc::mbar_arrive(&tempty[acc]);
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1;
+    if constexpr (NL > 1) {
+      float bv[16];
+      int bx[16];
+      if (ok) send(bv, bx, kMailExit);
     }
-    if (ok && cur_rb >= 0) flush(cur_rb);
+  } else if (NL > 1 && warp >= 8) {
+    // ---------------- follower: list f of the rows of one lane quarter ----------------
+    // Takes batches of 16 pairs from list f - 1, keeps the 32 best of what it has seen
+    // and passes the rest on; the last one publishes the rows' L-th best score.
+    const int q = warp & 3;
+    const int f = (warp >> 2) - 1;  // 1 .. NL - 1
+    const int r = q * 32 + lane;
+    const bool last = f == NL - 1;
+    const int in = 4 * (f - 1) + q, out = 4 * f + q;
+    const uint32_t is = tc::smem_u32(mail_s) + (uint32_t)((f - 1) * C::kMailBytes) + 8u * (uint32_t)r;
+    const uint32_t os = is + (uint32_t)C::kMailBytes;  // not used by the last one
+    const int m = L - 32 * f < 32 ? L - 32 * f : 32;  // entries of this list that count (>= 1)
+    float lv[32];
+    int li[32];
+    reset_list(lv, li);
+    uint32_t got = 0;
+    int64_t rb = t_begin / col_tiles;  // flushes come once per row block, in order
+    while (true) {
+      if (!tc::mbar_wait(&mfull[in], got & 1u, abort_flag)) break;
+      const int cmd = mail_cmd[in];
+      float bv[16];
+      int bx[16];
+      if (cmd == kMailMerge) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) lds_pair(is + (uint32_t)(e * BM * 8), bv[e], bx[e]);
+      }
+      ++got;
+      __syncwarp();
+      tc::mbar_arrive(&mempty[in]);
+      if (cmd == kMailMerge) {
+        clean16(bv, bx);
+        merge_32_16(lv, li, bv, bx);
+        if (last) tau_s[r] = list_at(lv, m - 1);
+      } else if (cmd == kMailFlush) {
+        const int64_t row = rb * RB + (int64_t)rank * BM + r;
+        const int64_t slot = cta - first_cta(rb * col_tiles, tiles, G);
+        const int64_t e0 = (row * slots + slot) * L + 32 * f;
+        if (row < m_rows) store_list(lv, li, m, cand_s + e0, cand_i + e0);
+        reset_list(lv, li);
+        ++rb;
+        if (last) {
+          tau_s[r] = INFINITY;
+          tc::mbar_arrive(&flushed[q]);
+        }
+      }
+      if (!last) {
+        if (!tc::mbar_wait(&mempty[out], (got & 1u), abort_flag)) break;
+        if (cmd == kMailMerge) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) sts_pair(os + (uint32_t)(e * BM * 8), bv[e], bx[e]);
+        }
+        if (lane == 0) mail_cmd[out] = cmd;
+        tc::mbar_arrive(&mfull[out]);
+      }
+      if (cmd == kMailExit) break;
+    }
   }
 
   tc::tc_fence_before();
@@ -832,15 +898,15 @@ __global__ void __launch_bounds__(RR_WARPS * 32)
   }
 }
 
-template <int LCAP, bool PAIR>
+template <int NL, bool PAIR>
 static int set_smem_attr() {
-  using C = Cfg<LCAP, PAIR>;
+  using C = Cfg<NL, PAIR>;
   static bool attr_set[64] = {false};
   int dev = 0;
   UMAPB_CUDA_TRY(cudaGetDevice(&dev), "knn_brute: cudaGetDevice");
   if (dev < 0 || dev >= 64) return set_error(UMAPB_ERR_UNSUPPORTED, "knn_brute: device index %d", dev);
   if (!attr_set[dev]) {
-    UMAPB_CUDA_TRY(cudaFuncSetAttribute(topk_kernel<LCAP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    UMAPB_CUDA_TRY(cudaFuncSetAttribute(topk_kernel<NL, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         C::kSmem),
                    "knn_brute: set smem attribute");
     attr_set[dev] = true;
@@ -877,7 +943,7 @@ static int64_t resident_pairs() {
   std::lock_guard<std::mutex> lock(mu);
   if (!known[dev]) {
     int64_t pairs = 0;
-    if (set_smem_attr<32, true>() == UMAPB_OK) {
+    if (set_smem_attr<1, true>() == UMAPB_OK) {  // every list count runs one CTA per SM
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -886,11 +952,11 @@ static int64_t resident_pairs() {
       attr[0].val.clusterDim.z = 1;
       cfg.gridDim = dim3(2 * (unsigned)num_sms(), 1, 1);
       cfg.blockDim = dim3(THREADS, 1, 1);
-      cfg.dynamicSmemBytes = Cfg<32, true>::kSmem;
+      cfg.dynamicSmemBytes = Cfg<1, true>::kSmem;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, topk_kernel<32, true>, &cfg) == cudaSuccess) pairs = clusters;
+      if (cudaOccupancyMaxActiveClusters(&clusters, topk_kernel<1, true>, &cfg) == cudaSuccess) pairs = clusters;
     }
     cudaGetLastError();  // a refused query only disables pairing
     clear_error();
@@ -900,20 +966,17 @@ static int64_t resident_pairs() {
   return cached[dev];
 }
 
-template <int LCAP>
+template <int NL>
 static int launch_topk(const Plan& p, const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t stream) {
-  int s = set_smem_attr<LCAP, false>();
+  int s = p.pair ? set_smem_attr<NL, true>() : set_smem_attr<NL, false>();
   if (s) return s;
-  topk_kernel<LCAP, false><<<(unsigned)p.grid, THREADS, Cfg<LCAP, false>::kSmem, stream>>>(
-      ta, tb, (int)p.n, p.num_kb, p.col_tiles, p.tiles, p.slots, p.L, p.cand_s, p.cand_i, p.status, (int)p.m,
-      (int)p.r0);
-  UMAPB_LAUNCH_CHECK("knn_brute: topk kernel launch");
-  return UMAPB_OK;
-}
-
-static int launch_topk_pair(const Plan& p, const CUtensorMap& ta, const CUtensorMap& tb, cudaStream_t stream) {
-  int s = set_smem_attr<32, true>();
-  if (s) return s;
+  if (!p.pair) {
+    topk_kernel<NL, false><<<(unsigned)p.grid, Cfg<NL, false>::kThreads, Cfg<NL, false>::kSmem, stream>>>(
+        ta, tb, (int)p.n, p.num_kb, p.col_tiles, p.tiles, p.slots, p.L, p.cand_s, p.cand_i, p.status, (int)p.m,
+        (int)p.r0);
+    UMAPB_LAUNCH_CHECK("knn_brute: topk kernel launch");
+    return UMAPB_OK;
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -921,12 +984,12 @@ static int launch_topk_pair(const Plan& p, const CUtensorMap& ta, const CUtensor
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(2 * (unsigned)p.grid, 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg<32, true>::kSmem;
+  cfg.blockDim = dim3(Cfg<NL, true>::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg<NL, true>::kSmem;
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  UMAPB_CUDA_TRY(cudaLaunchKernelEx(&cfg, topk_kernel<32, true>, ta, tb, (int)p.n, p.num_kb, p.col_tiles, p.tiles,
+  UMAPB_CUDA_TRY(cudaLaunchKernelEx(&cfg, topk_kernel<NL, true>, ta, tb, (int)p.n, p.num_kb, p.col_tiles, p.tiles,
                                     p.slots, p.L, p.cand_s, p.cand_i, p.status, (int)p.m, (int)p.r0),
                  "knn_brute: pair topk kernel launch");
   return UMAPB_OK;
@@ -941,10 +1004,12 @@ static int run_tiles(const Plan& p, cudaStream_t stream) {
     return s;
   if ((s = make_tmap_bf16_2d(&tb, p.xb, (uint64_t)p.n, (uint64_t)p.ld, (uint64_t)p.ld, p.pair ? BN / 2 : BN, BK)))
     return s;
-  if (p.pair) return launch_topk_pair(p, ta, tb, stream);
-  if (p.lcap == 32) return launch_topk<32>(p, ta, tb, stream);
-  if (p.lcap == 64) return launch_topk<64>(p, ta, tb, stream);
-  return launch_topk<128>(p, ta, tb, stream);
+  switch (p.lists) {
+    case 1: return launch_topk<1>(p, ta, tb, stream);
+    case 2: return launch_topk<2>(p, ta, tb, stream);
+    case 3: return launch_topk<3>(p, ta, tb, stream);
+    default: return launch_topk<4>(p, ta, tb, stream);
+  }
 }
 
 static int next_pow2(int v) {
@@ -1124,6 +1189,12 @@ extern "C" int umapb_knn_brute_noalloc(const float* X, int64_t n, int64_t d, int
   knn::Plan p;
   int s = knn::make_plan(n, d, k, extra, nullptr, p);
   if (s) return s;
+  // a few shapes need one slot per row more on CTA pairs than on single CTAs
+  bool pair_ok = true;
+  if (p.ws_bytes > (size_t)UMAPB_NOALLOC_SCRATCH_BYTES && !p.exact && p.pair) {
+    pair_ok = false;
+    if ((s = knn::make_plan(n, d, k, extra, nullptr, p, 0, -1, pair_ok))) return s;
+  }
   if (p.ws_bytes > (size_t)UMAPB_NOALLOC_SCRATCH_BYTES)
     return set_error(UMAPB_ERR_UNSUPPORTED,
                      "knn_brute_noalloc: n=%lld, d=%lld, k+extra=%d needs %zu bytes of scratch but the static array "
@@ -1131,7 +1202,7 @@ extern "C" int umapb_knn_brute_noalloc(const float* X, int64_t n, int64_t d, int
                      (long long)n, (long long)d, p.L, p.ws_bytes, (size_t)UMAPB_NOALLOC_SCRATCH_BYTES);
   void* scratch = nullptr;
   if ((s = scratch_address(&scratch))) return s;
-  knn::make_plan(n, d, k, extra, scratch, p);
+  knn::make_plan(n, d, k, extra, scratch, p, 0, -1, pair_ok);
   if (p.exact) {
     if ((s = knnx::run(X, p.xp, squared, out_idx, out_dist, stream))) return s;
     if (device_status)

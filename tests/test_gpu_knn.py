@@ -86,6 +86,20 @@ def test_brute_candidate_list_sizes(k, extra):
     assert_exact_knn(X, idx, dist, k)
 
 
+@pytest.mark.parametrize("pair", ["1", "0"])
+@pytest.mark.parametrize("n,k", [(260, 17), (513, 48), (1030, 49), (700, 80), (300, 81), (1500, 112), (100, 99)])
+def test_brute_list_edges(n, k, pair, monkeypatch):
+    """Candidate lists of 33, 64, 65, 96, 97, 128 and n - 1 entries: the first and last
+    size of every number of 32-entry lists, on CTA pairs and on single CTAs, rows and
+    columns past a tile's edge, duplicates and rows sorted by cluster."""
+    monkeypatch.setenv("UMAPB_KNN_PAIR", pair)
+    rng = np.random.default_rng(n + k)
+    X = (np.repeat(rng.normal(size=(5, 20)) * 3, -(-n // 5), axis=0)[:n] + rng.normal(size=(n, 20))).astype(np.float32)
+    X[-20:] = X[:20]
+    idx, d2 = run_knn(X, k, squared=True)
+    assert_exact_knn(X, idx, d2, k, squared=True)
+
+
 def test_brute_squared_and_duplicates():
     rng = np.random.default_rng(5)
     X = rng.normal(size=(400, 16)).astype(np.float32)
