@@ -182,7 +182,8 @@ static int make_plan(int64_t n, int64_t d, int k, int extra, void* ws, Plan& p, 
 
 // ---- 1. prep: augmented BF16 operands (one warp per row) ---------------------
 __global__ void prep_kernel(const float* __restrict__ X, int64_t n, int d, int ld, __nv_bfloat16* __restrict__ xa,
-                            __nv_bfloat16* __restrict__ xb) {
+                            __nv_bfloat16* __restrict__ xb, int32_t* __restrict__ status) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;  // the call's status word, before the tile kernel
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= n) return;
@@ -777,124 +778,226 @@ __global__ void __launch_bounds__(Cfg<NL, PAIR>::kThreads, 1)
 }
 
 // ---- 3. merge slots + exact FP32 rerank -------------------------------------
-__device__ __forceinline__ bool key_less(float a, int ia, float b, int ib) {
-  return a < b || (a == b && (unsigned)ia < (unsigned)ib);
+__device__ __forceinline__ uint32_t score_key(float s) {  // unsigned order = float order
+  const uint32_t u = __float_as_uint(s);
+  return u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u);
 }
-
-// Warp-cooperative bitonic sort of P (power of two) (key, idx) pairs in shared memory.
-__device__ void warp_bitonic(float* key, int* idx, int P, int lane) {
-  for (int size = 2; size <= P; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = lane; i < (P >> 1); i += 32) {
-        const int lo = 2 * i - (i & (stride - 1));
-        const int hi = lo + stride;
-        const bool asc = (lo & size) == 0;
-        const float ka = key[lo], kb = key[hi];
-        const int ia = idx[lo], ib = idx[hi];
-        const bool swap = asc ? key_less(kb, ib, ka, ia) : key_less(ka, ia, kb, ib);
-        if (swap) {
-          key[lo] = kb;
-          key[hi] = ka;
-          idx[lo] = ib;
-          idx[hi] = ia;
-        }
-      }
-      __syncwarp();
-    }
-  }
+__device__ __forceinline__ float key_score(uint32_t k) {
+  return __uint_as_float(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xffffffffu));
 }
 
 constexpr int RR_WARPS = 8;
+constexpr int RR_U = 4;  // candidates a lane group has in flight
 
+// One warp per row.  Merging the row's slots is a selection, not a sort: the L-th
+// smallest score by bisection (halving the score range, about a dozen steps; the ordered
+// bits finish ties), then the exact distances, then each candidate's place by
+// counting the smaller ones.  G lanes share one candidate's distance (32 / G * RR_U of
+// them in flight), so that short rows keep every lane loading and reduce in log2(G)
+// shuffles.  The summation order is the same for every G and VEC: 32 partial sums,
+// partial c over the 16-byte words (VEC 4) or the elements (VEC 2, 1) whose number is c
+// mod 32, added as a butterfly 16, 8, 4, 2, 1 -- in a lane's registers as far as the
+// lane holds both sides.  Bound by the gather of the candidates' rows from L2 for long rows
+// (20000 x 784, k = 15: 1.9 GB in 0.20 ms), by the latency of one row's chain for short
+// ones: 2000 x 64, k = 15 (8 slots) 40 -> 17 us, 9999 x 50, k = 30 133 -> 50 us against
+// sorting all slots in shared memory (and a launch fewer: only lists that were
+// written are read, so nothing is cleared first).
+template <int VEC, int G>
 __global__ void __launch_bounds__(RR_WARPS * 32)
     rerank_kernel(const float* __restrict__ X, int64_t n, int d, const float* __restrict__ cand_s,
-                  const int32_t* __restrict__ cand_i, int slots, int L, int P, int PL, int k, int squared,
-                  int32_t* __restrict__ out_idx, float* __restrict__ out_dist, int64_t r0 = 0) {
+                  const int32_t* __restrict__ cand_i, int slots, int rb_rows, int64_t col_tiles, int64_t tiles,
+                  int64_t units, int cols, int L, int k, int squared, int32_t* __restrict__ out_idx,
+                  float* __restrict__ out_dist, int64_t r0) {
   extern __shared__ uint8_t smem_raw[];
+  constexpr unsigned kAll = 0xffffffffu;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  float* key = reinterpret_cast<float*>(smem_raw) + (size_t)warp * 2 * P;
-  int* idx = reinterpret_cast<int*>(key + P);
+  const unsigned below = (1u << lane) - 1u;
+  const int cap = slots * L;
+  uint32_t* key = reinterpret_cast<uint32_t*>(smem_raw) + (size_t)warp * 2 * cap;
+  int32_t* idx = reinterpret_cast<int32_t*>(key + cap);
   const int64_t row = (int64_t)blockIdx.x * RR_WARPS + warp;
   if (row >= n) return;
-  const int m = slots * L;
-  for (int e = lane; e < P; e += 32) {
-    float s = INFINITY;
-    int j = 0x7fffffff;
-    if (e < m) {
-      const int c = cand_i[row * m + e];
-      if (c >= 0) {
-        s = cand_s[row * m + e];
-        j = c;
-      }
-    }
-    key[e] = s;
+  // the units that worked on this row block wrote one list each (entries outside the
+  // columns are empty ones, or what a tile kernel that gave up left unwritten)
+  const int64_t t0b = (row / rb_rows) * col_tiles;
+  const int m = (int)(first_cta(t0b + col_tiles - 1, tiles, units) - first_cta(t0b, tiles, units) + 1) * L;
+  int valid = 0;
+  uint32_t lo = kAll, hi = 0u;
+  for (int e = lane; e < m; e += 32) {
+    int j = cand_i[row * cap + e];
+    j = (unsigned)j < (unsigned)cols ? j : -1;
+    const float s = cand_s[row * cap + e];
+    const uint32_t x = j >= 0 ? score_key(s) : kAll;
+    key[e] = x;
     idx[e] = j;
+    if (j >= 0) {
+      ++valid;
+      lo = min(lo, x);
+      hi = max(hi, x);
+    }
   }
   __syncwarp();
-  warp_bitonic(key, idx, P, lane);
-  // exact squared distances of the best L candidates (direct form, FP32), four
-  // candidates per pass so every lane keeps several independent loads in flight
-  const float* xr = X + (r0 + row) * d;  // rows: the query range [r0, r0 + n)
-  const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  for (int e0 = 0; e0 < PL; e0 += 4) {
-    int j[4];
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 4; ++u) j[u] = (e0 + u < L) ? idx[e0 + u] : 0x7fffffff;
-    if (vec) {
-      const float4* xr4 = reinterpret_cast<const float4*>(xr);
-      for (int c = lane; c < (d >> 2); c += 32) {
-        const float4 a = __ldg(xr4 + c);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (j[u] != 0x7fffffff) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(X + (int64_t)j[u] * d) + c);
-            const float t0 = a.x - b.x, t1 = a.y - b.y, t2 = a.z - b.z, t3 = a.w - b.w;
-            acc[u] = fmaf(t0, t0, acc[u]);
-            acc[u] = fmaf(t1, t1, acc[u]);
-            acc[u] = fmaf(t2, t2, acc[u]);
-            acc[u] = fmaf(t3, t3, acc[u]);
-          }
+  valid = __reduce_add_sync(kAll, valid);
+  int c = valid < L ? valid : L;  // candidates to rerank
+  if (valid != c || valid < m) {   // compact the c best to the front
+    lo = __reduce_min_sync(kAll, lo);
+    hi = __reduce_max_sync(kAll, hi);
+    int ties = m;  // keys equal to hi that survive
+    if (valid > L) {
+      bool found = false;
+      for (int step = 0; !found && lo < hi; ++step) {
+        uint32_t mid = lo + (hi - lo) / 2;
+        if (step < 16) {
+          const uint32_t h = score_key(0.5f * key_score(lo) + 0.5f * key_score(hi));
+          mid = h >= lo && h < hi ? h : mid;
+        }
+        int cnt = 0;
+        for (int e = lane; e < m; e += 32) cnt += key[e] <= mid ? 1 : 0;
+        cnt = __reduce_add_sync(kAll, cnt);
+        if (cnt >= L) {
+          hi = mid;
+          found = cnt == L;
+        } else {
+          lo = mid + 1u;
         }
       }
-    } else {
-      for (int c = lane; c < d; c += 32) {
-        const float a = __ldg(xr + c);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (j[u] != 0x7fffffff) {
-            const float t = a - __ldg(X + (int64_t)j[u] * d + c);
-            acc[u] = fmaf(t, t, acc[u]);
-          }
-        }
+      if (!found) {
+        int less = 0;
+        for (int e = lane; e < m; e += 32) less += key[e] < hi ? 1 : 0;
+        ties = L - __reduce_add_sync(kAll, less);
       }
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+    int base = 0, tied = 0;
+    for (int e0 = 0; e0 < m; e0 += 32) {  // in place: an entry only moves towards the front
+      const int e = e0 + lane;
+      const uint32_t x = e < m ? key[e] : kAll;
+      const int j = e < m ? idx[e] : -1;
+      const bool tie = j >= 0 && x == hi;
+      const unsigned tb = __ballot_sync(kAll, tie);
+      const bool keep = j >= 0 && (x < hi || (tie && tied + __popc(tb & below) < ties));
+      tied += __popc(tb);
+      const unsigned kb = __ballot_sync(kAll, keep);
+      if (keep) idx[base + __popc(kb & below)] = j;
+      base += __popc(kb);
+      __syncwarp();
     }
-    __syncwarp();
-    if (lane < 4 && e0 + lane < PL) {
-      float a = acc[0];
-      int jj = j[0];
-#pragma unroll
-      for (int u = 1; u < 4; ++u)
-        if (lane == u) {
-          a = acc[u];
-          jj = j[u];
-        }
-      key[e0 + lane] = jj != 0x7fffffff ? a : INFINITY;
-      idx[e0 + lane] = jj;
-    }
-    __syncwarp();
   }
-  warp_bitonic(key, idx, PL, lane);
-  for (int e = lane; e < k; e += 32) {
-    const float v = key[e];
-    out_idx[row * k + e] = idx[e];
-    out_dist[row * k + e] = squared ? v : sqrtf(v);
+
+  // exact squared distances of the candidates (direct form, FP32)
+  const float* xr = X + (r0 + row) * d;  // rows: the query range [r0, r0 + n)
+  constexpr int C = 32 / G;
+  constexpr int B = VEC == 2 ? 2 : 1;   // partial sums per loaded word
+  constexpr int R = 32 / (G * B);       // words of a lane that belong to different partial sums
+  static_assert(R >= 1, "float2 words take at most 16 lanes");
+  const int slot = lane / G, t0 = lane & (G - 1);
+  const int V = d / VEC;
+  for (int e0 = 0; e0 < c; e0 += C * RR_U) {
+    const float* xc[RR_U];
+    float acc[RR_U][R][B];
+#pragma unroll
+    for (int u = 0; u < RR_U; ++u) {
+      const int e = e0 + u * C + slot;
+      xc[u] = X + (int64_t)idx[e < c ? e : c - 1] * d;  // past the end: the last one again
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int v = 0; v < B; ++v) acc[u][r][v] = 0.f;
+    }
+    for (int tb = t0; tb < V; tb += G * R) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int t = tb + G * r;
+        if (t >= V) continue;
+        float a[VEC], b[RR_U][VEC];
+        if constexpr (VEC == 4) {
+          const float4 q = __ldg(reinterpret_cast<const float4*>(xr) + t);
+          a[0] = q.x, a[1] = q.y, a[2] = q.z, a[3] = q.w;
+#pragma unroll
+          for (int u = 0; u < RR_U; ++u) {
+            const float4 y = __ldg(reinterpret_cast<const float4*>(xc[u]) + t);
+            b[u][0] = y.x, b[u][1] = y.y, b[u][2] = y.z, b[u][3] = y.w;
+          }
+        } else if constexpr (VEC == 2) {
+          const float2 q = __ldg(reinterpret_cast<const float2*>(xr) + t);
+          a[0] = q.x, a[1] = q.y;
+#pragma unroll
+          for (int u = 0; u < RR_U; ++u) {
+            const float2 y = __ldg(reinterpret_cast<const float2*>(xc[u]) + t);
+            b[u][0] = y.x, b[u][1] = y.y;
+          }
+        } else {
+          a[0] = __ldg(xr + t);
+#pragma unroll
+          for (int u = 0; u < RR_U; ++u) b[u][0] = __ldg(xc[u] + t);
+        }
+#pragma unroll
+        for (int u = 0; u < RR_U; ++u)
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) {
+            const float diff = a[v] - b[u][v];
+            float& s = acc[u][r][VEC == 2 ? v : 0];
+            s = fmaf(diff, diff, s);
+          }
+      }
+    }
+    float sum[RR_U];
+#pragma unroll
+    for (int u = 0; u < RR_U; ++u) {
+      float p[B];
+#pragma unroll
+      for (int v = 0; v < B; ++v) {  // the widest steps of the butterfly, within the lane
+        if constexpr (R == 4)
+          p[v] = (acc[u][0][v] + acc[u][2][v]) + (acc[u][1][v] + acc[u][3][v]);
+        else if constexpr (R == 2)
+          p[v] = acc[u][0][v] + acc[u][1][v];
+        else
+          p[v] = acc[u][0][v];
+#pragma unroll
+        for (int o = G >> 1; o > 0; o >>= 1) p[v] += __shfl_xor_sync(kAll, p[v], o);
+      }
+      sum[u] = B == 2 ? p[0] + p[B - 1] : p[0];
+    }
+#pragma unroll
+    for (int u = 0; u < RR_U; ++u) {
+      const int e = e0 + u * C + slot;
+      if (t0 == 0 && e < c) key[e] = __float_as_uint(sum[u]);  // not negative: the bits order like the value
+    }
+  }
+  __syncwarp();
+
+  // places by (distance, index)
+  constexpr int NE = 4;  // L <= 128
+  uint32_t mk[NE];
+  int32_t mi[NE];
+  int rank[NE];
+#pragma unroll
+  for (int u = 0; u < NE; ++u) {
+    const int e = u * 32 + lane;
+    mk[u] = e < c ? key[e] : kAll;
+    mi[u] = e < c ? idx[e] : 0x7fffffff;
+    rank[u] = 0;
+  }
+  const int chunks = (c + 31) / 32;
+#pragma unroll 4
+  for (int t = 0; t < c; ++t) {
+    const uint32_t kt = key[t];
+    const int32_t it = idx[t];
+#pragma unroll
+    for (int u = 0; u < NE; ++u)
+      if (u < chunks) rank[u] += kt < mk[u] || (kt == mk[u] && it < mi[u]) ? 1 : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < NE; ++u) {
+    if (u * 32 + lane < c && rank[u] < k) {
+      const float v = __uint_as_float(mk[u]);
+      out_idx[row * k + rank[u]] = mi[u];
+      out_dist[row * k + rank[u]] = squared ? v : sqrtf(v);
+    }
+  }
+  for (int e = c + lane; e < k; e += 32) {  // fewer candidates than k: scores that overflowed
+    out_idx[row * k + e] = 0x7fffffff;
+    out_dist[row * k + e] = INFINITY;
   }
 }
 
@@ -914,8 +1017,15 @@ static int set_smem_attr() {
   return UMAPB_OK;
 }
 
-// The rerank kernel's dynamic shared memory (2 P floats per warp) can exceed the
-// 48 KB default; the attribute is raised once per device (up to 200 KB).
+static decltype(&rerank_kernel<4, 8>) const kRerank[8] = {
+    rerank_kernel<4, 8>,  rerank_kernel<4, 16>, rerank_kernel<4, 32>, rerank_kernel<2, 8>,
+    rerank_kernel<2, 16>, rerank_kernel<1, 8>,  rerank_kernel<1, 16>, rerank_kernel<1, 32>};
+
+// Enqueues the rerank of rows [r0, r0 + m).  Its dynamic shared memory (2 slots * L
+// words per warp) can exceed the 48 KB default; the attribute is raised once per device
+// (up to 200 KB).
+static size_t rerank_smem(const Plan& p) { return (size_t)RR_WARPS * 2 * p.slots * p.L * sizeof(float); }
+
 static int rerank_smem_attr(size_t smem) {
   if (smem <= 48 * 1024) return UMAPB_OK;
   if (smem > 200 * 1024)
@@ -927,10 +1037,31 @@ static int rerank_smem_attr(size_t smem) {
   if (dev < 0 || dev >= 64) return set_error(UMAPB_ERR_UNSUPPORTED, "knn_brute: device index %d", dev);
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
-    UMAPB_CUDA_TRY(cudaFuncSetAttribute(rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(200 * 1024)),
-                   "knn_brute: rerank smem attribute");
+    for (int v = 0; v < 8; ++v)
+      UMAPB_CUDA_TRY(cudaFuncSetAttribute((const void*)kRerank[v], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(200 * 1024)),
+                     "knn_brute: rerank smem attribute");
     done[dev] = true;
   }
+  return UMAPB_OK;
+}
+
+static int run_rerank(const Plan& p, const float* X, int squared, int32_t* out_idx, float* out_dist,
+                      cudaStream_t stream) {
+  const size_t smem = rerank_smem(p);
+  const unsigned blocks = (unsigned)ceil_div(p.m, RR_WARPS);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(X);
+  const int vec = (p.d & 3) == 0 && (at & 15) == 0 ? 4 : (p.d & 1) == 0 && (at & 7) == 0 ? 2 : 1;
+  // lanes per candidate: the least that cover a row in a few loads each, so that short
+  // rows have more candidates in flight
+  const int64_t loads = p.d / vec;
+  const int by8 = loads <= 32 ? 0 : 1;
+  const int by32 = by8 ? (loads <= 96 ? 1 : 2) : 0;
+  const auto kernel = kRerank[vec == 4 ? by32 : vec == 2 ? 3 + by8 : 5 + by32];
+  kernel<<<blocks, RR_WARPS * 32, smem, stream>>>(X, p.m, (int)p.d, p.cand_s, p.cand_i, p.slots, p.rb_rows,
+                                                  p.col_tiles, p.tiles, p.grid, (int)p.n, p.L, p.k, squared, out_idx,
+                                                  out_dist, p.r0);
+  UMAPB_LAUNCH_CHECK("knn_brute: rerank kernel launch");
   return UMAPB_OK;
 }
 
@@ -1012,12 +1143,6 @@ static int run_tiles(const Plan& p, cudaStream_t stream) {
   }
 }
 
-static int next_pow2(int v) {
-  int p = 1;
-  while (p < v) p <<= 1;
-  return p;
-}
-
 }  // namespace knn
 }  // namespace umapb
 
@@ -1041,30 +1166,18 @@ static int enqueue_knn(const float* X, int64_t n, int64_t d, int32_t k, int32_t 
     return knnx::run(X, p.xp, squared, out_idx, out_dist, stream);
   }
   int s;
-  const int P = knn::next_pow2(p.slots * p.L);
-  const int PL = knn::next_pow2(p.L);
-  const size_t smem = (size_t)knn::RR_WARPS * 2 * P * sizeof(float);
-  if ((s = knn::rerank_smem_attr(smem))) return s;
-  UMAPB_CUDA_TRY(cudaMemsetAsync(p.status, 0, sizeof(int32_t), stream), "knn_brute: status reset");
-  UMAPB_CUDA_TRY(cudaMemsetAsync(p.cand_i, 0xFF, (size_t)p.m * p.slots * p.L * sizeof(int32_t), stream),
-                 "knn_brute: candidate reset");
+  if ((s = knn::rerank_smem_attr(knn::rerank_smem(p)))) return s;
   if (ev) UMAPB_CUDA_TRY(cudaEventRecord(ev[0], stream), "knn_brute: event");
   {
     const int64_t warps = n;
     const unsigned blocks = (unsigned)ceil_div(warps * 32, 256);
-    knn::prep_kernel<<<blocks, 256, 0, stream>>>(X, n, (int)d, (int)p.ld, p.xa, p.xb);
+    knn::prep_kernel<<<blocks, 256, 0, stream>>>(X, n, (int)d, (int)p.ld, p.xa, p.xb, p.status);
     UMAPB_LAUNCH_CHECK("knn_brute: prep kernel launch");
   }
   if (ev) UMAPB_CUDA_TRY(cudaEventRecord(ev[1], stream), "knn_brute: event");
   if ((s = knn::run_tiles(p, stream))) return s;
   if (ev) UMAPB_CUDA_TRY(cudaEventRecord(ev[2], stream), "knn_brute: event");
-  {
-    const unsigned blocks = (unsigned)ceil_div(p.m, knn::RR_WARPS);
-    knn::rerank_kernel<<<blocks, knn::RR_WARPS * 32, smem, stream>>>(X, p.m, (int)d, p.cand_s, p.cand_i, p.slots,
-                                                                      p.L, P, PL, k, squared, out_idx, out_dist,
-                                                                      p.r0);
-    UMAPB_LAUNCH_CHECK("knn_brute: rerank kernel launch");
-  }
+  if ((s = knn::run_rerank(p, X, squared, out_idx, out_dist, stream))) return s;
   if (ev) UMAPB_CUDA_TRY(cudaEventRecord(ev[3], stream), "knn_brute: event");
   count_launches(3);
   return UMAPB_OK;
@@ -1151,7 +1264,7 @@ extern "C" int umapb_knn_brute_timed(const float* X, int64_t n, int64_t d, int32
 // device's address of the array with cudaGetSymbolAddress (with the device
 // current); make that first call before any stream capture begins.  All calls
 // share the one array and it keeps the previous call's contents, so the parts
-// that must start at zero (the status word and the candidate lists) are reset
+// that must start at a known value (the status word) are reset
 // by each call, and calls whose work overlaps on the GPU (for example on two
 // streams at once) race on it: serialise them.
 // ---------------------------------------------------------------------------
@@ -1211,20 +1324,12 @@ extern "C" int umapb_knn_brute_noalloc(const float* X, int64_t n, int64_t d, int
     return UMAPB_OK;
   }
 
-  const int P = knn::next_pow2(p.slots * p.L);
-  const int PL = knn::next_pow2(p.L);
-  const size_t smem = (size_t)knn::RR_WARPS * 2 * P * sizeof(float);
-  if ((s = knn::rerank_smem_attr(smem))) return s;  // before any launch: a refusal leaves nothing enqueued
+  if ((s = knn::rerank_smem_attr(knn::rerank_smem(p)))) return s;  // before any launch: a refusal leaves nothing enqueued
 
-  UMAPB_CUDA_TRY(cudaMemsetAsync(p.status, 0, sizeof(int32_t), stream), "knn_brute_noalloc: status reset");
-  UMAPB_CUDA_TRY(cudaMemsetAsync(p.cand_i, 0xFF, (size_t)n * p.slots * p.L * sizeof(int32_t), stream),
-                 "knn_brute_noalloc: candidate reset");
-  knn::prep_kernel<<<(unsigned)ceil_div(n * 32, 256), 256, 0, stream>>>(X, n, (int)d, (int)p.ld, p.xa, p.xb);
+  knn::prep_kernel<<<(unsigned)ceil_div(n * 32, 256), 256, 0, stream>>>(X, n, (int)d, (int)p.ld, p.xa, p.xb, p.status);
   UMAPB_LAUNCH_CHECK("knn_brute_noalloc: prep kernel launch");
   if ((s = knn::run_tiles(p, stream))) return s;
-  knn::rerank_kernel<<<(unsigned)ceil_div(n, knn::RR_WARPS), knn::RR_WARPS * 32, smem, stream>>>(
-      X, n, (int)d, p.cand_s, p.cand_i, p.slots, p.L, P, PL, k, squared, out_idx, out_dist);
-  UMAPB_LAUNCH_CHECK("knn_brute_noalloc: rerank kernel launch");
+  if ((s = knn::run_rerank(p, X, squared, out_idx, out_dist, stream))) return s;
   if (device_status)
     UMAPB_CUDA_TRY(cudaMemcpyAsync(device_status, p.status, sizeof(int32_t), cudaMemcpyDeviceToDevice, stream),
                    "knn_brute_noalloc: status copy");

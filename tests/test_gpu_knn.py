@@ -100,6 +100,26 @@ def test_brute_list_edges(n, k, pair, monkeypatch):
     assert_exact_knn(X, idx, d2, k, squared=True)
 
 
+@pytest.mark.parametrize("d", [33, 36, 50, 62, 66, 130, 132, 194, 390])
+def test_brute_rerank_loads_and_alignment(d):
+    """The rerank's load widths and lanes per candidate: row lengths that are multiples of
+    four, two and one on either side of each change of lane count, and the same rows at
+    addresses that are 16-, 8- and 4-byte aligned only."""
+    from mlx_vis_b200 import _lib
+
+    rng = np.random.default_rng(d)
+    X = rng.normal(size=(500, d)).astype(np.float32)
+    idx, dist = run_knn(X, 15)
+    assert_exact_knn(X, idx, dist, 15)
+    buf = torch.empty(500 * d + 4, device="cuda")
+    for off in (1, 2):
+        view = buf[off:off + 500 * d].view(500, d)
+        view.copy_(torch.from_numpy(X))
+        i2, d2 = _lib.knn_brute(view, 15)
+        assert np.array_equal(i2.cpu().numpy(), idx)
+        np.testing.assert_allclose(d2.cpu().numpy(), dist, rtol=1e-6)  # FP32 sums of d terms in another order
+
+
 def test_brute_squared_and_duplicates():
     rng = np.random.default_rng(5)
     X = rng.normal(size=(400, 16)).astype(np.float32)
