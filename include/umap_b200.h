@@ -217,6 +217,22 @@ int umapb_nnd_iteration(const void* Xd, const float* sqd, int32_t dd, int32_t ld
                         int32_t mc_new, int32_t j_nn, int32_t converging, int32_t recompute_cur, int32_t* idx_new,
                         float* dist_new, uint8_t* flags_new, unsigned long long* changed,
                         unsigned long long* evals, umapb_stream_t stream);
+/* umapb_nnd_select: the row update of a full-path iteration after umapb_nnd_join with
+ * mc == k (every neighbour a source): the k smallest (distance, id) of the current list,
+ * the nn-of-nn candidates (nnbuf) and the reverse candidates, first occurrence of an id
+ * kept.  The reverse candidates are the buckets in the join's workspace (nullptr: none);
+ * d0 holds every row's distance to row 0 in the iteration's space, for the empty
+ * reverse slots (umapb_nnd_dist_row0).  recompute_cur takes the current distances
+ * from curd instead of dist_old.  k <= 32.
+ * umapb_nnd_pad_cols: rows of dd floats copied to rows of pitch ldo, zero padded (the
+ * joins read FP32 rows whose length is a multiple of 4). */
+int umapb_nnd_select(const int32_t* idx_old, const float* dist_old, const int32_t* order, const float* nnbuf,
+                     const float* curd, const float* d0, int64_t n, int32_t k, int32_t j_nn, int32_t recompute_cur,
+                     const void* join_workspace, size_t join_workspace_bytes, int32_t* idx_new, float* dist_new,
+                     uint8_t* flags_new, unsigned long long* changed, umapb_stream_t stream);
+int umapb_nnd_dist_row0(const void* Xd, const float* sqd, int64_t n, int32_t dd, int32_t ldx, int32_t half, float* out,
+                        umapb_stream_t stream);
+int umapb_nnd_pad_cols(const float* X, int64_t n, int32_t dd, int32_t ldo, float* out, umapb_stream_t stream);
 int umapb_nnd_sqrt(const float* d2, int64_t count, float* out, umapb_stream_t stream);
 int umapb_nnd_random_start_workspace(int64_t n, int32_t k, int32_t d, int32_t pd1, int32_t pd2, size_t* bytes);
 int umapb_nnd_random_start(uint32_t* state, int64_t n, int32_t k, int32_t d, int32_t* idx, float* P, int32_t pd1,

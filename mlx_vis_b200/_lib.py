@@ -59,6 +59,9 @@ SIGNATURES = {
     "umapb_nnd_iteration": [_p, _p, _i32, _i32, _i32, _p, _p, _p, _p, _p, _p, _p, _i64, _i32, _i32, _i32, _i32, _i32, _p,
                             _p,
                             _p, _p, _p, _p],
+    "umapb_nnd_select": [_p, _p, _p, _p, _p, _p, _i64, _i32, _i32, _i32, _p, _sz, _p, _p, _p, _p, _p],
+    "umapb_nnd_dist_row0": [_p, _p, _i64, _i32, _i32, _i32, _p, _p],
+    "umapb_nnd_pad_cols": [_p, _i64, _i32, _i32, _p, _p],
     "umapb_kernel_launches": [],
     "umapb_gemm_bf16": [_p, _p, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _i32, _p, _p, _i32, _p, _i32, _p,
                         _i32, _p, _p, _p],

@@ -244,6 +244,16 @@ class NNDescent:
         # candidate distance inside the row kernel instead
         join_on = os.environ.get("UMAPB_NND_JOIN", "1") != "0"
         nnbuf = curd = join_ws = None
+        # FP32 rows for the joins, which read whole float4s: rows of another length are
+        # copied once to zero-padded ones
+        Xi, di = X, d
+        if join_on and k <= JOIN_MAX_K and d % 4 != 0:
+            di = (d + 3) // 4 * 4
+            Xi = torch.empty((n, di), dtype=torch.float32, device=dev)
+            call("umapb_nnd_pad_cols", ptr(X), n, d, di, ptr(Xi), s)
+            if X_low is X:
+                X_low = Xi
+        dist0 = {}  # every row's distance to row 0 by (space, precision), for empty reverse slots
         self.kernel_log_ = []  # (start event, end event, info) per iteration kernel when profile_kernels
 
         t0 = time.time()
@@ -282,16 +292,16 @@ class NNDescent:
                 if use_rev:
                     call("umapb_nnd_reverse", P(idx), n, k, P(rev), P(rev_ws), rev_ws.numel(), s)
                 # the nn-of-nn distances of the NEW-first sources from the blocked join
-                join = join_on and k <= JOIN_MAX_K and mc_conv > 0 and j_nn > 0 and d % 4 == 0
+                join = join_on and k <= JOIN_MAX_K and mc_conv > 0 and j_nn > 0
                 if join and nnbuf is None:
                     nnbuf = torch.empty(n * k * k, dtype=torch.float32, device=dev)
                     curd = torch.empty((n, k), dtype=torch.float32, device=dev)
                     join_ws = _lib.workspace(query("umapb_nnd_join_workspace", n, k, k), dev)
                 ev[0].record() if ev else None
                 if join:
-                    call("umapb_nnd_join_new", P(X), P(sq), d, P(idx), P(flags), P(order), n, k, mc_conv,
+                    call("umapb_nnd_join_new", P(Xi), P(sq), di, P(idx), P(flags), P(order), n, k, mc_conv,
                          j_nn, P(nnbuf), evals_p, P(join_ws), join_ws.numel(), s)
-                call("umapb_nnd_iteration", P(X), P(sq), d, d, 0, P(idx), P(dist), P(flags),
+                call("umapb_nnd_iteration", P(Xi), P(sq), di, di, 0, P(idx), P(dist), P(flags),
                      P(rev if use_rev else None), P(order), P(nnbuf if join else None), P(None), n, k,
                      mc_conv, j_nn, 1, 0, P(idx2), P(dist2), P(flags2), changed_p, evals_p, s)
                 ev[1].record() if ev else None
@@ -303,48 +313,52 @@ class NNDescent:
                 elif it == 1 and X300 is not None:
                     Xd, sqd = X300, sq300
                 else:
-                    Xd, sqd = X, sq
+                    Xd, sqd = Xi, sq
                 use_half = it in (1, 2, 3, 4)
                 recompute = (it == 0) or use_half
-                dd = Xd.shape[1]
+                join = join_on and k <= JOIN_MAX_K and mc_nn > 0
                 if fp32_due:
-                    if not (Xd is X and not use_half and join_on and k <= JOIN_MAX_K and mc_nn == k
-                            and d % 4 == 0):
+                    if not (Xd is Xi and not use_half and join and mc_nn == k):
                         call("umapb_nnd_gather", P(X), P(sq), n, d, P(idx), P(dist), k, 0, s)
                     else:
                         recompute = True  # the join's current-neighbour distances (curd)
                     fp32_due = False
+                dd = Xd.shape[1]
                 ldx = dd
                 if use_half:
-                    ldx = (dd + 7) // 8 * 8  # FP16 rows padded to 16-byte chunks
-                    if Xd is X and Xh is not None:
-                        src = Xh
-                    elif Xd is X300:
+                    if Xd is X300:
                         src = X300h
                     else:
-                        src = torch.empty((n, ldx), dtype=torch.float16, device=dev)
-                        call("umapb_nnd_to_half", P(Xd), n, dd, ldx, P(src), s)
+                        src, dd = Xh, d
+                    ldx = (dd + 7) // 8 * 8  # FP16 rows padded to 16-byte chunks
                 else:
                     src = Xd
-                join = join_on and k <= JOIN_MAX_K and mc_nn > 0 and (use_half or dd % 4 == 0)
                 if join and nnbuf is None:
                     nnbuf = torch.empty(n * k * k, dtype=torch.float32, device=dev)
                     curd = torch.empty((n, k), dtype=torch.float32, device=dev)
                     join_ws = _lib.workspace(query("umapb_nnd_join_workspace", n, k, k), dev)
-                # with every neighbour a source (mc_nn == k) the join's per-source
-                # buckets are the reverse-candidate buckets: it writes rev itself
-                rev_in_join = join and use_rev and mc_nn == k
-                if use_rev and not rev_in_join:
+                # with every neighbour a source (mc_nn == k) the join holds every distance the
+                # row update needs, its per-source buckets the reverse candidates among them
+                select = join and mc_nn == k and j_nn > 0
+                if use_rev and not select:
                     call("umapb_nnd_reverse", P(idx), n, k, P(rev), P(rev_ws), rev_ws.numel(), s)
+                if select and use_rev and (id(Xd), use_half) not in dist0:
+                    d0 = torch.empty(n, dtype=torch.float32, device=dev)
+                    call("umapb_nnd_dist_row0", P(src), P(sqd), n, dd, ldx, int(use_half), P(d0), s)
+                    dist0[id(Xd), use_half] = d0
                 ev[0].record() if ev else None
                 if join:
                     call("umapb_nnd_join", P(src), P(sqd), dd, ldx, int(use_half), P(idx), P(order), n, k,
-                         mc_nn, j_nn, P(nnbuf), P(curd), P(rev if rev_in_join else None), evals_p,
-                         P(join_ws), join_ws.numel(), s)
-                call("umapb_nnd_iteration", P(src), P(sqd), dd, ldx, int(use_half), P(idx), P(dist), P(None),
-                     P(rev if use_rev else None), P(order), P(nnbuf if join else None),
-                     P(curd if join else None), n, k, mc_nn, j_nn, 0, int(recompute), P(idx2),
-                     P(dist2), P(flags2), changed_p, evals_p, s)
+                         mc_nn, j_nn, P(nnbuf), P(curd), P(None), evals_p, P(join_ws), join_ws.numel(), s)
+                if select:
+                    call("umapb_nnd_select", P(idx), P(dist), P(order), P(nnbuf), P(curd),
+                         P(dist0[id(Xd), use_half] if use_rev else None), n, k, j_nn, int(recompute),
+                         P(join_ws if use_rev else None), join_ws.numel(), P(idx2), P(dist2), P(flags2), changed_p, s)
+                else:
+                    call("umapb_nnd_iteration", P(src), P(sqd), dd, ldx, int(use_half), P(idx), P(dist), P(None),
+                         P(rev if use_rev else None), P(order), P(nnbuf if join else None),
+                         P(curd if join else None), n, k, mc_nn, j_nn, 0, int(recompute), P(idx2),
+                         P(dist2), P(flags2), changed_p, evals_p, s)
                 ev[1].record() if ev else None
                 if it == 4:  # FP32 recompute after the last FP16 iteration (nndescent.py:376-378)
                     fp32_due = True

@@ -30,18 +30,15 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "nnd_select.cuh"
+#include "nnd_sort.cuh"
 #include "nnd_wide.cuh"
 #include "scan.cuh"
 
 namespace umapb {
 namespace nnd {
 
-constexpr float kBig = 1e30f;
 constexpr int kWarps = 4;  // warps per block in the row kernels
-
-__device__ __forceinline__ bool key_lt(float a, int ia, float b, int ib) {
-  return a < b || (a == b && ia < ib);
-}
 
 // ---- distance helpers --------------------------------------------------------
 template <class T>
@@ -93,55 +90,6 @@ __device__ __forceinline__ void dot4(const T* __restrict__ X, const T* xs, int d
 __device__ __forceinline__ float d2_from_dot(float sq_i, float sq_c, float dot, bool half_round) {
   if (half_round) dot = __half2float(__float2half_rn(dot));
   return fmaxf(__fsub_rn(__fadd_rn(sq_i, sq_c), __fmul_rn(2.0f, dot)), 0.0f);
-}
-
-// ascending bitonic sort of one (distance, id) key per lane across the warp
-__device__ __forceinline__ void warp_sort_keys(float& d, int& id, int lane) {
-#pragma unroll
-  for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const float od = __shfl_xor_sync(0xffffffffu, d, stride);
-      const int oi = __shfl_xor_sync(0xffffffffu, id, stride);
-      const bool lower = (lane & stride) == 0, asc = (lane & size) == 0;
-      const bool take = (lower == asc) ? key_lt(od, oi, d, id) : key_lt(d, id, od, oi);
-      if (take) {
-        d = od;
-        id = oi;
-      }
-    }
-  }
-}
-
-// ascending order of a bitonic sequence held one key per lane
-__device__ __forceinline__ void warp_bitonic_clean(float& d, int& id, int lane) {
-#pragma unroll
-  for (int stride = 16; stride > 0; stride >>= 1) {
-    const float od = __shfl_xor_sync(0xffffffffu, d, stride);
-    const int oi = __shfl_xor_sync(0xffffffffu, id, stride);
-    const bool take = (lane & stride) == 0 ? key_lt(od, oi, d, id) : key_lt(d, id, od, oi);
-    if (take) {
-      d = od;
-      id = oi;
-    }
-  }
-}
-
-// Inserts (d, id) into the warp-distributed ascending list (lane l holds entry l).
-// Inserts (d, id) into the warp-distributed ascending list (lane l holds entry l).
-__device__ __forceinline__ void list_insert(float& lv, int& li, float d, int id, int k, int lane) {
-  const int pos = __popc(__ballot_sync(0xffffffffu, lane < k && key_lt(lv, li, d, id)));
-  const float up_v = __shfl_up_sync(0xffffffffu, lv, 1);
-  const int up_i = __shfl_up_sync(0xffffffffu, li, 1);
-  if (lane < k) {
-    if (lane > pos) {
-      lv = up_v;
-      li = up_i;
-    } else if (lane == pos) {
-      lv = d;
-      li = id;
-    }
-  }
 }
 
 // ---- small kernels -------------------------------------------------------------
@@ -583,6 +531,7 @@ struct JoinArgs {
   int half_round;
   float* nnbuf;  // (n, mc * j_nn)
   float* curd;   // (n, k), nullable: current-neighbour distances not wanted
+  float* entd;   // the same distances in bucket order (one per entry)
   unsigned long long* evals;  // nullable
 };
 
@@ -590,13 +539,16 @@ __device__ __forceinline__ int join_col_id(const JoinArgs& a, int64_t s, int col
   return col == 0 ? (int)s : a.idx_old[s * a.k + col - 1];
 }
 
-__device__ __forceinline__ void join_store(const JoinArgs& a, int64_t s, int ent, int col, float dot) {
+__device__ __forceinline__ void join_store(const JoinArgs& a, int64_t s, int e, int ent, int col, float dot) {
   const int64_t i = ent >> 5;
   const int p = ent & 31;
   const int cid = join_col_id(a, s, col);
   const float d = d2_from_dot(a.sqd[i], a.sqd[cid], dot, a.half_round != 0);
   if (col == 0) {
-    if (a.curd) a.curd[i * a.k + p] = d;
+    if (a.curd) {
+      a.curd[i * a.k + p] = d;
+      a.entd[e] = d;
+    }
   } else {
     a.nnbuf[i * (int64_t)(a.mc * a.j_nn) + p * a.j_nn + (col - 1)] = d;
   }
@@ -655,7 +607,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) join_f16_kernel(JoinArgs a) {
         for (int u = 0; u < 4; ++u) {
           const int col = cb + (u < 2 ? 2 * c + u : 8 + 2 * c + (u - 2));
           const float dot = u < 2 ? d0[2 * h + u] : d1[2 * h + (u - 2)];
-          if (col < ncol) join_store(a, s, en, col, dot);
+          if (col < ncol) join_store(a, s, e0 + g + 8 * h, en, col, dot);
         }
       }
     }
@@ -787,7 +739,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) join_f32_kernel(JoinArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int col = cb + bt + 4 * j;
-          if (col < ncol) join_store(a, s, en, col, acc[u][j]);
+          if (col < ncol) join_store(a, s, e, en, col, acc[u][j]);
         }
       }
     }
@@ -1014,7 +966,6 @@ __global__ void __launch_bounds__(kWarps * 32, 10) iter_kernel(IterArgs a) {
   // (the first chunk, when the list is empty) is sorted across the warp (bitonic, 15
   // exchange steps) and merged: the 32 smallest of the list and the sorted chunk,
   // paired in reverse, form a bitonic sequence that five exchange steps order.
-  constexpr float kSent = kBig * 4.0f;  // above every real key, including 1e30 entries
   float lv = kSent;
   int li = 0x7fffffff;
   float tau = lv;
@@ -1243,19 +1194,39 @@ extern "C" int umapb_nnd_reverse(const int32_t* idx, int64_t n, int32_t k, int32
   return UMAPB_OK;
 }
 
+// The join's workspace; umapb_nnd_select reads its buckets afterwards.
+namespace {
+struct JoinWs {
+  int32_t *off, *fill, *entries, *choff, *chunk_pos, *srcs;
+  int64_t* total;  // total, then scan scratch at total + 8
+  float* entd;
+  int64_t max_chunks;
+  size_t bytes;
+};
+
+JoinWs join_carve(void* ws, int64_t n, int mc) {
+  const size_t m = (size_t)n * (mc > 0 ? mc : 1);
+  JoinWs w;
+  Carver c(ws);
+  c.take<int32_t>(64);
+  w.off = c.take<int32_t>((size_t)n + 1);   // source counts -> bucket offsets
+  w.fill = c.take<int32_t>((size_t)n + 1);  // fill counters
+  w.entries = c.take<int32_t>(m);
+  w.choff = c.take<int32_t>((size_t)n + 1);  // chunk counts -> chunk offsets
+  w.max_chunks = n + n * mc / 16;            // sum of ceil(count / 16) <= n + n*mc/16
+  w.chunk_pos = c.take<int32_t>((size_t)w.max_chunks + 1);  // chunk -> source
+  w.total = c.take<int64_t>(8 + kScanMaxBlocks);
+  w.srcs = c.take<int32_t>(m);  // the NEW-first source lists (umapb_nnd_join_new)
+  w.entd = c.take<float>(m);    // current-neighbour distances in bucket order
+  w.bytes = c.bytes();
+  return w;
+}
+}  // namespace
+
 extern "C" int umapb_nnd_join_workspace(int64_t n, int32_t k, int32_t mc, size_t* bytes) {
   clear_error();
   UMAPB_REQUIRE(bytes && n >= 1 && k >= 1 && mc >= 0 && mc <= k, "nnd_join_workspace: bad arguments");
-  Carver c(nullptr);
-  c.take<int32_t>(64);
-  c.take<int32_t>((size_t)n + 1);                // source counts -> bucket offsets
-  c.take<int32_t>((size_t)n + 1);                // fill counters
-  c.take<int32_t>((size_t)n * (mc > 0 ? mc : 1));  // entries
-  c.take<int32_t>((size_t)n + 1);                // chunk counts -> chunk offsets
-  c.take<int32_t>((size_t)n + (size_t)n * mc / 16 + 1);  // chunk -> source
-  c.take<int64_t>(8 + kScanMaxBlocks);  // totals, then scan_exclusive's block totals
-  c.take<int32_t>((size_t)n * (mc > 0 ? mc : 1));  // the NEW-first source lists (umapb_nnd_join_new)
-  *bytes = c.bytes();
+  *bytes = join_carve(nullptr, n, mc).bytes;
   return UMAPB_OK;
 }
 
@@ -1278,18 +1249,13 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
   else
     UMAPB_REQUIRE(dd % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(Xd) & 15) == 0,
                   "nnd_join: FP32 rows need dd and the pitch multiples of 4 and a 16-byte aligned base");
-  Carver c(workspace);
-  c.take<int32_t>(64);
-  int32_t* off = c.take<int32_t>((size_t)n + 1);
-  int32_t* fill = c.take<int32_t>((size_t)n + 1);
-  int32_t* entries = c.take<int32_t>((size_t)n * (mc > 0 ? mc : 1));
-  int32_t* choff = c.take<int32_t>((size_t)n + 1);
-  const int64_t max_chunks = n + n * mc / 16;  // sum of ceil(count / 16) <= n + n*mc/16
-  int32_t* chunk_pos = c.take<int32_t>((size_t)max_chunks + 1);
-  int64_t* total = c.take<int64_t>(8 + kScanMaxBlocks);  // total, then scan scratch at total + 8
-  int32_t* srcs = c.take<int32_t>((size_t)n * (mc > 0 ? mc : 1));
-  if (!workspace || workspace_bytes < c.bytes())
-    return set_error(UMAPB_ERR_WORKSPACE, "nnd_join: workspace of %zu bytes, need %zu", workspace_bytes, c.bytes());
+  const JoinWs w = join_carve(workspace, n, mc);
+  if (!workspace || workspace_bytes < w.bytes)
+    return set_error(UMAPB_ERR_WORKSPACE, "nnd_join: workspace of %zu bytes, need %zu", workspace_bytes, w.bytes);
+  int32_t *off = w.off, *fill = w.fill, *entries = w.entries, *choff = w.choff, *chunk_pos = w.chunk_pos;
+  int32_t* srcs = w.srcs;
+  int64_t* total = w.total;
+  const int64_t max_chunks = w.max_chunks;
   if (mc == 0) return UMAPB_OK;
   const int64_t m = n * mc;
   UMAPB_CUDA_TRY(cudaMemsetAsync(off, 0, sizeof(int32_t) * (n + 1), stream), "nnd_join: reset");
@@ -1330,6 +1296,7 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
   a.half_round = half;
   a.nnbuf = nnbuf;
   a.curd = curd;
+  a.entd = w.entd;
   a.evals = evals;
   const unsigned jb = (unsigned)ceil_div(max_chunks, nnd::kWarps);  // warps past the chunk count exit
   if (half) {
@@ -1372,6 +1339,113 @@ extern "C" int umapb_nnd_join_new(const float* X, const float* sq, int32_t dd, c
   UMAPB_REQUIRE(flags_old, "nnd_join_new: null flags");
   return join_impl(X, sq, dd, dd, 0, idx_old, flags_old, order, n, k, mc, j_nn, nnbuf, nullptr, nullptr, evals,
                    workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int umapb_nnd_select(const int32_t* idx_old, const float* dist_old, const int32_t* order,
+                                const float* nnbuf, const float* curd, const float* d0, int64_t n, int32_t k,
+                                int32_t j_nn, int32_t recompute_cur, const void* join_workspace,
+                                size_t join_workspace_bytes, int32_t* idx_new, float* dist_new, uint8_t* flags_new,
+                                unsigned long long* changed, umapb_stream_t stream_) {
+  clear_error();
+  UMAPB_REQUIRE(idx_old && dist_old && nnbuf && idx_new && dist_new && flags_new && changed,
+                "nnd_select: null array argument");
+  UMAPB_REQUIRE(n >= 2 && n < ((int64_t)1 << 26), "nnd_select: need 2 <= n < 2^26");
+  UMAPB_REQUIRE(k >= 1 && k <= 32 && j_nn >= 1 && j_nn <= k, "nnd_select: need 1 <= j_nn <= k <= 32");
+  UMAPB_REQUIRE(!recompute_cur || curd, "nnd_select: recomputed distances need curd");
+  UMAPB_REQUIRE(!join_workspace || d0, "nnd_select: reverse candidates need the distances to row 0");
+  nnd::SelectArgs a = {};
+  a.idx_old = idx_old;
+  a.dist_old = dist_old;
+  a.curd = recompute_cur ? curd : nullptr;
+  a.order = order;
+  a.nnbuf = nnbuf;
+  a.d0 = d0;
+  a.n = n;
+  a.k = k;
+  a.j_nn = j_nn;
+  a.magic = (1u << 20) / (uint32_t)j_nn + 1u;  // exact for columns below 1024 and j_nn <= 32
+  a.idx_new = idx_new;
+  a.dist_new = dist_new;
+  a.flags_new = flags_new;
+  a.changed = changed;
+  if (join_workspace) {  // the buckets of the join with every neighbour a source are the reverse candidates
+    const JoinWs w = join_carve(const_cast<void*>(join_workspace), n, k);
+    if (join_workspace_bytes < w.bytes)
+      return set_error(UMAPB_ERR_WORKSPACE, "nnd_select: join workspace of %zu bytes, need %zu", join_workspace_bytes,
+                       w.bytes);
+    a.off = w.off;
+    a.entries = w.entries;
+    a.entd = w.entd;
+  }
+  return nnd::select_rows(a, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+namespace umapb {
+namespace nnd {
+// out[i] = d(i, 0) of a distance space, one warp per row
+template <class T>
+__global__ void dist_row0_kernel(const T* __restrict__ X, const float* __restrict__ sq, int64_t n, int dd, int ldx,
+                                 int half_round, float* __restrict__ out) {
+  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= n) return;
+  constexpr int V = 16 / sizeof(T);
+  const T* xr = X + row * ldx;
+  float acc = 0.f;
+  if (ldx % V == 0 && dd % V == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+    for (int t = lane; t < dd / V; t += 32) {
+      const uint4 a4 = __ldg(reinterpret_cast<const uint4*>(xr) + t), b4 = __ldg(reinterpret_cast<const uint4*>(X) + t);
+      const T* a = reinterpret_cast<const T*>(&a4);
+      const T* b = reinterpret_cast<const T*>(&b4);
+#pragma unroll
+      for (int e = 0; e < V; ++e) acc = fmaf(to_f<T>(a[e]), to_f<T>(b[e]), acc);
+    }
+  } else {
+    for (int t = lane; t < dd; t += 32) acc = fmaf(to_f<T>(xr[t]), to_f<T>(X[t]), acc);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) out[row] = d2_from_dot(sq[row], sq[0], acc, half_round != 0);
+}
+
+// rows of dd floats copied to rows of pitch ldo >= dd, zero padded
+__global__ void pad_cols_kernel(const float* __restrict__ X, int64_t n, int dd, int ldo, float* __restrict__ out) {
+  const int64_t m = n * ldo;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = t / ldo;
+    const int c = (int)(t - r * ldo);
+    out[t] = c < dd ? X[r * dd + c] : 0.f;
+  }
+}
+}  // namespace nnd
+}  // namespace umapb
+
+extern "C" int umapb_nnd_dist_row0(const void* Xd, const float* sqd, int64_t n, int32_t dd, int32_t ldx, int32_t half,
+                                   float* out, umapb_stream_t stream_) {
+  clear_error();
+  UMAPB_REQUIRE(Xd && sqd && out && n >= 1 && dd >= 1 && ldx >= dd, "nnd_dist_row0: bad arguments");
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  const unsigned blocks = (unsigned)ceil_div(n * 32, 256);
+  if (half)
+    nnd::dist_row0_kernel<__half><<<blocks, 256, 0, stream>>>(static_cast<const __half*>(Xd), sqd, n, dd, ldx, 1, out);
+  else
+    nnd::dist_row0_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(Xd), sqd, n, dd, ldx, 0, out);
+  UMAPB_LAUNCH_CHECK("nnd_dist_row0 kernel");
+  count_launches(1);
+  return UMAPB_OK;
+}
+
+extern "C" int umapb_nnd_pad_cols(const float* X, int64_t n, int32_t dd, int32_t ldo, float* out,
+                                  umapb_stream_t stream_) {
+  clear_error();
+  UMAPB_REQUIRE(X && out && n >= 0 && dd >= 1 && ldo >= dd, "nnd_pad_cols: bad arguments");
+  if (n == 0) return UMAPB_OK;
+  const int64_t want = ceil_div(n * ldo, 256);
+  const unsigned blocks = (unsigned)(want < num_sms() * 16 ? want : num_sms() * 16);
+  nnd::pad_cols_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(X, n, dd, ldo, out);
+  UMAPB_LAUNCH_CHECK("nnd_pad_cols kernel");
+  count_launches(1);
+  return UMAPB_OK;
 }
 
 extern "C" int umapb_nnd_iteration(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, int32_t half,

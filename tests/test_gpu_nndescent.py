@@ -373,3 +373,74 @@ def test_pair_gathers_by_row_block_equal_the_gather(n, d, k, blocks):
     _lib.call("umapb_nnd_sort_rows", _lib.ptr(ib), _lib.ptr(db), n, k, s)
     assert np.array_equal(ia.cpu().numpy(), ib.cpu().numpy())
     assert np.array_equal(da.cpu().numpy().view(np.int32), db.cpu().numpy().view(np.int32))
+
+
+@pytest.mark.parametrize("use_rev", [False, True])
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("n,k,j_nn", [(2, 1, 1), (6, 5, 3), (20, 15, 15), (40, 32, 32), (300, 15, 15), (500, 16, 16),
+                                      (257, 17, 8), (1000, 22, 22), (900, 23, 23), (700, 32, 32), (350, 31, 20)])
+def test_select_matches_the_general_row_update(n, k, j_nn, recompute, use_rev):
+    """umapb_nnd_select against umapb_nnd_iteration on the same join: integer coordinates
+    make every distance exact, so the lists have to be equal, ties and fillers included.
+    Rows of 1 to 32 neighbours on either side of 8, 16 and 32 registers of candidates,
+    repeated ids, the row itself, hubs listed by more than 32 rows and rows listed by
+    none, fewer distinct candidates than k."""
+    from mlx_vis_b200 import _lib
+
+    rng = np.random.default_rng(n * 100 + k)
+    X = rng.integers(-3, 4, size=(n, 8)).astype(np.float32)
+    idx = rng.integers(0, n, size=(n, k)).astype(np.int32)
+    hubs = rng.random((n, k)) < 0.15
+    idx[hubs] = rng.integers(0, min(n, 3), size=int(hubs.sum()))
+    d2 = ((X[:, None, :] - X[idx]) ** 2).sum(-1).astype(np.float32)
+    s = _lib.stream_handle()
+
+    def dev(a):
+        return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    Xd, idx_d, dist = dev(X), dev(idx), dev(d2)
+    sq = dev((X ** 2).sum(1).astype(np.float32))
+    order = dev(rng.permutation(n).astype(np.int32))
+    nnbuf = torch.empty(n * k * j_nn, device="cuda")
+    curd = torch.empty((n, k), device="cuda")
+    rev = torch.empty((n, k), dtype=torch.int32, device="cuda")
+    d0 = torch.empty(n, device="cuda")
+    ws = _lib.workspace(_lib.query("umapb_nnd_join_workspace", n, k, k), Xd.device)
+    _lib.call("umapb_nnd_join", _lib.ptr(Xd), _lib.ptr(sq), 8, 8, 0, _lib.ptr(idx_d), _lib.ptr(order), n, k, k, j_nn,
+              _lib.ptr(nnbuf), _lib.ptr(curd), _lib.ptr(rev), _lib.ptr(None), _lib.ptr(ws), ws.numel(), s)
+    _lib.call("umapb_nnd_dist_row0", _lib.ptr(Xd), _lib.ptr(sq), n, 8, 8, 0, _lib.ptr(d0), s)
+    got = []
+    for general in (True, False):
+        out = (torch.empty_like(idx_d), torch.empty_like(dist), torch.empty((n, k), dtype=torch.uint8, device="cuda"),
+               torch.zeros(1, dtype=torch.int64, device="cuda"))
+        if general:
+            _lib.call("umapb_nnd_iteration", _lib.ptr(Xd), _lib.ptr(sq), 8, 8, 0, _lib.ptr(idx_d), _lib.ptr(dist),
+                      _lib.ptr(None), _lib.ptr(rev if use_rev else None), _lib.ptr(order), _lib.ptr(nnbuf),
+                      _lib.ptr(curd), n, k, k, j_nn, 0, int(recompute), *(_lib.ptr(t) for t in out), _lib.ptr(None), s)
+        else:
+            _lib.call("umapb_nnd_select", _lib.ptr(idx_d), _lib.ptr(dist), _lib.ptr(order), _lib.ptr(nnbuf),
+                      _lib.ptr(curd), _lib.ptr(d0), n, k, j_nn, int(recompute), _lib.ptr(ws if use_rev else None),
+                      ws.numel(), *(_lib.ptr(t) for t in out), s)
+        got.append([t.cpu().numpy() for t in out])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("d", [5, 50, 102])
+def test_rows_that_are_not_whole_float4s(d):
+    """Row lengths that are not a multiple of four go through the joins on zero-padded
+    copies: the same graph as without the join, but for ties in the FP32 sums."""
+    import os
+
+    from mlx_vis_b200 import NNDescent
+
+    X = np.random.default_rng(d).integers(-40, 41, size=(1500, d)).astype(np.float32)  # exact FP32 distances
+    idx, dist = NNDescent(k=12, random_state=3, n_iters=1).build(X)
+    os.environ["UMAPB_NND_JOIN"] = "0"
+    try:
+        idx0, dist0 = NNDescent(k=12, random_state=3, n_iters=1).build(X)
+    finally:
+        del os.environ["UMAPB_NND_JOIN"]
+    # d > 100: the first iteration runs on the rounded products with the random projection
+    assert np.mean(idx != idx0) <= (0.002 if d > 100 else 0.0)
+    np.testing.assert_allclose(dist, dist0, rtol=1e-5 if d > 100 else 0.0)
