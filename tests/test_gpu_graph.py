@@ -260,3 +260,52 @@ def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim):
     assert np.abs(outs[0] - Y0).max() > 1e-3 * scale
     assert np.median(np.abs(outs[1] - outs[0])) < 1e-5 * scale
     assert np.abs(outs[1] - outs[0]).max() < 1e-2 * scale
+
+
+@pytest.mark.parametrize("n,k,dim", [(17, 16, 2), (300, 5, 1), (300, 40, 4), (2560, 12, 4), (2561, 12, 4),
+                                     (5120, 9, 2), (5121, 9, 2), (9000, 24, 3)])
+def test_power_iteration_forms_match_float64(n, k, dim):
+    """The cluster form (up to 5,120 rows of 16 bytes, 2,560 of 32) and the grid-wide one on
+    either side of their border, uneven row counts per CTA and more edges than a CTA's
+    shared memory was sized for, against float64 torch.  FP32 storage of V leaves 100
+    rounded steps: 1e-5 of the 0..10 range."""
+    from mlx_vis_b200 import _lib
+
+    rng = np.random.default_rng(n + dim)
+    deg = np.where(np.arange(n) < n // 4, k, np.maximum(1, k // 4))  # the first quarter has most of the edges
+    rows = np.repeat(np.arange(n), deg).astype(np.int32)
+    near = (rows + rng.integers(1, min(n - 1, 40) + 1, size=rows.size)) % n
+    cols = near.astype(np.int32)
+    vals = rng.uniform(0.2, 1.0, size=rows.size).astype(np.float32)
+    V0 = rng.normal(size=(n, dim + 1)).astype(np.float32)
+    noise = (1e-4 * rng.normal(size=(n, dim))).astype(np.float32)
+    ne = torch.tensor([rows.size], dtype=torch.int64, device="cuda")
+    Y = _lib.spectral(cuda(rows), cuda(cols), cuda(vals), ne, n, dim, cuda(V0), cuda(noise), n_iter=100,
+                      check=True).cpu().numpy()
+    r, c, w = torch.from_numpy(rows).long(), torch.from_numpy(cols).long(), torch.from_numpy(vals).double()
+    d = torch.zeros(n, dtype=torch.float64).index_add_(0, r, w).clamp_min(1e-10)
+    wn = w / (d[r] * d[c]).sqrt()
+    V = torch.from_numpy(V0).double()
+    for _ in range(100):
+        V = torch.zeros_like(V).index_add_(0, r, wn[:, None] * V[c])
+        V, R = torch.linalg.qr(V)
+        V = V * R.diagonal().sign()  # the reference's norms are positive
+    e = V[:, 1:]
+    e = e * (10.0 / e.abs().max()) + torch.from_numpy(noise).double()
+    want = (10.0 * (e - e.amin(0)) / (e.amax(0) - e.amin(0) + 1e-10)).numpy()
+    assert np.abs(Y - want).max() < 1e-4
+
+
+@pytest.mark.parametrize("n,k", [(40, 2), (333, 9), (333, 10), (1000, 66), (40000, 17), (40000, 18)])
+def test_fuzzy_lanes_match_float64(n, k):
+    """The bisection with 8 lanes per row (few rows) and 2 (many): neighbours on either side
+    of the gaps a lane keeps in registers, rows with equal and with zero distances."""
+    rng = np.random.default_rng(n + k)
+    dist = np.sort(rng.uniform(0.5, 3.0, size=(n, k)), axis=1).astype(np.float32)
+    dist[::7, : k // 2] = 0.0
+    dist[::11] = 1.25
+    idx = ((np.arange(n)[:, None] + 1 + np.arange(k)) % n).astype(np.int32)
+    (r, c, v), _ = gpu_fuzzy(idx, dist, 200, fp64=True)
+    (ro, co, vo), _ = ofz.fuzzy_simplicial_set(idx, dist, 200, dtype=np.float64)
+    assert np.array_equal(r, ro) and np.array_equal(c, co)
+    np.testing.assert_allclose(v, vo, rtol=1e-6)
