@@ -352,15 +352,18 @@ int umapb_layout_epoch_injected(float* Y, int64_t n, int32_t dim, const int32_t*
  *   C + s M ldc, whose sum is the product); UMAPB_GEMM_BIAS_GELU (Z = C + bias,
  *   H = bf16(gelu(Z)), optional H^T);
  *   UMAPB_GEMM_GELU_BACK (H = bf16(C * gelu'(Z)), optional H^T, optional column
- *   sums of H in colsum, zeroed by the call).  *status (device int32) reports an
- *   expired bounded wait.
+ *   sums of H in colsum, zeroed by the call); UMAPB_GEMM_BIAS_GELU_H (H alone).
+ *   *status (device int32) reports an expired bounded wait.
+ * umapb_gemm_bf16_layout: the same with either operand stored by K rows when its flag is
+ *   set (A: K x M, pitch lda >= M; B: K x N, pitch ldb >= N): both flags with
+ *   UMAPB_GEMM_F32, b_mn alone with UMAPB_GEMM_F32 or UMAPB_GEMM_GELU_BACK.
  * umapb_mlp_convert: X f32 (rows x d; row r taken from row row_idx[r] when row_idx,
  *   a device int64 array, is given) -> BF16 (rows x ldx, zero padded) and an
  *   optional transposed BF16 copy (d x rows, pitch ldt).
  * umapb_mlp_head_forward: Y = H W^T + b for the last layer (c <= 4, FP32 W).
  * umapb_mlp_head_backward: MSE loss mean_b |Y - T|^2 (device f32; T row t_idx[b] when
  *   the device int64 array t_idx is given), dY, dW = dY^T H2,
- *   db = sum dY, dZ2 = bf16((dY W) * gelu'(Z2)) row-major and transposed, and
+ *   db = sum dY, dZ2 = bf16((dY W) * gelu'(Z2)) row-major and (dZ2T not null) transposed, and
  *   dbias2 = column sums of dZ2 (loss, dW, db, dbias2 zeroed by the call).
  * umapb_adamw: decoupled-weight-decay Adam on n_groups (<= 8) FP32 master
  *   tensors in one launch (host arrays of device pointers and shapes), bias-
@@ -374,10 +377,15 @@ int umapb_layout_epoch_injected(float* Y, int64_t n, int32_t dim, const int32_t*
 #define UMAPB_GEMM_F32 0
 #define UMAPB_GEMM_BIAS_GELU 1
 #define UMAPB_GEMM_GELU_BACK 2
+#define UMAPB_GEMM_BIAS_GELU_H 3
 int umapb_gemm_bf16(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t lda, int32_t ldb,
                     int32_t epilogue, int32_t ksplit, float* C, int32_t ldc, const float* bias, float* Z, int32_t ldz,
                     void* H, int32_t ldh, void* HT, int32_t ldt, float* colsum, int32_t* status,
                     umapb_stream_t stream);
+int umapb_gemm_bf16_layout(const void* A, int32_t a_mn, const void* B, int32_t b_mn, int32_t M, int32_t N, int32_t K,
+                           int32_t lda, int32_t ldb, int32_t epilogue, int32_t ksplit, float* C, int32_t ldc,
+                           const float* bias, float* Z, int32_t ldz, void* H, int32_t ldh, void* HT, int32_t ldt,
+                           float* colsum, int32_t* status, umapb_stream_t stream);
 int umapb_mlp_convert(const float* X, const int64_t* row_idx, int32_t rows, int32_t d, int32_t ldx, void* Xb,
                       void* XT, int32_t ldt, umapb_stream_t stream);
 int umapb_mlp_head_forward(const void* H, int32_t ldh, int32_t B, int32_t Hd, const float* W, const float* bias,

@@ -65,6 +65,8 @@ SIGNATURES = {
     "umapb_kernel_launches": [],
     "umapb_gemm_bf16": [_p, _p, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _i32, _p, _p, _i32, _p, _i32, _p,
                         _i32, _p, _p, _p],
+    "umapb_gemm_bf16_layout": [_p, _i32, _p, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _p, _i32, _p, _p, _i32,
+                               _p, _i32, _p, _i32, _p, _p, _p],
     "umapb_mlp_convert": [_p, _p, _i32, _i32, _i32, _p, _p, _i32, _p],
     "umapb_mlp_head_forward": [_p, _i32, _i32, _i32, _p, _p, _i32, _p, _p],
     "umapb_mlp_head_backward": [_p, _p, _p, _i32, _i32, _p, _i32, _p, _i32, _p, _i32, _p, _p, _p, _p, _i32, _p,

@@ -25,7 +25,7 @@ from mlx_vis_b200 import _lib
 from mlx_vis_b200._device import device, to_device_f32, to_host
 from mlx_vis_b200._lib import call, ptr, stream_handle
 
-F32, BIAS_GELU, GELU_BACK = 0, 1, 2
+F32, BIAS_GELU, GELU_BACK, BIAS_GELU_H = 0, 1, 2, 3
 
 
 def _pad8(x: int) -> int:
@@ -67,10 +67,14 @@ class Encoder:
                        "W2": torch.empty((self.KSPLIT_MAX, h, h), device=self.dev)}
         for k, t in self._gpart.items():
             self.grads[k] = t[0]
+        # the sums that the head's backward kernel accumulates, one array: one memset
+        sums = torch.empty(c * h + c + h, device=self.dev)
+        self.grads["W3"] = sums[:c * h].view(c, h)
+        self.grads["b3"] = sums[c * h:c * h + c]
+        self.grads["b2"] = sums[c * h + c:]
         bf = torch.bfloat16
         self.W1b = torch.zeros((h, self.ldx), dtype=bf, device=self.dev)
         self.W2b = torch.empty((h, h), dtype=bf, device=self.dev)
-        self.W2bT = torch.empty((h, h), dtype=bf, device=self.dev)
         self._refresh_bf16()
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.step_t = torch.zeros(1, dtype=torch.int32, device=self.dev)  # AdamW step number on the device
@@ -78,48 +82,49 @@ class Encoder:
         self.history_ = []
         self.y_scale_ = None  # (mean, std) of the targets the encoder was trained on
 
+    @property
+    def W2bT(self) -> torch.Tensor:
+        """W2^T in BF16: a view, the backward product reads W2 as it is stored."""
+        return self.W2b.t()
+
     # ------------------------------------------------------------------
     def _refresh_bf16(self):
         p = self.params
         self.W1b[:, : self.d].copy_(p["W1"].to(torch.bfloat16))
         self.W2b.copy_(p["W2"].to(torch.bfloat16))
-        self.W2bT.copy_(p["W2"].t().to(torch.bfloat16))
 
     def _buffers(self, B: int, train: bool):
         key = (B, train)
         if key in self._buf:
             return self._buf[key]
         dev, bf, h, c = self.dev, torch.bfloat16, self.h, self.c
-        ldb = _pad8(B)
-        b = {"Xb": torch.empty((B, self.ldx), dtype=bf, device=dev), "Z1": torch.empty((B, h), device=dev),
-             "H1": torch.empty((B, h), dtype=bf, device=dev), "Z2": torch.empty((B, h), device=dev),
-             "H2": torch.empty((B, h), dtype=bf, device=dev), "Y": torch.empty((B, c), device=dev), "ldb": ldb}
+        b = {"Xb": torch.empty((B, self.ldx), dtype=bf, device=dev), "H1": torch.empty((B, h), dtype=bf, device=dev),
+             "H2": torch.empty((B, h), dtype=bf, device=dev), "Y": torch.empty((B, c), device=dev)}
         if train:
-            b.update({"XT": torch.zeros((self.d, ldb), dtype=bf, device=dev),
-                      "H1T": torch.zeros((h, ldb), dtype=bf, device=dev),
+            b.update({"Z1": torch.empty((B, h), device=dev), "Z2": torch.empty((B, h), device=dev),
                       "dY": torch.empty((B, c), device=dev), "dZ2": torch.empty((B, h), dtype=bf, device=dev),
-                      "dZ2T": torch.zeros((h, ldb), dtype=bf, device=dev),
-                      "dZ1": torch.empty((B, h), dtype=bf, device=dev),
-                      "dZ1T": torch.zeros((h, ldb), dtype=bf, device=dev),
-                      "loss": torch.zeros(1, device=dev)})
+                      "dZ1": torch.empty((B, h), dtype=bf, device=dev), "loss": torch.zeros(1, device=dev)})
         self._buf[key] = b
         return b
 
-    def _gemm(self, A, Bm, M, N, K, lda, ldb, epi, C=None, ldc=0, bias=None, Z=None, ldz=0, H=None, ldh=0, HT=None,
-              ldt=0, ksplit=1, colsum=None):
-        call("umapb_gemm_bf16", ptr(A), ptr(Bm), M, N, K, lda, ldb, epi, ksplit, ptr(C), ldc, ptr(bias), ptr(Z), ldz,
-             ptr(H), ldh, ptr(HT), ldt, ptr(colsum), ptr(self.status), stream_handle())
+    def _gemm(self, A, Bm, M, N, K, lda, ldb, epi, C=None, ldc=0, bias=None, Z=None, ldz=0, H=None, ldh=0, ksplit=1,
+              colsum=None, a_mn=0, b_mn=0):
+        """C = A Bm^T; ``a_mn`` / ``b_mn``: the operand is stored with K as its row index."""
+        call("umapb_gemm_bf16_layout", ptr(A), a_mn, ptr(Bm), b_mn, M, N, K, lda, ldb, epi, ksplit, ptr(C), ldc,
+             ptr(bias), ptr(Z), ldz, ptr(H), ldh, ptr(None), 0, ptr(colsum), ptr(self.status), stream_handle())
 
-    def _forward(self, X: torch.Tensor, b, train: bool, rows=None):
+    def _forward(self, X: torch.Tensor, b, train: bool, rows=None, out=None):
+        """The layers on X's rows (or its rows ``rows``); the last one into ``out`` or b["Y"]."""
         B = X.shape[0] if rows is None else rows.numel()
         h, p, s = self.h, self.params, stream_handle()
-        call("umapb_mlp_convert", ptr(X), ptr(rows), B, self.d, self.ldx, ptr(b["Xb"]),
-             ptr(b["XT"] if train else None), b["ldb"], s)
-        self._gemm(b["Xb"], self.W1b, B, h, self.d, self.ldx, self.ldx, BIAS_GELU, bias=p["b1"], Z=b["Z1"], ldz=h,
-                   H=b["H1"], ldh=h, HT=b["H1T"] if train else None, ldt=b["ldb"])
-        self._gemm(b["H1"], self.W2b, B, h, h, h, h, BIAS_GELU, bias=p["b2"], Z=b["Z2"], ldz=h, H=b["H2"], ldh=h)
-        call("umapb_mlp_head_forward", ptr(b["H2"]), h, B, h, ptr(p["W3"]), ptr(p["b3"]), self.c, ptr(b["Y"]), s)
-        return b["Y"]
+        Y = b["Y"] if out is None else out
+        call("umapb_mlp_convert", ptr(X), ptr(rows), B, self.d, self.ldx, ptr(b["Xb"]), ptr(None), 0, s)
+        epi = BIAS_GELU if train else BIAS_GELU_H  # the pre-activations are for the backward pass
+        self._gemm(b["Xb"], self.W1b, B, h, self.d, self.ldx, self.ldx, epi, bias=p["b1"], Z=b.get("Z1"), ldz=h,
+                   H=b["H1"], ldh=h)
+        self._gemm(b["H1"], self.W2b, B, h, h, h, h, epi, bias=p["b2"], Z=b.get("Z2"), ldz=h, H=b["H2"], ldh=h)
+        call("umapb_mlp_head_forward", ptr(b["H2"]), h, B, h, ptr(p["W3"]), ptr(p["b3"]), self.c, ptr(Y), s)
+        return Y
 
     # ------------------------------------------------------------------
     def train_step(self, X: torch.Tensor, T: torch.Tensor, rows=None) -> torch.Tensor:
@@ -134,17 +139,17 @@ class Encoder:
         s = stream_handle()
         ks = self._ksplit(B)
         self._forward(X, b, True, rows)
-        # dY, loss, dW3, db3, dZ2 (+ transpose), db2
+        # dY, loss, dW3, db3, dZ2, db2
         call("umapb_mlp_head_backward", ptr(b["Y"]), ptr(T), ptr(rows), B, c, ptr(p["W3"]), h, ptr(b["Z2"]), h,
-             ptr(b["H2"]), h, ptr(b["dY"]), ptr(g["W3"]), ptr(g["b3"]), ptr(b["dZ2"]), h, ptr(b["dZ2T"]), b["ldb"],
+             ptr(b["H2"]), h, ptr(b["dY"]), ptr(g["W3"]), ptr(g["b3"]), ptr(b["dZ2"]), h, ptr(None), 0,
              ptr(g["b2"]), ptr(b["loss"]), s)
-        # dW2 = dZ2^T H1 (K = B in ks slices)
-        self._gemm(b["dZ2T"], b["H1T"], h, h, B, b["ldb"], b["ldb"], F32, C=self._gpart["W2"], ldc=h, ksplit=ks)
-        # dZ1 = (dZ2 W2) * gelu'(Z1) (+ transpose), db1 = its column sums
-        self._gemm(b["dZ2"], self.W2bT, B, h, h, h, h, GELU_BACK, Z=b["Z1"], ldz=h, H=b["dZ1"], ldh=h, HT=b["dZ1T"],
-                   ldt=b["ldb"], colsum=g["b1"])
+        # dW2 = dZ2^T H1 (K = B in ks slices); both operands as they are stored, by batch rows
+        self._gemm(b["dZ2"], b["H1"], h, h, B, h, h, F32, C=self._gpart["W2"], ldc=h, ksplit=ks, a_mn=1, b_mn=1)
+        # dZ1 = (dZ2 W2) * gelu'(Z1), db1 = its column sums; W2 is stored by its K index
+        self._gemm(b["dZ2"], self.W2b, B, h, h, h, h, GELU_BACK, Z=b["Z1"], ldz=h, H=b["dZ1"], ldh=h,
+                   colsum=g["b1"], b_mn=1)
         # dW1 = dZ1^T X (K = B in ks slices)
-        self._gemm(b["dZ1T"], b["XT"], h, d, B, b["ldb"], b["ldb"], F32, C=self._gpart["W1"], ldc=d, ksplit=ks)
+        self._gemm(b["dZ1"], b["Xb"], h, d, B, h, self.ldx, F32, C=self._gpart["W1"], ldc=d, ksplit=ks, a_mn=1, b_mn=1)
         self.step_count += 1
         self.step_t.add_(1)
         self._adamw(ks)
@@ -164,7 +169,7 @@ class Encoder:
             n = len(names)
             P = ctypes.c_void_p * n
             I = ctypes.c_int32 * n
-            bf = {"W1": (self.W1b, self.ldx, None, 0), "W2": (self.W2b, self.h, self.W2bT, self.h)}
+            bf = {"W1": (self.W1b, self.ldx, None, 0), "W2": (self.W2b, self.h, None, 0)}
             shp = [(t.shape[0], t.shape[1]) if t.dim() == 2 else (1, t.shape[0]) for t in self.params.values()]
             self._adamw_names = names
             self._adamw_stride = (ctypes.c_int64 * n)(*[self.params[k].numel() if k in self._gpart else 0
@@ -247,7 +252,7 @@ class Encoder:
         for s0 in range(0, X.shape[0], chunk):
             xb = X[s0:s0 + chunk]
             b = self._buffers(xb.shape[0], False)
-            out[s0:s0 + xb.shape[0]].copy_(self._forward(xb, b, False))
+            self._forward(xb, b, False, out=out[s0:s0 + xb.shape[0]])
         if self.y_scale_ is not None:
             mean, std = self.y_scale_
             out = out * std + mean

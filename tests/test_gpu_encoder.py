@@ -66,6 +66,52 @@ def test_gemm_epilogues_match_float64():
     assert (cs.cpu().double() - want).abs().max() < 1e-4 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("M,N,K,a_mn,ksplit", [(512, 784, 4096, 1, 8), (512, 267, 1000, 1, 2), (100, 64, 70, 1, 1),
+                                               (8, 8, 1, 1, 1), (129, 65, 200, 1, 4), (1000, 512, 512, 0, 1),
+                                               (200, 72, 136, 0, 1), (20000, 136, 64, 0, 1)])
+def test_gemm_operands_stored_by_k(M, N, K, a_mn, ksplit):
+    """umapb_gemm_bf16_layout with B (and A) stored by K rows: tiles of 64 and 128 columns,
+    remainders in every direction, K slices, columns past the operands' padding."""
+    from mlx_vis_b200 import _lib
+
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randn((M, K), generator=g).to(torch.bfloat16)
+    B = torch.randn((N, K), generator=g).to(torch.bfloat16)
+
+    def stored(x, mn):  # rows of a multiple of 8 values; what lies past the operand must not count
+        x = x.T if mn else x
+        out = torch.full((x.shape[0], (x.shape[1] + 7) // 8 * 8), 7.0, dtype=torch.bfloat16, device="cuda")
+        out[:, :x.shape[1]] = x.cuda()
+        return out
+
+    Ad, Bd = stored(A, a_mn), stored(B, 1)
+    C = torch.full((ksplit, M, N), float("nan"), device="cuda")
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.call("umapb_gemm_bf16_layout", _lib.ptr(Ad), a_mn, _lib.ptr(Bd), 1, M, N, K, Ad.shape[1], Bd.shape[1], 0,
+              ksplit, _lib.ptr(C), N, *(_lib.ptr(None),) * 2, 0, _lib.ptr(None), 0, _lib.ptr(None), 0, _lib.ptr(None),
+              _lib.ptr(st), _lib.stream_handle())
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0
+    ref = A.double() @ B.double().T
+    assert (C.sum(0).cpu().double() - ref).abs().max() / ref.abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("B,d,c,hidden", [(1, 16, 1, 512), (130, 33, 3, 512), (300, 100, 2, 64), (1200, 7, 4, 512)])
+def test_transform_matches_float64(B, d, c, hidden):
+    """The inference path (no pre-activations kept) at row lengths on and off the vector
+    loads, the default width and another, against float64: BF16 operands in three layers."""
+    from mlx_vis_b200.encoder import Encoder
+
+    enc = Encoder(d, hidden=hidden, out_dim=c, seed=3)
+    X = torch.rand((B, d), generator=torch.Generator().manual_seed(d)).cuda()
+    got = enc.transform_device(X, chunk=1000).double()
+    p = {k: v.double() for k, v in enc.params.items()}
+    h = torch.nn.functional.gelu(X.double() @ p["W1"].T + p["b1"])
+    h = torch.nn.functional.gelu(h @ p["W2"].T + p["b2"])
+    want = h @ p["W3"].T + p["b3"]
+    assert (got - want).norm() / want.norm() < 2e-2
+
+
 def _params(enc):
     return {k: v.detach().cpu().numpy().copy() for k, v in enc.params.items()}
 
