@@ -28,6 +28,7 @@
 
 #include <mutex>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "philox.cuh"
 #include "scan.cuh"
@@ -37,6 +38,7 @@ namespace layout {
 
 constexpr int kBlock = 256;
 constexpr int kEdgesPerBlock = 1024;
+constexpr int64_t kClusterRows = 65536;  // the cluster form: row ids of 16 bits
 #ifndef UMAPB_LAYOUT_BLOCKS_PER_SM
 #define UMAPB_LAYOUT_BLOCKS_PER_SM 4
 #endif
@@ -300,6 +302,151 @@ __global__ void apply_kernel(float* __restrict__ Y, float* __restrict__ dY, int6
   }
 }
 
+// ---- few edges: all epochs in one launch of one cluster --------------------------
+// Two launches per epoch cost more than the work of a few thousand due edges (2,000 points:
+// 6.5 us an epoch, most of it launches and L2 round trips).  Here one cluster keeps everything
+// on chip for all epochs: every CTA a copy of Y and an equal share of the edges (schedule,
+// ids).  An epoch is: queue the due edges; gather from the own copy of Y, add the moves to
+// dY in L2; cluster barrier; every CTA adds all of dY to its copy.  dY is one of three arrays
+// in turn: while an epoch adds to one, a CTA may still be reading the previous one, and the
+// next one, which every CTA has read before the last barrier, is cleared.  The draws and the pair math are those of the launches.
+// (Moves added in the owners' shared memory took 23 us an epoch: float adds there are
+// compare-and-swap loops, remote ones a round trip a try.  Owners that apply their rows and
+// store them into all copies need a second barrier: 6.3 us.)  What bounds it: the
+// pair math on the cluster's SMs, so it serves up to kClusterEdges edges; beyond, the
+// whole chip is faster (60,000 edges: 8.5-10 us on a cluster, 7-8 by launches).  B200, per
+// epoch: 600 points, k = 5 8.0 -> 3.3 us; 2,000 points, k = 15 6.7 -> 5.2 us.
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterMax = 16;             // CTAs; 8 where 16 cannot be scheduled together
+constexpr int64_t kClusterEdges = 32768;
+constexpr size_t kClusterSmem = 216 * 1024;
+
+struct ClusterArgs {
+  float *Y, *dY;  // dY: three arrays of n * DIM
+  const int32_t *rows, *cols;
+  const float* eps;
+  float* next;
+  const int64_t* n_edges;
+  int n, epoch_begin, epoch_end, n_epochs, neg_rate;
+  int rows_per;  // rows that a CTA owns
+  int cap;       // edges per CTA
+  float a, b, m2ab, two_b, lr;
+  uint32_t k0, k1;
+};
+
+static size_t cluster_smem(int64_t n, int dim, int cap) { return 4 * (size_t)n * dim + (size_t)cap * 14 + 64; }
+
+template <int DIM, int NEG>
+__global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(ClusterArgs a) {
+  extern __shared__ __align__(16) unsigned char layout_smem[];
+  float* sy = reinterpret_cast<float*>(layout_smem);  // Y
+  float* s_next = sy + (size_t)a.n * DIM;             // the share's edges: schedule ...
+  float* s_eps = s_next + a.cap;
+  uint32_t* s_ids = reinterpret_cast<uint32_t*>(s_eps + a.cap);  // ... head | tail << 16
+  uint16_t* s_queue = reinterpret_cast<uint16_t*>(s_ids + a.cap);
+  __shared__ int s_due;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int rank = (int)cluster::rank(), ctas = (int)cluster::size();
+  const int64_t E = *a.n_edges < (int64_t)a.cap * ctas ? *a.n_edges : (int64_t)a.cap * ctas;
+  const int per = (int)((E + ctas - 1) / ctas);
+  const int64_t e0 = (int64_t)rank * per;
+  const int m = (int)(E - e0 < 0 ? 0 : E - e0 < per ? E - e0 : per);
+  const int r0 = rank * a.rows_per;
+  const int own = a.n - r0 < 0 ? 0 : a.n - r0 < a.rows_per ? a.n - r0 : a.rows_per;
+  for (int t = tid; t < a.n * DIM; t += kClusterThreads) sy[t] = a.Y[t];
+  const int values = a.n * DIM;
+  for (int t = tid; t < own * DIM; t += kClusterThreads) __stcg(a.dY + r0 * DIM + t, 0.f);  // the first array
+  for (int t = tid; t < m; t += kClusterThreads) {
+    s_next[t] = a.next[e0 + t];
+    s_eps[t] = a.eps[e0 + t];
+    s_ids[t] = (uint32_t)a.rows[e0 + t] | ((uint32_t)a.cols[e0 + t] << 16);
+  }
+  auto row = [&](uint32_t i, float (&v)[DIM]) {
+    if constexpr (DIM == 2) {
+      const float2 t = *reinterpret_cast<const float2*>(sy + 2 * i);
+      v[0] = t.x;
+      v[1] = t.y;
+    } else {
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) v[c] = sy[i * DIM + c];
+    }
+  };
+  if (tid == 0) s_due = 0;
+  __syncwarp();
+  cluster::barrier();  // the first array is zero
+
+  Params p;
+  p.a = a.a;
+  p.b = a.b;
+  p.m2ab = a.m2ab;
+  p.two_b = a.two_b;
+  int turn = 0;
+  for (int ep = a.epoch_begin; ep < a.epoch_end; ++ep) {
+    float* dY = a.dY + (size_t)turn * values;
+    const int then = turn == 2 ? 0 : turn + 1;
+    float* next_dY = a.dY + (size_t)then * values;
+    // make_params' double arithmetic
+    p.alpha = (float)__dmul_rn((double)a.lr, __dsub_rn(1.0, __ddiv_rn((double)ep, (double)a.n_epochs)));
+    const float epf = (float)ep;
+    for (int b0 = tid - lane; b0 < m; b0 += kClusterThreads) {
+      const int t = b0 + lane;
+      bool due = false;
+      if (t < m) {
+        const float nx = s_next[t];
+        due = nx <= epf;
+        if (due) s_next[t] = __fadd_rn(nx, s_eps[t]);
+      }
+      const unsigned b = __ballot_sync(0xffffffffu, due);
+      int slot = 0;
+      if (lane == 0 && b) slot = atomicAdd(&s_due, __popc(b));
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+      if (due) s_queue[slot + __popc(b & below)] = (uint16_t)t;
+    }
+    __syncthreads();
+    const int total = s_due;
+    for (int q = tid; q < total; q += kClusterThreads) {
+      const int t = s_queue[q];
+      const uint32_t e = (uint32_t)(e0 + t);  // below 2^32: the share fits a CTA
+      const uint32_t ij = s_ids[t], i = ij & 0xffffu, j = ij >> 16;
+      float yi[DIM], yj[DIM], acc[DIM], pos[DIM], neg_pos[DIM];
+      row(i, yi);
+      row(j, yj);
+      attract<DIM>(yi, yj, p, pos);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        acc[c] = pos[c];
+        neg_pos[c] = -pos[c];
+      }
+      atomic_add_row<DIM>(dY, (int)j, neg_pos);
+      const int nr = NEG > 0 ? NEG : a.neg_rate;
+#pragma unroll 1
+      for (int m0 = 0; m0 < nr; m0 += 4) {
+        const U4 r = philox4x32_10(U4{e, 0u, (uint32_t)ep, (uint32_t)(m0 >> 2)}, a.k0, a.k1);
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (m0 + u < nr) {
+            float yt[DIM];
+            row((uint32_t)to_range(w[u], (uint32_t)a.n), yt);
+            repel_add<DIM>(yi, yt, p, acc);
+          }
+        }
+      }
+      atomic_add_row<DIM>(dY, (int)i, acc);
+    }
+    for (int t = tid; t < own * DIM; t += kClusterThreads) __stcg(next_dY + r0 * DIM + t, 0.f);
+    __syncwarp();
+    cluster::barrier();  // all moves have been added, and the next array is zero
+    if (tid == 0) s_due = 0;
+    for (int t = tid; t < values; t += kClusterThreads) sy[t] = __fadd_rn(sy[t], __ldcg(dY + t));
+    turn = then;
+    __syncthreads();
+  }
+  for (int t = tid; t < m; t += kClusterThreads) a.next[e0 + t] = s_next[t];
+  for (int t = tid; t < own * DIM; t += kClusterThreads) a.Y[r0 * DIM + t] = sy[r0 * DIM + t];
+}
+
 // ---- injected path (reference-ordered negatives) ------------------------------
 __global__ void count_active_kernel(const float* __restrict__ next, const int64_t* __restrict__ n_edges, int epoch,
                                     int32_t* __restrict__ block_counts) {
@@ -534,7 +681,7 @@ static Layout carve(void* ws, int64_t n, int dim, int64_t e_cap) {
   Layout l;
   l.status = c.take<int32_t>(64);
   l.wmax = c.take<float>(64);
-  l.dY = c.take<float>((size_t)n * dim);
+  l.dY = c.take<float>((size_t)n * dim * (n < kClusterRows && dim <= 4 ? 3 : 1));  // three: the cluster form
   l.block_counts = c.take<int32_t>((size_t)ceil_div(e_cap > 0 ? e_cap : 1, kEdgesPerBlock) + 1);
   l.total = c.take<int64_t>(8);
   l.scan_ws = c.take<int64_t>(kScanMaxBlocks);
@@ -613,6 +760,56 @@ static void launch_injected(const Layout& l, float* Y, int64_t n, const int32_t*
   apply_kernel<<<(unsigned)ceil_div(m, kBlock), kBlock, 0, stream>>>(Y, l.dY, m);
 }
 
+// Enqueues epochs [begin, end) on one cluster; false: the problem does not fit one, or the
+// device cannot schedule one (the launches serve it then).
+template <int DIM, int NEG>
+static bool launch_cluster(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
+  static std::mutex mu;
+  static int known[64] = {0};  // CTAs per cluster on this device; 0 unknown, -1 none
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  const auto kernel = layout_cluster_kernel<DIM, NEG>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kClusterThreads, 1, 1);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[dev] == 0) {
+      known[dev] = -1;
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem) == cudaSuccess &&
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        for (int c = kClusterMax; c >= 8 && known[dev] < 0; c /= 2) {
+          attr[0].val.clusterDim.x = c;
+          cfg.gridDim = dim3(c, 1, 1);
+          cfg.dynamicSmemBytes = kClusterSmem;
+          int clusters = 0;
+          if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) known[dev] = c;
+        }
+      }
+      cudaGetLastError();
+    }
+  }
+  const int ctas = known[dev];
+  if (ctas < 0) return false;
+  a.rows_per = (int)ceil_div(a.n, ctas);
+  a.cap = (int)ceil_div(e_cap, ctas);
+  cfg.dynamicSmemBytes = cluster_smem(a.n, DIM, a.cap);
+  if (cfg.dynamicSmemBytes > kClusterSmem) return false;
+  attr[0].val.clusterDim.x = ctas;
+  cfg.gridDim = dim3(ctas, 1, 1);
+  if (cudaLaunchKernelEx(&cfg, kernel, a) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
 }  // namespace layout
 }  // namespace umapb
 
@@ -644,17 +841,68 @@ extern "C" int umapb_layout_prepare(const float* vals, const int64_t* n_edges, i
   return UMAPB_OK;
 }
 
-static int enqueue_epochs(float* Y, int64_t n, int32_t dim, const int32_t* rows, const int32_t* cols,
-                          const float* eps, float* next, const int64_t* n_edges, int64_t e_cap, int32_t epoch_begin,
-                          int32_t epoch_end, int32_t n_epochs, float a, float b, float learning_rate,
-                          int32_t neg_rate, uint64_t seed, void* workspace, size_t workspace_bytes,
-                          cudaStream_t stream) {
+static int check_epochs(const float* Y, int64_t n, int32_t dim, const int32_t* rows, const int32_t* cols,
+                        const float* eps, const float* next, const int64_t* n_edges, int64_t e_cap,
+                        int32_t epoch_begin, int32_t epoch_end, int32_t n_epochs, int32_t neg_rate,
+                        const void* workspace, size_t workspace_bytes) {
   UMAPB_REQUIRE(Y && rows && cols && eps && next && n_edges, "layout_epochs: null array argument");
   UMAPB_REQUIRE(n >= 1 && n < ((int64_t)1 << 31), "layout_epochs: need 1 <= n < 2^31");
   UMAPB_REQUIRE(dim >= 1 && dim <= 32, "layout_epochs: dim must be in [1, 32]");
   UMAPB_REQUIRE(neg_rate >= 0, "layout_epochs: negative_sample_rate must be >= 0");
   UMAPB_REQUIRE(0 <= epoch_begin && epoch_begin <= epoch_end && epoch_end <= n_epochs,
                 "layout_epochs: need 0 <= epoch_begin <= epoch_end <= n_epochs");
+  const layout::Layout l = layout::carve(nullptr, n, dim, e_cap);
+  if (!workspace || workspace_bytes < l.bytes)
+    return set_error(UMAPB_ERR_WORKSPACE, "layout: workspace of %zu bytes, need %zu", workspace_bytes, l.bytes);
+  return UMAPB_OK;
+}
+
+// The cluster form, where the checked arguments allow it.
+static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* rows, const int32_t* cols,
+                            const float* eps, float* next, const int64_t* n_edges, int64_t e_cap, int32_t epoch_begin,
+                            int32_t epoch_end, int32_t n_epochs, float a, float b, float learning_rate,
+                            int32_t neg_rate, uint64_t seed, void* workspace, cudaStream_t stream) {
+  // below four epochs the load of the edges and the store of their schedule cost more than the
+  // launches (a callback after every epoch runs them one by one)
+  if (dim > 4 || n >= layout::kClusterRows || e_cap > layout::kClusterEdges || epoch_end - epoch_begin < 4) return false;
+  const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
+  layout::ClusterArgs c = {};
+  c.Y = Y;
+  c.dY = layout::carve(workspace, n, dim, e_cap).dY;
+  c.rows = rows;
+  c.cols = cols;
+  c.eps = eps;
+  c.next = next;
+  c.n_edges = n_edges;
+  c.n = (int)n;
+  c.epoch_begin = epoch_begin;
+  c.epoch_end = epoch_end;
+  c.n_epochs = n_epochs;
+  c.neg_rate = neg_rate;
+  c.a = p.a;
+  c.b = p.b;
+  c.m2ab = p.m2ab;
+  c.two_b = p.two_b;
+  c.lr = learning_rate;
+  c.k0 = (uint32_t)seed;
+  c.k1 = (uint32_t)(seed >> 32);
+  const bool five = neg_rate == 5;
+  bool ok = false;
+  switch (dim) {
+    case 1: ok = layout::launch_cluster<1, 0>(c, e_cap, stream); break;
+    case 2: ok = five ? layout::launch_cluster<2, 5>(c, e_cap, stream) : layout::launch_cluster<2, 0>(c, e_cap, stream); break;
+    case 3: ok = five ? layout::launch_cluster<3, 5>(c, e_cap, stream) : layout::launch_cluster<3, 0>(c, e_cap, stream); break;
+    default: ok = layout::launch_cluster<4, 0>(c, e_cap, stream); break;
+  }
+  if (ok) count_launches(1);
+  return ok;
+}
+
+static int enqueue_epochs(float* Y, int64_t n, int32_t dim, const int32_t* rows, const int32_t* cols,
+                          const float* eps, float* next, const int64_t* n_edges, int64_t e_cap, int32_t epoch_begin,
+                          int32_t epoch_end, int32_t n_epochs, float a, float b, float learning_rate,
+                          int32_t neg_rate, uint64_t seed, void* workspace, size_t workspace_bytes,
+                          cudaStream_t stream) {
   layout::Layout l = layout::carve(nullptr, n, dim, e_cap);
   if (!workspace || workspace_bytes < l.bytes)
     return set_error(UMAPB_ERR_WORKSPACE, "layout: workspace of %zu bytes, need %zu", workspace_bytes, l.bytes);
@@ -684,6 +932,12 @@ extern "C" int umapb_layout_epochs(float* Y, int64_t n, int32_t dim, const int32
                                    float learning_rate, int32_t neg_rate, uint64_t seed, void* workspace,
                                    size_t workspace_bytes, umapb_stream_t stream_) {
   clear_error();
+  if (const int rc = check_epochs(Y, n, dim, rows, cols, eps, next, n_edges, e_cap, epoch_begin, epoch_end, n_epochs,
+                                  neg_rate, workspace, workspace_bytes))
+    return rc;
+  if (enqueue_cluster(Y, n, dim, rows, cols, eps, next, n_edges, e_cap, epoch_begin, epoch_end, n_epochs, a, b,
+                      learning_rate, neg_rate, seed, workspace, reinterpret_cast<cudaStream_t>(stream_)))
+    return UMAPB_OK;
   return enqueue_epochs(Y, n, dim, rows, cols, eps, next, n_edges, e_cap, epoch_begin, epoch_end, n_epochs, a, b,
                         learning_rate, neg_rate, seed, workspace, workspace_bytes,
                         reinterpret_cast<cudaStream_t>(stream_));
@@ -715,6 +969,12 @@ extern "C" int umapb_layout_epochs_graph(float* Y, int64_t n, int32_t dim, const
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   UMAPB_CUDA_TRY(cudaStreamIsCapturing(stream, &cs), "layout_epochs_graph: capture query");
   UMAPB_REQUIRE(cs == cudaStreamCaptureStatusNone, "layout_epochs_graph: the stream is already being captured");
+  if (const int rc = check_epochs(Y, n, dim, rows, cols, eps, next, n_edges, e_cap, epoch_begin, epoch_end, n_epochs,
+                                  neg_rate, workspace, workspace_bytes))
+    return rc;
+  if (enqueue_cluster(Y, n, dim, rows, cols, eps, next, n_edges, e_cap, epoch_begin, epoch_end, n_epochs, a, b,
+                      learning_rate, neg_rate, seed, workspace, stream))
+    return UMAPB_OK;  // one launch: nothing to record
   std::lock_guard<std::mutex> lock(g_graph_mu);
   cudaStream_t& cap = g_capture_stream[dev];
   if (!cap) UMAPB_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "layout_epochs_graph: stream");

@@ -19,6 +19,7 @@
 
 #include <mutex>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "philox.cuh"
 
@@ -572,20 +573,6 @@ constexpr int kClusterThreads = 512;
 constexpr size_t kClusterSmem = 216 * 1024;
 constexpr size_t kClusterVBytes = 160 * 1024;  // both buffers of V: up to 5,120 rows of 16 bytes
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_address(uint32_t smem, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
-  return r;
-}
-
 template <int KK>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     power_cluster_kernel(float* __restrict__ V0, float* __restrict__ V1, const int64_t* __restrict__ row_ptr,
@@ -605,7 +592,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   __shared__ int s_next;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = threadIdx.x & (kLanes - 1);
-  const int rank = (int)cluster_rank();
+  const int rank = (int)cluster::rank();
   const int r_first = rank * rows_per_cta;
   const int rows = r_first < n ? (n - r_first < rows_per_cta ? n - r_first : rows_per_cta) : 0;
   const int64_t e_first = rows > 0 ? row_ptr[r_first] : 0;
@@ -620,10 +607,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   for (int t = threadIdx.x; t < v_words; t += kClusterThreads) v_all[t] = reinterpret_cast<const float4*>(V0)[t];
   cols += e_first;
   wn += e_first;
-  const uint32_t v_at = static_cast<uint32_t>(__cvta_generic_to_shared(v_all));
-  const uint32_t parts_at = static_cast<uint32_t>(__cvta_generic_to_shared(&parts[0][0][0]));
+  const uint32_t v_at = cluster::smem_address(v_all);
+  const uint32_t parts_at = cluster::smem_address(parts);
   // every CTA runs and has read V0 before its neighbours store into its copy
-  cluster_barrier();
+  cluster::barrier();
 
   bool rotate = false;
   int step = 0, every = 1, factored = 0;
@@ -686,7 +673,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         const uint32_t at = out_at + (uint32_t)((r_first + lr) * (vp / 4)) * 16u;
 #pragma unroll
         for (int p = 0; p < kClusterCtas / 2; ++p) {
-          const uint32_t dst = peer_address(at, (uint32_t)(2 * p + sub));
+          const uint32_t dst = cluster::peer(at, (uint32_t)(2 * p + sub));
           asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(out[0]), "f"(out[1]),
                        "f"(out[2]), "f"(out[3])
                        : "memory");
@@ -722,11 +709,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         const uint32_t at = parts_at + (uint32_t)((parity * kClusterCtas + rank) * KK * KK + (int)threadIdx.x) * 8u;
 #pragma unroll
         for (int p = 0; p < kClusterCtas; ++p)
-          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer_address(at, (uint32_t)p)), "d"(g) : "memory");
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster::peer(at, (uint32_t)p)), "d"(g) : "memory");
       }
     }
     __syncwarp();
-    cluster_barrier();
+    cluster::barrier();
     rotate = factor;
     if (factor) {
       if (threadIdx.x == 0) {

@@ -309,3 +309,36 @@ def test_fuzzy_lanes_match_float64(n, k):
     (ro, co, vo), _ = ofz.fuzzy_simplicial_set(idx, dist, 200, dtype=np.float64)
     assert np.array_equal(r, ro) and np.array_equal(c, co)
     np.testing.assert_allclose(v, vo, rtol=1e-6)
+
+
+@pytest.mark.parametrize("n,k,dim,neg", [(2, 1, 2, 5), (17, 3, 1, 5), (513, 7, 2, 5), (700, 9, 3, 5), (300, 5, 4, 2),
+                                         (2000, 15, 2, 0), (1025, 11, 2, 11), (3276, 10, 2, 5), (20, 1600, 2, 5)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_layout_cluster_matches_launches(n, k, dim, neg, graph):
+    """Epochs 3 to 12 on one cluster against the same epochs one call each (the launches):
+    the same due edges and draws; a small step keeps the sums' order from growing.  Row
+    counts around a power of two per CTA, every narrow dimension, no and many negatives,
+    the largest number of edges and an uneven last share; the schedule goes on after it."""
+    from mlx_vis_b200 import _lib
+
+    rng = np.random.default_rng(n + k)
+    E = n * k - n * k // 7  # fewer edges than the arrays have room for
+    rows = np.sort(rng.integers(0, n, size=n * k)).astype(np.int32)
+    cols = rng.integers(0, n, size=n * k).astype(np.int32)
+    vals = rng.uniform(0.05, 1.0, size=n * k).astype(np.float32)
+    ne = torch.tensor([E], dtype=torch.int64, device="cuda")
+    Y0 = cuda((10 * rng.normal(size=(n, dim))).astype(np.float32))
+    # an epoch pulls a row by up to 2ab = 2.8 rate per edge that lists it, 2 k of them: above 1 in
+    # all, a difference of the last bit grows from epoch to epoch instead of dying out
+    rate = min(0.01, 0.5 / (2.8 * 2 * k))
+    out = []
+    for calls in ([(3, 12), (12, 13)], [(e, e + 1) for e in range(3, 13)]):
+        lay = _lib.Layout(cuda(rows), cuda(cols), cuda(vals), ne, n, dim, 200)
+        Y = Y0.clone()
+        for b, e in calls:
+            lay.epochs(Y, b, e, 1.577, 0.895, rate, neg, 12345, graph=graph)
+        out.append((Y.cpu().numpy(), lay.next[:E].cpu().numpy()))
+    assert np.array_equal(out[0][1], out[1][1])
+    # float32 sums of up to (1 + neg) k clipped moves of at most 0.04 per epoch, in another order
+    scale = np.abs(Y0.cpu().numpy()).max()
+    assert np.abs(out[0][0] - out[1][0]).max() < 2e-5 * scale
