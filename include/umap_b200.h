@@ -202,6 +202,15 @@ int umapb_nnd_join(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, in
                    const int32_t* order, int64_t n, int32_t k, int32_t mc, int32_t j_nn, float* nnbuf, float* curd,
                    int32_t* rev_out, unsigned long long* evals, void* workspace, size_t workspace_bytes,
                    umapb_stream_t stream);
+/* umapb_nnd_join_prepare, umapb_nnd_join_prepared: umapb_nnd_join in two calls on one
+ * workspace, the buckets of the lists and the distances; the first depends on the
+ * lists alone, so it can be enqueued before the next iteration's space is known. */
+int umapb_nnd_join_prepare(const int32_t* idx_old, const int32_t* order, int64_t n, int32_t k, int32_t mc,
+                           void* workspace, size_t workspace_bytes, umapb_stream_t stream);
+int umapb_nnd_join_prepared(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, int32_t half,
+                            const int32_t* idx_old, const int32_t* order, int64_t n, int32_t k, int32_t mc,
+                            int32_t j_nn, float* nnbuf, float* curd, int32_t* rev_out, unsigned long long* evals,
+                            void* workspace, size_t workspace_bytes, umapb_stream_t stream);
 /* umapb_nnd_join_new: the blocked join of the converging path (nndescent.py:103-126):
  * the sources of row i are the first mc of its neighbours in NEW-first stable order
  * (none for a row without a NEW flag, whose list the iteration keeps); FP32 rows of

@@ -253,6 +253,7 @@ class NNDescent:
             call("umapb_nnd_pad_cols", ptr(X), n, d, di, ptr(Xi), s)
             if X_low is X:
                 X_low = Xi
+        prepared = False  # the join workspace holds the current lists' buckets
         dist0 = {}  # every row's distance to row 0 by (space, precision), for empty reverse slots
         self.kernel_log_ = []  # (start event, end event, info) per iteration kernel when profile_kernels
 
@@ -284,7 +285,9 @@ class NNDescent:
             changed_p = _c.c_void_p(cbase + 16 * it)  # counters[it, 0] and counters[it, 1]
             evals_p = _c.c_void_p(cbase + 16 * it + 8)
             ev = self._events()
+            select = False
             if update_frac < 0.5:
+                prepared = False  # the workspace serves other buckets
                 # converging path: FP32, full dimension, stored distances
                 if fp32_due:
                     call("umapb_nnd_gather", P(X), P(sq), n, d, P(idx), P(dist), k, 0, s)
@@ -348,8 +351,9 @@ class NNDescent:
                     dist0[id(Xd), use_half] = d0
                 ev[0].record() if ev else None
                 if join:
-                    call("umapb_nnd_join", P(src), P(sqd), dd, ldx, int(use_half), P(idx), P(order), n, k,
+                    call("umapb_nnd_join_prepared" if prepared and mc_nn == k else "umapb_nnd_join", P(src), P(sqd), dd, ldx, int(use_half), P(idx), P(order), n, k,
                          mc_nn, j_nn, P(nnbuf), P(curd), P(None), evals_p, P(join_ws), join_ws.numel(), s)
+                prepared = False
                 if select:
                     call("umapb_nnd_select", P(idx), P(dist), P(order), P(nnbuf), P(curd),
                          P(dist0[id(Xd), use_half] if use_rev else None), n, k, j_nn, int(recompute),
@@ -364,6 +368,11 @@ class NNDescent:
                     fp32_due = True
                 info = dict(path="full", mc_new=mc_nn, j_nn=j_nn, use_rev=use_rev, use_half=use_half, space=dd,
                             elem=2 if use_half else 4, join=join)
+            # the buckets of the next full iteration's join follow from the new lists alone: made
+            # while the host reads the count, unless the search is about to leave the full path
+            if select and update_frac >= 0.6 and it + 1 < self.n_iters:
+                call("umapb_nnd_join_prepare", P(idx2), P(order), n, k, k, P(join_ws), join_ws.numel(), s)
+                prepared = True
             if it == 0 and while_first_iteration is not None:
                 while_first_iteration()
             n_changed, n_evals = counters[it].tolist()  # the one host read per iteration

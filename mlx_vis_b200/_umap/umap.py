@@ -166,15 +166,16 @@ class UMAP:
         rows, cols, vals, n_edges = _lib.fuzzy(knn_idx, knn_dist, self.n_epochs, fp64=True)
         ev.mark("fuzzy")
 
-        a, b = find_ab_params(self.spread, self.min_dist)
-        self.a_, self.b_ = a, b
-
         if self.verbose:
             print("Initializing embedding...")
         self._spectral_ws = None
         self.init_used_ = self.init
         Y = self._init_embedding(Xd, rows, cols, vals, n_edges, n, seed, draws)
         ev.mark("init")
+        # the curve fit (host, about 0.4 ms of small least-squares solves) while the device
+        # works on the start: the layout follows the start without a gap
+        a, b = find_ab_params(self.spread, self.min_dist)
+        self.a_, self.b_ = a, b
 
         self._optimize(rows, cols, vals, n_edges, Y, a, b, n, seed, epoch_callback)
         ev.mark("layout")

@@ -108,13 +108,35 @@ __global__ void sqnorm_kernel(const T* __restrict__ X, int64_t n, int dd, float*
   if (lane == 0) sq[row] = acc;
 }
 
-// FP16 copy of (n, dd) FP32 rows into rows of pitch ldh >= dd, zero padded
-__global__ void to_half_kernel(const float* __restrict__ X, int64_t n, int dd, int ldh, __half* __restrict__ H) {
-  const int64_t m = n * ldh;
+// FP16 copy of (n, dd) FP32 rows into rows of pitch ldh >= dd, zero padded.  A thread makes
+// eight columns: two 16-byte loads (vec: rows that allow them) and, when the pitch is a
+// multiple of 8, one 16-byte store.  Bound by HBM: 70000 x 784 in 48 us against 140 with
+// a value and a division per thread.
+__global__ void to_half_kernel(const float* __restrict__ X, int64_t n, int dd, int ldh, int vec,
+                               __half* __restrict__ H) {
+  const int groups = (ldh + 7) / 8;
+  const int64_t m = n * groups;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = t / ldh;
-    const int c = (int)(t - r * ldh);
-    H[t] = c < dd ? __float2half_rn(X[r * dd + c]) : __float2half_rn(0.0f);
+    const int64_t r = t / groups;
+    const int c0 = (int)(t - r * groups) * 8;
+    const float* x = X + r * dd + c0;
+    __half* h = H + r * ldh + c0;
+    __align__(16) __half v[8];
+    if (vec && c0 + 8 <= dd) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(x)), b = __ldg(reinterpret_cast<const float4*>(x) + 1);
+      v[0] = __float2half_rn(a.x), v[1] = __float2half_rn(a.y), v[2] = __float2half_rn(a.z), v[3] = __float2half_rn(a.w);
+      v[4] = __float2half_rn(b.x), v[5] = __float2half_rn(b.y), v[6] = __float2half_rn(b.z), v[7] = __float2half_rn(b.w);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = c0 + u < dd ? __float2half_rn(__ldg(x + u)) : __float2half_rn(0.0f);
+    }
+    if ((ldh & 7) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0) {
+      *reinterpret_cast<uint4*>(h) = *reinterpret_cast<const uint4*>(v);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (c0 + u < ldh) h[u] = v[u];
+    }
   }
 }
 
@@ -455,17 +477,19 @@ __device__ __forceinline__ int entry_source(const int32_t* __restrict__ idx, con
   return srcs ? srcs[t] : idx[(t / mc) * k + (t % mc)];
 }
 
+// cnt[s] = entries of source s; rank[t] = the entry's place among them (any order), so that
+// the fill needs no counters of its own
 __global__ void src_count_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ srcs, int64_t n, int k,
-                                 int mc, int32_t* __restrict__ cnt) {
+                                 int mc, int32_t* __restrict__ cnt, int32_t* __restrict__ rank) {
   const int64_t m = n * mc;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
     const int sidx = entry_source(idx, srcs, t, k, mc);
-    if (sidx >= 0) atomicAdd(&cnt[sidx], 1);
+    if (sidx >= 0) rank[t] = atomicAdd(&cnt[sidx], 1);
   }
 }
 
 __global__ void src_fill_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ srcs, int64_t n, int k,
-                                int mc, const int32_t* __restrict__ off, int32_t* __restrict__ fill,
+                                int mc, const int32_t* __restrict__ off, const int32_t* __restrict__ rank,
                                 int32_t* __restrict__ entries) {
   const int64_t m = n * mc;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
@@ -473,7 +497,7 @@ __global__ void src_fill_kernel(const int32_t* __restrict__ idx, const int32_t* 
     if (sidx < 0) continue;
     const int64_t i = t / mc;
     const int p = (int)(t % mc);
-    entries[off[sidx] + atomicAdd(&fill[sidx], 1)] = (int32_t)(i * 32 + p);
+    entries[off[sidx] + rank[t]] = (int32_t)(i * 32 + p);
   }
 }
 
@@ -509,6 +533,7 @@ __global__ void chunk_count_kernel(const int32_t* __restrict__ off, const int32_
     const int64_t s = order ? order[r] : r;
     nch[r] = (off[s + 1] - off[s] + 15) >> 4;
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) nch[n] = 0;  // the scan's last value: the total
 }
 
 __global__ void chunk_fill_kernel(const int32_t* __restrict__ choff, int64_t n, int32_t* __restrict__ chunk_pos) {
@@ -1067,11 +1092,11 @@ extern "C" int umapb_nnd_to_half(const float* X, int64_t n, int32_t dd, int32_t 
                                  umapb_stream_t stream_) {
   clear_error();
   UMAPB_REQUIRE(X && H && n >= 0 && dd >= 1 && ldh >= dd, "nnd_to_half: bad arguments");
-  const int64_t count = n * ldh;
-  if (count == 0) return UMAPB_OK;
-  const int64_t want = ceil_div(count, 256);
-  const unsigned blocks = (unsigned)(want < num_sms() * 8 ? want : num_sms() * 8);
-  nnd::to_half_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(X, n, dd, ldh,
+  if (n == 0) return UMAPB_OK;
+  const int64_t want = ceil_div(n * ceil_div(ldh, 8), 256);
+  const unsigned blocks = (unsigned)(want < num_sms() * 16 ? want : num_sms() * 16);
+  const int vec = dd % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  nnd::to_half_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(X, n, dd, ldh, vec,
                                                                                     static_cast<__half*>(H));
   UMAPB_LAUNCH_CHECK("nnd_to_half kernel");
   count_launches(1);
@@ -1197,7 +1222,7 @@ extern "C" int umapb_nnd_reverse(const int32_t* idx, int64_t n, int32_t k, int32
 // The join's workspace; umapb_nnd_select reads its buckets afterwards.
 namespace {
 struct JoinWs {
-  int32_t *off, *fill, *entries, *choff, *chunk_pos, *srcs;
+  int32_t *off, *entries, *choff, *chunk_pos, *srcs;
   int64_t* total;  // total, then scan scratch at total + 8
   float* entd;
   int64_t max_chunks;
@@ -1210,14 +1235,13 @@ JoinWs join_carve(void* ws, int64_t n, int mc) {
   Carver c(ws);
   c.take<int32_t>(64);
   w.off = c.take<int32_t>((size_t)n + 1);   // source counts -> bucket offsets
-  w.fill = c.take<int32_t>((size_t)n + 1);  // fill counters
   w.entries = c.take<int32_t>(m);
   w.choff = c.take<int32_t>((size_t)n + 1);  // chunk counts -> chunk offsets
   w.max_chunks = n + n * mc / 16;            // sum of ceil(count / 16) <= n + n*mc/16
   w.chunk_pos = c.take<int32_t>((size_t)w.max_chunks + 1);  // chunk -> source
   w.total = c.take<int64_t>(8 + kScanMaxBlocks);
   w.srcs = c.take<int32_t>(m);  // the NEW-first source lists (umapb_nnd_join_new)
-  w.entd = c.take<float>(m);    // current-neighbour distances in bucket order
+  w.entd = c.take<float>(m);    // current-neighbour distances in bucket order (first the entries' ranks)
   w.bytes = c.bytes();
   return w;
 }
@@ -1230,12 +1254,39 @@ extern "C" int umapb_nnd_join_workspace(int64_t n, int32_t k, int32_t mc, size_t
   return UMAPB_OK;
 }
 
-// The blocked join over the sources idx_old[i][p < mc] or, with flags, over the
-// NEW-first source lists of the converging path (new_sources_kernel).
+// The join's buckets: (row, position) entries by source, over the sources idx_old[i][p < mc]
+// or, with flags, over the NEW-first source lists of the converging path
+// (new_sources_kernel), and the chunks of 16 entries in `order`.
+static int join_buckets(const int32_t* idx_old, const uint8_t* flags, const int32_t* order, int64_t n, int32_t k,
+                        int32_t mc, const JoinWs& w, cudaStream_t stream) {
+  const int64_t m = n * mc;
+  int32_t* rank = reinterpret_cast<int32_t*>(w.entd);
+  UMAPB_CUDA_TRY(cudaMemsetAsync(w.off, 0, sizeof(int32_t) * (n + 1), stream), "nnd_join: reset");
+  const int64_t want = ceil_div(m, 256);
+  const unsigned blocks = (unsigned)(want < num_sms() * 8 ? want : num_sms() * 8);
+  const int32_t* srcs = nullptr;
+  if (flags) {
+    nnd::new_sources_kernel<<<(unsigned)ceil_div(n * 32, 256), 256, 0, stream>>>(idx_old, flags, n, k, mc, w.srcs);
+    srcs = w.srcs;
+  }
+  nnd::src_count_kernel<<<blocks, 256, 0, stream>>>(idx_old, srcs, n, k, mc, w.off, rank);
+  scan_exclusive(w.off, n + 1, w.total, w.total + 8, stream);
+  nnd::src_fill_kernel<<<blocks, 256, 0, stream>>>(idx_old, srcs, n, k, mc, w.off, rank, w.entries);
+  const unsigned sblocks = (unsigned)ceil_div(n, 256);
+  nnd::chunk_count_kernel<<<sblocks, 256, 0, stream>>>(w.off, order, n, w.choff);
+  scan_exclusive(w.choff, n + 1, w.total, w.total + 8, stream);
+  nnd::chunk_fill_kernel<<<sblocks, 256, 0, stream>>>(w.choff, n, w.chunk_pos);
+  UMAPB_LAUNCH_CHECK("nnd_join bucket kernels");
+  count_launches(6 + (flags ? 1 : 0));
+  return UMAPB_OK;
+}
+
+// The blocked join; `prepared`: its buckets are in the workspace already.
 static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, int32_t half,
                      const int32_t* idx_old, const uint8_t* flags, const int32_t* order, int64_t n, int32_t k,
                      int32_t mc, int32_t j_nn, float* nnbuf, float* curd, int32_t* rev_out,
-                     unsigned long long* evals, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+                     unsigned long long* evals, bool prepared, void* workspace, size_t workspace_bytes,
+                     cudaStream_t stream) {
   UMAPB_REQUIRE(Xd && sqd && idx_old, "nnd_join: null array argument");
   UMAPB_REQUIRE(n >= 2 && dd >= 1 && ldx >= dd, "nnd_join: bad shape");
   UMAPB_REQUIRE(n < ((int64_t)1 << 26), "nnd_join: n must be below 2^26");
@@ -1252,43 +1303,24 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
   const JoinWs w = join_carve(workspace, n, mc);
   if (!workspace || workspace_bytes < w.bytes)
     return set_error(UMAPB_ERR_WORKSPACE, "nnd_join: workspace of %zu bytes, need %zu", workspace_bytes, w.bytes);
-  int32_t *off = w.off, *fill = w.fill, *entries = w.entries, *choff = w.choff, *chunk_pos = w.chunk_pos;
-  int32_t* srcs = w.srcs;
-  int64_t* total = w.total;
-  const int64_t max_chunks = w.max_chunks;
   if (mc == 0) return UMAPB_OK;
-  const int64_t m = n * mc;
-  UMAPB_CUDA_TRY(cudaMemsetAsync(off, 0, sizeof(int32_t) * (n + 1), stream), "nnd_join: reset");
-  UMAPB_CUDA_TRY(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (n + 1), stream), "nnd_join: reset");
-  const int64_t want = ceil_div(m, 256);
-  const unsigned blocks = (unsigned)(want < num_sms() * 8 ? want : num_sms() * 8);
-  if (flags)
-    nnd::new_sources_kernel<<<(unsigned)ceil_div(n * 32, 256), 256, 0, stream>>>(idx_old, flags, n, k, mc, srcs);
-  else
-    srcs = nullptr;
-  nnd::src_count_kernel<<<blocks, 256, 0, stream>>>(idx_old, srcs, n, k, mc, off);
-  scan_exclusive(off, n + 1, total, total + 8, stream);
-  nnd::src_fill_kernel<<<blocks, 256, 0, stream>>>(idx_old, srcs, n, k, mc, off, fill, entries);
+  if (!prepared)
+    if (const int rc = join_buckets(idx_old, flags, order, n, k, mc, w, stream)) return rc;
   if (rev_out) {  // with mc == k the buckets are the reverse-candidate buckets
     nnd::bucket_select_kernel<<<(unsigned)ceil_div(n, nnd::kWarps * nnd::kSelRows), nnd::kWarps * 32, 0,
-                                stream>>>(entries, off, nullptr, n, k, 5, rev_out);
+                                stream>>>(w.entries, w.off, nullptr, n, k, 5, rev_out);
   }
-  const unsigned sblocks = (unsigned)ceil_div(n, 256);
-  UMAPB_CUDA_TRY(cudaMemsetAsync(choff + n, 0, sizeof(int32_t), stream), "nnd_join: reset");
-  nnd::chunk_count_kernel<<<sblocks, 256, 0, stream>>>(off, order, n, choff);
-  scan_exclusive(choff, n + 1, total, total + 8, stream);
-  nnd::chunk_fill_kernel<<<sblocks, 256, 0, stream>>>(choff, n, chunk_pos);
   nnd::JoinArgs a;
   a.Xd = Xd;
   a.sqd = sqd;
   a.dd = dd;
   a.ldx = ldx;
   a.idx_old = idx_old;
-  a.off = off;
-  a.entries = entries;
+  a.off = w.off;
+  a.entries = w.entries;
   a.order = order;
-  a.choff = choff;
-  a.chunk_pos = chunk_pos;
+  a.choff = w.choff;
+  a.chunk_pos = w.chunk_pos;
   a.n = n;
   a.k = k;
   a.mc = mc;
@@ -1298,7 +1330,7 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
   a.curd = curd;
   a.entd = w.entd;
   a.evals = evals;
-  const unsigned jb = (unsigned)ceil_div(max_chunks, nnd::kWarps);  // warps past the chunk count exit
+  const unsigned jb = (unsigned)ceil_div(w.max_chunks, nnd::kWarps);  // warps past the chunk count exit
   if (half) {
     nnd::join_f16_kernel<<<jb, nnd::kWarps * 32, 0, stream>>>(a);
   } else {
@@ -1317,8 +1349,31 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
     nnd::join_f32_kernel<<<jb, nnd::kWarps * 32, jsmem, stream>>>(a);
   }
   UMAPB_LAUNCH_CHECK("nnd_join kernels");
-  count_launches((rev_out ? 8 : 7) + (flags ? 1 : 0));
+  count_launches(rev_out ? 2 : 1);
   return UMAPB_OK;
+}
+
+extern "C" int umapb_nnd_join_prepare(const int32_t* idx_old, const int32_t* order, int64_t n, int32_t k, int32_t mc,
+                                      void* workspace, size_t workspace_bytes, umapb_stream_t stream_) {
+  clear_error();
+  UMAPB_REQUIRE(idx_old, "nnd_join_prepare: null array argument");
+  UMAPB_REQUIRE(n >= 2 && n < ((int64_t)1 << 26), "nnd_join_prepare: need 2 <= n < 2^26");
+  UMAPB_REQUIRE(k >= 1 && k <= 32 && mc >= 1 && mc <= k, "nnd_join_prepare: need 1 <= mc <= k <= 32");
+  const JoinWs w = join_carve(workspace, n, mc);
+  if (!workspace || workspace_bytes < w.bytes)
+    return set_error(UMAPB_ERR_WORKSPACE, "nnd_join_prepare: workspace of %zu bytes, need %zu", workspace_bytes,
+                     w.bytes);
+  return join_buckets(idx_old, nullptr, order, n, k, mc, w, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int umapb_nnd_join_prepared(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, int32_t half,
+                                       const int32_t* idx_old, const int32_t* order, int64_t n, int32_t k, int32_t mc,
+                                       int32_t j_nn, float* nnbuf, float* curd, int32_t* rev_out,
+                                       unsigned long long* evals, void* workspace, size_t workspace_bytes,
+                                       umapb_stream_t stream_) {
+  clear_error();
+  return join_impl(Xd, sqd, dd, ldx, half, idx_old, nullptr, order, n, k, mc, j_nn, nnbuf, curd, rev_out, evals, true,
+                   workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int umapb_nnd_join(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, int32_t half,
@@ -1328,7 +1383,7 @@ extern "C" int umapb_nnd_join(const void* Xd, const float* sqd, int32_t dd, int3
                               size_t workspace_bytes, umapb_stream_t stream_) {
   clear_error();
   return join_impl(Xd, sqd, dd, ldx, half, idx_old, nullptr, order, n, k, mc, j_nn, nnbuf, curd, rev_out, evals,
-                   workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
+                   false, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int umapb_nnd_join_new(const float* X, const float* sq, int32_t dd, const int32_t* idx_old,
@@ -1338,7 +1393,7 @@ extern "C" int umapb_nnd_join_new(const float* X, const float* sq, int32_t dd, c
   clear_error();
   UMAPB_REQUIRE(flags_old, "nnd_join_new: null flags");
   return join_impl(X, sq, dd, dd, 0, idx_old, flags_old, order, n, k, mc, j_nn, nnbuf, nullptr, nullptr, evals,
-                   workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
+                   false, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int umapb_nnd_select(const int32_t* idx_old, const float* dist_old, const int32_t* order,
