@@ -304,31 +304,25 @@ __global__ void __launch_bounds__(kBlock) finish_orth_wide_kernel(const float* _
 // and keeps their edges (ids, weights and row offsets) in shared memory, as many as
 // fit, so that an iteration reads nothing but the gathered rows of V, which other blocks
 // write and which come through L2 (ld.global.cg).  One grid barrier ends an
-// iteration.
+// iteration.  R^-1 is applied to a row's sums, after the gather, so the block's last warp
+// factors the completed Gram matrix while the others gather; it has no rows.
 //
-// Orthonormalisation: V_{t+1} = W V_t spans the same space whether or not V_t was
-// orthonormalised first, and the triangular factors multiply up, so the columns after
-// any number of plain multiplications and one factorisation are those of a
-// factorisation at each step.  What limits the number of plain steps is the FP32
-// storage of V: a column whose own part shrinks by lambda per step keeps a relative
-// error of 2^-24 / lambda^m.  Each factorisation measures that shrinkage (the diagonal
-// of R) and the next one comes after 1, 2, 4 or 8 multiplications, the most for which
-// it stays above 0.05.  Every block factors the completed Gram matrix itself.
-//
-// What bounds it: n k random 16-byte reads of V from L2 an iteration (1.05 M of the 70,000-row
-// iteration's 6.6 us are 3.6 us at the measured random-access rate), then the barrier.
-// B200, 100 iterations, k = 15, 2 components: 70,000 rows 1072 -> 658 us against a
-// factorisation per iteration with the edges read from L2 and 4 blocks per SM in the
-// barrier.
+// What bounds it: n k random 16-byte reads of V from L2 an iteration (1.05 M of the
+// 70,000-row iteration's 7.7 us are 3.6 us at the measured random-access rate), then the
+// barrier.  B200, 100 iterations, k = 15, 2 components: 70,000 rows 1072 -> 768 us against
+// one thread's factorisation between the barrier and the gather, the edges read from L2
+// and 4 blocks per SM in the barrier.
+// (A factorisation every few iterations only, as the shrinkage of the columns allows, is
+// as exact but rounds V to FP32 in another basis; 25 layout epochs later that differs
+// visibly from a factorisation per iteration.)
 //
 // The barrier gives up after limit_ns (umapb_set_wait_limit_ns, 2 s by default), raises
 // a shared abort flag and the status word, and every block then returns.
 
-// R and its inverse in registers (KK a constant), one reciprocal per pivot; returns the
-// smallest pivot
+// the inverse of R in registers (KK a constant), one reciprocal square root per pivot
 template <int KK>
-__device__ __forceinline__ double chol_inverse_fixed(const double (&G)[KK * KK], double (&ri)[KK * KK]) {
-  double R[KK][KK], inv[KK], least = 0.0;
+__device__ __forceinline__ void chol_inverse_fixed(const double (&G)[KK * KK], double (&ri)[KK * KK]) {
+  double R[KK][KK], inv[KK];
 #pragma unroll
   for (int j = 0; j < KK; ++j) {
 #pragma unroll
@@ -341,9 +335,7 @@ __device__ __forceinline__ double chol_inverse_fixed(const double (&G)[KK * KK],
     double s = G[j * KK + j];
 #pragma unroll
     for (int p = 0; p < j; ++p) s -= R[p][j] * R[p][j];
-    R[j][j] = sqrt(fmax(s, 0.0) + 1e-10);
-    inv[j] = 1.0 / R[j][j];
-    least = j == 0 ? R[j][j] : fmin(least, R[j][j]);
+    inv[j] = rsqrt(fmax(s, 0.0) + 1e-10);  // the pivot itself is not needed
   }
 #pragma unroll
   for (int j = 0; j < KK; ++j) {
@@ -355,7 +347,6 @@ __device__ __forceinline__ double chol_inverse_fixed(const double (&G)[KK * KK],
       ri[i * KK + j] = (i <= j) ? s * inv[i] : 0.0;
     }
   }
-  return least;
 }
 
 __device__ __forceinline__ unsigned long long gtimer() {
@@ -392,15 +383,53 @@ __device__ bool grid_barrier(unsigned* bar, unsigned target, int* abort_g, unsig
   return s_ok != 0;
 }
 
-// multiplications until the next factorisation, from the least pivot after `step` of them
-__device__ __forceinline__ int plain_steps(double least, int step) {
-  int m = 1;
-  const float log_step = logf(fminf((float)least, 1.0f)) / (float)step;
-  while (m < 8 && 2.0f * (float)m * log_step > -2.9957f) m *= 2;  // log(0.05)
-  return m;
+// The upper triangle of a block's Gram matrix.  Both lanes of a row hold the same products, so
+// each sums half of the entries over its warp; warp e then adds entry e over the warps and holds it
+// in every lane.  (Every entry over all lanes and one thread's chain over 32 warps were
+// 0.2 us more of an iteration: 788 -> 768 us at 70,000 rows, 354 -> 325 us in the cluster at 2,000.)
+template <int KK>
+struct Upper {
+  static constexpr int kEntries = KK * (KK + 1) / 2, kHalf = (kEntries + 1) / 2;
+  static __host__ __device__ constexpr int at(int e) {  // entry e of the triangle in KK x KK
+    int i = 0;
+    while (e >= KK - i) {
+      e -= KK - i;
+      ++i;
+    }
+    return i * KK + i + e;
+  }
+};
+
+template <int KK, int WARPS>
+__device__ __forceinline__ double block_gram(const double (&part)[KK * KK], double (*gsum)[WARPS]) {
+  using U = Upper<KK>;
+  static_assert(U::kEntries <= WARPS && WARPS <= 32, "one warp per entry, one lane per warp");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = threadIdx.x & 1;
+  double tri[2 * U::kHalf];
+  tri[2 * U::kHalf - 1] = 0.0;
+#pragma unroll
+  for (int i = 0, e = 0; i < KK; ++i)
+#pragma unroll
+    for (int j = i; j < KK; ++j, ++e) tri[e] = part[i * KK + j];
+#pragma unroll
+  for (int h = 0; h < U::kHalf; ++h) {
+    double g = sub ? tri[U::kHalf + h] : tri[h];
+#pragma unroll
+    for (int o = 16; o > 1; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    if (lane < 2 && sub * U::kHalf + h < U::kEntries) gsum[sub * U::kHalf + h][warp] = g;
+  }
+  __syncthreads();
+  double g = 0.0;
+  if (warp < U::kEntries) {
+    g = lane < WARPS ? gsum[warp][lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+  }
+  return g;
 }
 
-constexpr int kPowerThreads = 1024;  // two lanes for each of 512 rows: one pass up to 75,000 rows
+constexpr int kPowerThreads = 1024;  // two lanes for each of 496 rows (one pass up to 73,408 rows) and the factor warp
+constexpr int kPowerRowThreads = kPowerThreads - 32;
 constexpr size_t kPowerSmem = 200 * 1024;  // dynamic shared memory at most
 
 template <int KK>  // columns of V: n_components + 1
@@ -417,8 +446,7 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
   int32_t* s_col = s_off + off_cap;                         // edge_cap ids
   float* s_w = reinterpret_cast<float*>(s_col + edge_cap);  // edge_cap weights
   __shared__ double ri[KK * KK];
-  __shared__ double gsum[kWarps][KK * KK];
-  __shared__ int s_next;
+  __shared__ double gsum[Upper<KK>::kEntries][kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = threadIdx.x & (kLanes - 1);
   const int64_t r_first = (int64_t)blockIdx.x * rows_per_block;
@@ -438,21 +466,34 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
   wn += e_first;
   __syncthreads();
 
-  bool rotate = false;       // apply R^-1 of the factorisation just made
-  int step = 0, every = 1;   // multiplications since the last factorisation; the next one after `every`
-  int factored = 0;
-  for (int it = 0; it < n_iter; ++it) {
+  for (int it = 0; it <= n_iter; ++it) {
+    // the factor warp: R^-1 of the previous iteration's product, for this one's rows
+    if (warp == kWarps - 1 && it > 0) {
+      const double* Gp = G + (size_t)(it - 1) * KK * KK;
+      const double mine = lane < KK * KK ? __ldcg(Gp + lane) : 0.0;
+      double Gl[KK * KK], rl[KK * KK];
+#pragma unroll
+      for (int t = 0; t < KK * KK; ++t) Gl[t] = __shfl_sync(0xffffffffu, mine, t);  // the upper triangle counts
+      chol_inverse_fixed<KK>(Gl, rl);
+      if (lane == 0) {
+#pragma unroll
+        for (int t = 0; t < KK * KK; ++t) ri[t] = rl[t];
+        if (blockIdx.x == 0)
+          for (int t = 0; t < KK * KK; ++t) Rinv[(size_t)(it - 1) * KK * KK + t] = rl[t];
+      }
+    }
+    if (it == n_iter) break;
     const float* Vin = (it & 1) ? V1 : V0;
     float* Vout = (it & 1) ? V0 : V1;
-    const bool factor = ++step == every || it == n_iter - 1;
     double part[KK * KK];
 #pragma unroll
     for (int t = 0; t < KK * KK; ++t) part[t] = 0.0;
-    // the loop bound is the warp's first row, so every lane of a warp makes the
-    // same passes and meets the shuffle below; rows past the last do no work
-    for (int w0 = warp * (32 / kLanes); w0 < rows; w0 += kPowerThreads / kLanes) {
+    // every warp takes the first pass (R^-1 is ready after it) and then the passes that begin at
+    // a row of the block, so its lanes meet the shuffle below; rows past the last do no work
+    bool first = true;
+    for (int w0 = warp * (32 / kLanes); first || w0 < rows; w0 += kPowerRowThreads / kLanes) {
       const int lr = w0 + lane / kLanes;
-      const bool valid = lr < rows;
+      const bool valid = lr < rows && warp < kWarps - 1;
       double acc[KK];
 #pragma unroll
       for (int j = 0; j < KK; ++j) acc[j] = 0.0;
@@ -487,12 +528,14 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
       }
 #pragma unroll
       for (int j = 0; j < KK; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);  // kLanes == 2
-      if (valid && sub == 0) {
+      if (first) __syncthreads();  // R^-1
+      first = false;
+      if (valid) {
         double q[KK];
 #pragma unroll
         for (int j = 0; j < KK; ++j) {
           q[j] = acc[j];
-          if (rotate) {
+          if (it > 0) {
             q[j] = 0.0;
 #pragma unroll
             for (int i = 0; i <= j; ++i) q[j] += acc[i] * ri[i * KK + j];
@@ -502,61 +545,21 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
 #pragma unroll
         for (int j = 0; j < vp; ++j) out[j] = j < KK ? (float)q[j < KK ? j : 0] : 0.f;
         float4* dst = reinterpret_cast<float4*>(Vout + (r_first + lr) * vp);
-        dst[0] = make_float4(out[0], out[1], out[2], out[3]);
-        if constexpr (vp == 8) dst[1] = make_float4(out[4], out[5], out[6], out[7]);
-        if (factor) {
+        if (sub == 0) dst[0] = make_float4(out[0], out[1], out[2], out[3]);
+        if constexpr (vp == 8)
+          if (sub == 1) dst[1] = make_float4(out[4], out[5], out[6], out[7]);
 #pragma unroll
-          for (int i = 0; i < KK; ++i)
+        for (int i = 0; i < KK; ++i)
 #pragma unroll
-            for (int j = i; j < KK; ++j) part[i * KK + j] += q[i] * q[j];
-        }
+          for (int j = i; j < KK; ++j) part[i * KK + j] += q[i] * q[j];
       }
     }
-    double* Git = G + (size_t)it * KK * KK;
-    if (factor) {
-      // block reduction of the Gram partials, then one atomic per entry and block
-#pragma unroll
-      for (int i = 0; i < KK; ++i) {
-#pragma unroll
-        for (int j = i; j < KK; ++j) {
-          double g = part[i * KK + j];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-          if (lane == 0) gsum[warp][i * KK + j] = g;
-        }
-      }
-      __syncthreads();
-      if (threadIdx.x < KK * KK) {
-        const int i = threadIdx.x / KK, j = threadIdx.x % KK;
-        if (i <= j) {
-          double g = 0.0;
-          for (int w = 0; w < kWarps; ++w) g += gsum[w][i * KK + j];
-          atomicAdd(&Git[i * KK + j], g);
-        }
-      }
-    }
+    // one atomic per entry and block
+    const double gram = block_gram<KK, kWarps>(part, gsum);
+    if (warp < Upper<KK>::kEntries && lane == 0) atomicAdd(G + (size_t)it * KK * KK + Upper<KK>::at(warp), gram);
     if (!grid_barrier(bar, (unsigned)(it + 1) * gridDim.x, abort_g, limit_ns)) {
       if (threadIdx.x == 0) atomicExch(status, (int32_t)kDevTimeoutEpilogue);
       return;
-    }
-    rotate = factor;
-    if (factor) {
-      if (threadIdx.x == 0) {
-        double Gl[KK * KK], rl[KK * KK];
-#pragma unroll
-        for (int t = 0; t < KK * KK; ++t) Gl[t] = __ldcg(Git + t);  // the upper triangle
-        const double least = chol_inverse_fixed<KK>(Gl, rl);
-#pragma unroll
-        for (int t = 0; t < KK * KK; ++t) ri[t] = rl[t];
-        if (blockIdx.x == 0)
-          for (int t = 0; t < KK * KK; ++t) Rinv[(size_t)it * KK * KK + t] = rl[t];
-        // the least a column shrank per multiplication; V0's norm says nothing, nor does its first product
-        s_next = factored > 0 ? plain_steps(least, step) : 1;
-      }
-      __syncthreads();
-      every = s_next;
-      step = 0;
-      ++factored;
     }
   }
 }
@@ -565,11 +568,11 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
 // buffers) in its shared memory, computes its share of the rows and stores them into
 // all eight copies, so an iteration gathers from its own shared memory and ends with the
 // cluster's hardware barrier.  The CTAs' Gram matrices are exchanged the same way and
-// added in rank order, without atomics.  B200, 2,000 rows, k = 15: 284 us against 400 us
-// on 16 blocks of the grid-wide form (613 us at a factorisation per iteration), where
-// every iteration pays an L2 round trip each for V and for the barrier.
+// added in rank order, without atomics.  B200, 2,000 rows, k = 15: 613 -> 325 us against 16
+// blocks over L2, where every iteration pays a round trip each for V and the barrier.
 constexpr int kClusterCtas = 8;
-constexpr int kClusterThreads = 512;
+constexpr int kClusterThreads = 544;  // 16 warps with rows and the factor warp
+constexpr int kClusterRowThreads = kClusterThreads - 32;
 constexpr size_t kClusterSmem = 216 * 1024;
 constexpr size_t kClusterVBytes = 160 * 1024;  // both buffers of V: up to 5,120 rows of 16 bytes
 
@@ -587,9 +590,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   int32_t* s_col = s_off + rows_per_cta + 1;
   float* s_w = reinterpret_cast<float*>(s_col + edge_cap);
   __shared__ double ri[KK * KK];
-  __shared__ double gsum[kWarps][KK * KK];
-  __shared__ double parts[2][kClusterCtas][KK * KK];  // the CTAs' Gram matrices, by parity of the factorisation
-  __shared__ int s_next;
+  __shared__ double gsum[Upper<KK>::kEntries][kWarps];
+  __shared__ double parts[2][kClusterCtas][KK * KK];  // the CTAs' Gram matrices, by parity of the iteration
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = threadIdx.x & (kLanes - 1);
   const int rank = (int)cluster::rank();
@@ -612,18 +614,33 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   // every CTA runs and has read V0 before its neighbours store into its copy
   cluster::barrier();
 
-  bool rotate = false;
-  int step = 0, every = 1, factored = 0;
-  for (int it = 0; it < n_iter; ++it) {
+  for (int it = 0; it <= n_iter; ++it) {
+    // the factor warp: R^-1 of the previous iteration's product, for this one's rows
+    if (warp == kWarps - 1 && it > 0) {
+      const int t0 = lane < KK * KK ? lane : 0;
+      double mine = 0.0;
+      for (int p = 0; p < kClusterCtas; ++p) mine += parts[(it - 1) & 1][p][t0];
+      double Gl[KK * KK], rl[KK * KK];
+#pragma unroll
+      for (int t = 0; t < KK * KK; ++t) Gl[t] = __shfl_sync(0xffffffffu, mine, t);  // the upper triangle counts
+      chol_inverse_fixed<KK>(Gl, rl);
+      if (lane == 0) {
+#pragma unroll
+        for (int t = 0; t < KK * KK; ++t) ri[t] = rl[t];
+        if (rank == 0)
+          for (int t = 0; t < KK * KK; ++t) Rinv[(size_t)(it - 1) * KK * KK + t] = rl[t];
+      }
+    }
+    if (it == n_iter) break;
     const float4* Vin = v_all + (it & 1) * v_words;
     const uint32_t out_at = v_at + (uint32_t)(((it + 1) & 1) * v_words) * 16u;
-    const bool factor = ++step == every || it == n_iter - 1;
     double part[KK * KK];
 #pragma unroll
     for (int t = 0; t < KK * KK; ++t) part[t] = 0.0;
-    for (int w0 = warp * (32 / kLanes); w0 < rows; w0 += kClusterThreads / kLanes) {
+    bool first = true;  // every warp takes the first pass: R^-1 is ready after it
+    for (int w0 = warp * (32 / kLanes); first || w0 < rows; w0 += kClusterRowThreads / kLanes) {
       const int lr = w0 + lane / kLanes;
-      const bool valid = lr < rows;
+      const bool valid = lr < rows && warp < kWarps - 1;
       double acc[KK];
 #pragma unroll
       for (int j = 0; j < KK; ++j) acc[j] = 0.0;
@@ -656,12 +673,14 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       }
 #pragma unroll
       for (int j = 0; j < KK; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);  // kLanes == 2
+      if (first) __syncthreads();  // R^-1
+      first = false;
       if (valid) {  // both lanes hold the sums: each stores the row into half of the copies
         double q[KK];
 #pragma unroll
         for (int j = 0; j < KK; ++j) {
           q[j] = acc[j];
-          if (rotate) {
+          if (it > 0) {
             q[j] = 0.0;
 #pragma unroll
             for (int i = 0; i <= j; ++i) q[j] += acc[i] * ri[i * KK + j];
@@ -682,60 +701,19 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                          "f"(out[6]), "f"(out[7])
                          : "memory");
         }
-        if (factor && sub == 0) {
 #pragma unroll
-          for (int i = 0; i < KK; ++i)
+        for (int i = 0; i < KK; ++i)
 #pragma unroll
-            for (int j = i; j < KK; ++j) part[i * KK + j] += q[i] * q[j];
-        }
+          for (int j = i; j < KK; ++j) part[i * KK + j] += q[i] * q[j];
       }
     }
-    const int parity = factored & 1;
-    if (factor) {
-#pragma unroll
-      for (int i = 0; i < KK; ++i) {
-#pragma unroll
-        for (int j = i; j < KK; ++j) {
-          double g = part[i * KK + j];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
-          if (lane == 0) gsum[warp][i * KK + j] = g;
-        }
-      }
-      __syncthreads();
-      if (threadIdx.x < KK * KK && threadIdx.x / KK <= threadIdx.x % KK) {
-        double g = 0.0;
-        for (int w = 0; w < kWarps; ++w) g += gsum[w][threadIdx.x];
-        const uint32_t at = parts_at + (uint32_t)((parity * kClusterCtas + rank) * KK * KK + (int)threadIdx.x) * 8u;
-#pragma unroll
-        for (int p = 0; p < kClusterCtas; ++p)
-          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster::peer(at, (uint32_t)p)), "d"(g) : "memory");
-      }
+    const double gram = block_gram<KK, kWarps>(part, gsum);
+    if (warp < Upper<KK>::kEntries && lane < kClusterCtas) {
+      const uint32_t at = parts_at + (uint32_t)(((it & 1) * kClusterCtas + rank) * KK * KK + Upper<KK>::at(warp)) * 8u;
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster::peer(at, (uint32_t)lane)), "d"(gram) : "memory");
     }
     __syncwarp();
     cluster::barrier();
-    rotate = factor;
-    if (factor) {
-      if (threadIdx.x == 0) {
-        double Gl[KK * KK], rl[KK * KK];
-#pragma unroll
-        for (int t = 0; t < KK * KK; ++t) {
-          Gl[t] = 0.0;
-          if (t / KK <= t % KK)
-            for (int p = 0; p < kClusterCtas; ++p) Gl[t] += parts[parity][p][t];
-        }
-        const double least = chol_inverse_fixed<KK>(Gl, rl);
-#pragma unroll
-        for (int t = 0; t < KK * KK; ++t) ri[t] = rl[t];
-        if (rank == 0)
-          for (int t = 0; t < KK * KK; ++t) Rinv[(size_t)it * KK * KK + t] = rl[t];
-        s_next = factored > 0 ? plain_steps(least, step) : 1;
-      }
-      __syncthreads();
-      every = s_next;
-      step = 0;
-      ++factored;
-    }
   }
   float4* out = reinterpret_cast<float4*>((n_iter & 1) ? V1 : V0) + (int64_t)r_first * (vp / 4);
   const float4* mine = v_all + (n_iter & 1) * v_words + r_first * (vp / 4);
@@ -1034,7 +1012,7 @@ extern "C" int umapb_spectral(const int32_t* rows, const int32_t* cols, const fl
                      : kk == 3 ? (const void*)spectral::power_kernel<3>
                      : kk == 4 ? (const void*)spectral::power_kernel<4>
                                : (const void*)spectral::power_kernel<5>;
-    const int64_t min_rows = spectral::kPowerThreads / spectral::kLanes / 2;
+    const int64_t min_rows = spectral::kPowerRowThreads / spectral::kLanes / 2;
     int64_t grid = ceil_div(n, min_rows);
     if (grid > num_sms()) grid = num_sms();
     int per = (int)ceil_div(n, grid);
