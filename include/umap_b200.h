@@ -313,7 +313,10 @@ int umapb_spectral_fallback(const void* workspace, float* Y, int64_t n, int32_t 
  *   reference's host schedule.  Each epoch reads the epoch-start Y and
  *   accumulates all moves before applying them (the reference's synchronous
  *   scatter-add semantics).  Negative tails come from a counter-based Philox
- *   stream keyed by (seed, epoch, edge, sample).
+ *   stream keyed by (seed, epoch, edge, sample).  Four or more epochs whose Y and
+ *   edge shares fit the SMs' shared memory run in one launch; the first 32-bit word
+ *   of the workspace (zeroed by umapb_layout_prepare) is then 3 after a grid barrier
+ *   that waited more than 2 s, and Y is not valid.
  * umapb_layout_epoch_injected: one epoch whose negative tails are given in the
  *   reference's order (sample j pairs head ef[j % A] with neg_to[j], A = number
  *   of active edges, umap.py:433-436); neg_count must equal neg_rate * A.

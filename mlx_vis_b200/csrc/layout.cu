@@ -302,23 +302,28 @@ __global__ void apply_kernel(float* __restrict__ Y, float* __restrict__ dY, int6
   }
 }
 
-// ---- few edges: all epochs in one launch of one cluster --------------------------
-// Two launches per epoch cost more than the work of a few thousand due edges (2,000 points:
-// 6.5 us an epoch, most of it launches and L2 round trips).  Here one cluster keeps everything
-// on chip for all epochs: every CTA a copy of Y and an equal share of the edges (schedule,
-// ids).  An epoch is: queue the due edges; gather from the own copy of Y, add the moves to
-// dY in L2; cluster barrier; every CTA adds all of dY to its copy.  dY is one of three arrays
+// ---- few rows: all epochs in one launch ------------------------------------------
+// Two launches per epoch cost more than the work of a few thousand due edges (6.7 to 8.3 us an
+// epoch from 2,000 to 10,000 points, most of it launches and L2 round trips).  Here every CTA
+// keeps a copy of Y and an equal share of the edges (schedule, ids) in shared memory for
+// all epochs.  An epoch is: queue the due edges; gather from the own copy of Y, add the moves to
+// dY in L2; barrier; every CTA adds all of dY to its copy.  dY is one of three arrays
 // in turn: while an epoch adds to one, a CTA may still be reading the previous one, and the
-// next one, which every CTA has read before the last barrier, is cleared.  The draws and the pair math are those of the launches.
+// next one, which every CTA has read before the last barrier, is cleared.  The draws and
+// the pair math are those of the launches.
+// Up to kClusterEdges edges the CTAs are one cluster of 16 and the barrier is the
+// cluster's; beyond, a resident grid with a barrier in L2 (bounded: 2 s, then the
+// status word), since the pair math of more edges wants more SMs.  Either form needs Y
+// and the share in one SM's shared memory (about 22,000 rows of two components).
+// B200, per epoch, k = 15 where not said: 600 points, k = 5 8.0 -> 3.4 us (3.9 as a grid);
+// 1,000 points 4.0 either way; 2,000 points 6.7 -> 4.1 us (5.3 as a cluster); 4,000 points
+// 6.9 -> 4.8; 9,999 points, k = 10 8.4 -> 5.9; 20,000 points 9.8 -> 8.8.
 // (Moves added in the owners' shared memory took 23 us an epoch: float adds there are
 // compare-and-swap loops, remote ones a round trip a try.  Owners that apply their rows and
-// store them into all copies need a second barrier: 6.3 us.)  What bounds it: the
-// pair math on the cluster's SMs, so it serves up to kClusterEdges edges; beyond, the
-// whole chip is faster (60,000 edges: 8.5-10 us on a cluster, 7-8 by launches).  B200, per
-// epoch: 600 points, k = 5 8.0 -> 3.3 us; 2,000 points, k = 15 6.7 -> 5.2 us.
+// store them into all copies need a second barrier: 6.3 us.)
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterMax = 16;             // CTAs; 8 where 16 cannot be scheduled together
-constexpr int64_t kClusterEdges = 32768;
+constexpr int64_t kClusterEdges = 12288;
 constexpr size_t kClusterSmem = 216 * 1024;
 
 struct ClusterArgs {
@@ -332,11 +337,50 @@ struct ClusterArgs {
   int cap;       // edges per CTA
   float a, b, m2ab, two_b, lr;
   uint32_t k0, k1;
+  unsigned* bar;  // grid form: barrier counter, zero at launch
+  int* abort_g;
+  int32_t* status;
+  unsigned long long limit_ns;
 };
+
+__device__ __forceinline__ unsigned long long gtimer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Barrier of the resident grid; false once it has waited limit_ns or another block has.
+__device__ __forceinline__ bool grid_barrier(const ClusterArgs& a, unsigned target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    // the block's writes are ordered before this by the block barrier
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    const unsigned long long t0 = gtimer();
+    for (unsigned i = 1;; ++i) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+      if (v >= target) break;
+      if ((i & 255) == 0 && *(volatile int*)a.abort_g) {
+        ok = 0;
+        break;
+      }
+      if (gtimer() - t0 > a.limit_ns) {
+        atomicExch(a.abort_g, 1);
+        ok = 0;
+        break;
+      }
+    }
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
 
 static size_t cluster_smem(int64_t n, int dim, int cap) { return 4 * (size_t)n * dim + (size_t)cap * 14 + 64; }
 
-template <int DIM, int NEG>
+template <int DIM, int NEG, bool GRID>
 __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(ClusterArgs a) {
   extern __shared__ __align__(16) unsigned char layout_smem[];
   float* sy = reinterpret_cast<float*>(layout_smem);  // Y
@@ -347,7 +391,17 @@ __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(Clus
   __shared__ int s_due;
   const int tid = threadIdx.x, lane = tid & 31;
   const unsigned below = (1u << lane) - 1u;
-  const int rank = (int)cluster::rank(), ctas = (int)cluster::size();
+  const int rank = GRID ? (int)blockIdx.x : (int)cluster::rank(), ctas = GRID ? (int)gridDim.x : (int)cluster::size();
+  unsigned meetings = 0;
+  auto meet = [&]() {
+    if constexpr (GRID) {
+      return grid_barrier(a, ++meetings * gridDim.x);
+    } else {
+      __syncwarp();
+      cluster::barrier();
+      return true;
+    }
+  };
   const int64_t E = *a.n_edges < (int64_t)a.cap * ctas ? *a.n_edges : (int64_t)a.cap * ctas;
   const int per = (int)((E + ctas - 1) / ctas);
   const int64_t e0 = (int64_t)rank * per;
@@ -373,8 +427,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(Clus
     }
   };
   if (tid == 0) s_due = 0;
-  __syncwarp();
-  cluster::barrier();  // the first array is zero
+  bool ok = meet();  // the first array is zero
 
   Params p;
   p.a = a.a;
@@ -436,13 +489,14 @@ __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(Clus
       atomic_add_row<DIM>(dY, (int)i, acc);
     }
     for (int t = tid; t < own * DIM; t += kClusterThreads) __stcg(next_dY + r0 * DIM + t, 0.f);
-    __syncwarp();
-    cluster::barrier();  // all moves have been added, and the next array is zero
+    ok = meet();  // all moves have been added, and the next array is zero
+    if (!ok) break;
     if (tid == 0) s_due = 0;
     for (int t = tid; t < values; t += kClusterThreads) sy[t] = __fadd_rn(sy[t], __ldcg(dY + t));
     turn = then;
     __syncthreads();
   }
+  if (!ok && tid == 0) atomicExch(a.status, (int32_t)kDevTimeoutEpilogue);
   for (int t = tid; t < m; t += kClusterThreads) a.next[e0 + t] = s_next[t];
   for (int t = tid; t < own * DIM; t += kClusterThreads) a.Y[r0 * DIM + t] = sy[r0 * DIM + t];
 }
@@ -760,6 +814,51 @@ static void launch_injected(const Layout& l, float* Y, int64_t n, const int32_t*
   apply_kernel<<<(unsigned)ceil_div(m, kBlock), kBlock, 0, stream>>>(Y, l.dY, m);
 }
 
+// Enqueues epochs [begin, end) on a resident grid, one CTA per SM at most and at least 256
+// edges each (a smaller barrier); false: as launch_cluster.
+template <int DIM, int NEG>
+static bool launch_grid(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
+  static std::mutex mu;
+  static int known[64] = {0};  // 1: cooperative launches of the kernel work on this device; -1: not
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  const void* kernel = (const void*)layout_cluster_kernel<DIM, NEG, true>;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[dev] == 0) {
+      int coop = 0, per_sm = 0;
+      known[dev] = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+                           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)kClusterSmem) == cudaSuccess &&
+                           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kClusterThreads,
+                                                                         kClusterSmem) == cudaSuccess &&
+                           per_sm > 0
+                       ? 1
+                       : -1;
+      cudaGetLastError();
+    }
+    if (known[dev] < 0) return false;
+  }
+  int64_t ctas = ceil_div(e_cap, 256);
+  if (ctas > num_sms()) ctas = num_sms();
+  a.rows_per = (int)ceil_div(a.n, ctas);
+  a.cap = (int)ceil_div(e_cap, ctas);
+  const size_t smem = cluster_smem(a.n, DIM, a.cap);
+  if (smem > kClusterSmem || a.cap > 65535) return false;
+  if (cudaMemsetAsync(a.abort_g, 0, reinterpret_cast<char*>(a.bar + 1) - reinterpret_cast<char*>(a.abort_g), stream) !=
+      cudaSuccess) {  // the status word is cleared by umapb_layout_prepare
+    cudaGetLastError();
+    return false;
+  }
+  void* args[] = {&a};
+  if (cudaLaunchCooperativeKernel(kernel, dim3((unsigned)ctas), dim3(kClusterThreads), args, smem, stream) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
 // Enqueues epochs [begin, end) on one cluster; false: the problem does not fit one, or the
 // device cannot schedule one (the launches serve it then).
 template <int DIM, int NEG>
@@ -768,7 +867,7 @@ static bool launch_cluster(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
   static int known[64] = {0};  // CTAs per cluster on this device; 0 unknown, -1 none
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  const auto kernel = layout_cluster_kernel<DIM, NEG>;
+  const auto kernel = layout_cluster_kernel<DIM, NEG, false>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -810,6 +909,12 @@ static bool launch_cluster(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
   return true;
 }
 
+template <int DIM, int NEG>
+static bool launch_resident(const ClusterArgs& a, int64_t e_cap, cudaStream_t stream) {
+  return (e_cap <= kClusterEdges && launch_cluster<DIM, NEG>(a, e_cap, stream)) ||
+         launch_grid<DIM, NEG>(a, e_cap, stream);
+}
+
 }  // namespace layout
 }  // namespace umapb
 
@@ -832,7 +937,9 @@ extern "C" int umapb_layout_prepare(const float* vals, const int64_t* n_edges, i
   UMAPB_REQUIRE(n_epochs >= 1, "layout_prepare: n_epochs must be >= 1");
   UMAPB_REQUIRE(workspace && workspace_bytes >= 512, "layout_prepare: workspace too small");
   layout::Layout l = layout::carve(workspace, 1, 1, 1);  // status and wmax sit at fixed offsets
-  UMAPB_CUDA_TRY(cudaMemsetAsync(l.wmax, 0, 4, stream), "layout_prepare: reset");
+  UMAPB_CUDA_TRY(cudaMemsetAsync(l.status, 0, reinterpret_cast<char*>(l.wmax + 1) - reinterpret_cast<char*>(l.status),
+                                 stream),
+                 "layout_prepare: reset");
   const unsigned g = layout::edge_grid(e_cap);
   layout::max_kernel<<<g, layout::kBlock, 0, stream>>>(vals, n_edges, l.wmax);
   layout::eps_kernel<<<g, layout::kBlock, 0, stream>>>(vals, n_edges, l.wmax, n_epochs, eps, next);
@@ -864,11 +971,16 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
                             int32_t neg_rate, uint64_t seed, void* workspace, cudaStream_t stream) {
   // below four epochs the load of the edges and the store of their schedule cost more than the
   // launches (a callback after every epoch runs them one by one)
-  if (dim > 4 || n >= layout::kClusterRows || e_cap > layout::kClusterEdges || epoch_end - epoch_begin < 4) return false;
+  if (dim > 4 || n >= layout::kClusterRows || epoch_end - epoch_begin < 4) return false;
   const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
   layout::ClusterArgs c = {};
+  const layout::Layout l = layout::carve(workspace, n, dim, e_cap);
   c.Y = Y;
-  c.dY = layout::carve(workspace, n, dim, e_cap).dY;
+  c.dY = l.dY;
+  c.status = l.status;
+  c.abort_g = l.status + 32;
+  c.bar = reinterpret_cast<unsigned*>(l.status + 48);
+  c.limit_ns = 2000000000ull;
   c.rows = rows;
   c.cols = cols;
   c.eps = eps;
@@ -889,10 +1001,10 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
   const bool five = neg_rate == 5;
   bool ok = false;
   switch (dim) {
-    case 1: ok = layout::launch_cluster<1, 0>(c, e_cap, stream); break;
-    case 2: ok = five ? layout::launch_cluster<2, 5>(c, e_cap, stream) : layout::launch_cluster<2, 0>(c, e_cap, stream); break;
-    case 3: ok = five ? layout::launch_cluster<3, 5>(c, e_cap, stream) : layout::launch_cluster<3, 0>(c, e_cap, stream); break;
-    default: ok = layout::launch_cluster<4, 0>(c, e_cap, stream); break;
+    case 1: ok = layout::launch_resident<1, 0>(c, e_cap, stream); break;
+    case 2: ok = five ? layout::launch_resident<2, 5>(c, e_cap, stream) : layout::launch_resident<2, 0>(c, e_cap, stream); break;
+    case 3: ok = five ? layout::launch_resident<3, 5>(c, e_cap, stream) : layout::launch_resident<3, 0>(c, e_cap, stream); break;
+    default: ok = layout::launch_resident<4, 0>(c, e_cap, stream); break;
   }
   if (ok) count_launches(1);
   return ok;

@@ -312,13 +312,15 @@ def test_fuzzy_lanes_match_float64(n, k):
 
 
 @pytest.mark.parametrize("n,k,dim,neg", [(2, 1, 2, 5), (17, 3, 1, 5), (513, 7, 2, 5), (700, 9, 3, 5), (300, 5, 4, 2),
-                                         (2000, 15, 2, 0), (1025, 11, 2, 11), (3276, 10, 2, 5), (20, 1600, 2, 5)])
+                                         (2000, 15, 2, 0), (1025, 11, 2, 11), (1228, 10, 2, 5), (1229, 10, 2, 5), (4000, 9, 1, 5),
+                                         (20, 1600, 2, 5), (3000, 20, 4, 3), (20000, 15, 2, 5), (13001, 15, 3, 5)])
 @pytest.mark.parametrize("graph", [False, True])
-def test_layout_cluster_matches_launches(n, k, dim, neg, graph):
-    """Epochs 3 to 12 on one cluster against the same epochs one call each (the launches):
-    the same due edges and draws; a small step keeps the sums' order from growing.  Row
-    counts around a power of two per CTA, every narrow dimension, no and many negatives,
-    the largest number of edges and an uneven last share; the schedule goes on after it."""
+def test_layout_resident_forms_match_launches(n, k, dim, neg, graph):
+    """Epochs 3 to 12 in one launch (a cluster up to 12,288 edges, a resident grid beyond)
+    against the same epochs one call each (the launches): the same due edges and draws; a
+    small step keeps the sums' order from growing.  Either side of the border, every narrow
+    dimension, no and many negatives, the largest row count and an uneven last share; the
+    schedule goes on after it."""
     from mlx_vis_b200 import _lib
 
     rng = np.random.default_rng(n + k)
