@@ -38,7 +38,12 @@ namespace layout {
 
 constexpr int kBlock = 256;
 constexpr int kEdgesPerBlock = 1024;
-constexpr int64_t kClusterRows = 65536;  // the cluster form: row ids of 16 bits
+constexpr size_t kClusterSmem = 216 * 1024;
+
+// one launch for all epochs: row ids of 16 bits, a copy of Y in one SM's shared memory
+static bool resident_rows(int64_t n, int dim) {
+  return dim <= 4 && n < 65536 && 4 * n * dim + 64 <= (int64_t)kClusterSmem;
+}
 #ifndef UMAPB_LAYOUT_BLOCKS_PER_SM
 #define UMAPB_LAYOUT_BLOCKS_PER_SM 4
 #endif
@@ -324,7 +329,6 @@ __global__ void apply_kernel(float* __restrict__ Y, float* __restrict__ dY, int6
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterMax = 16;             // CTAs; 8 where 16 cannot be scheduled together
 constexpr int64_t kClusterEdges = 12288;
-constexpr size_t kClusterSmem = 216 * 1024;
 
 struct ClusterArgs {
   float *Y, *dY;  // dY: three arrays of n * DIM
@@ -735,7 +739,7 @@ static Layout carve(void* ws, int64_t n, int dim, int64_t e_cap) {
   Layout l;
   l.status = c.take<int32_t>(64);
   l.wmax = c.take<float>(64);
-  l.dY = c.take<float>((size_t)n * dim * (n < kClusterRows && dim <= 4 ? 3 : 1));  // three: the cluster form
+  l.dY = c.take<float>((size_t)n * dim * (resident_rows(n, dim) ? 3 : 1));  // three arrays in turn
   l.block_counts = c.take<int32_t>((size_t)ceil_div(e_cap > 0 ? e_cap : 1, kEdgesPerBlock) + 1);
   l.total = c.take<int64_t>(8);
   l.scan_ws = c.take<int64_t>(kScanMaxBlocks);
@@ -971,7 +975,7 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
                             int32_t neg_rate, uint64_t seed, void* workspace, cudaStream_t stream) {
   // below four epochs the load of the edges and the store of their schedule cost more than the
   // launches (a callback after every epoch runs them one by one)
-  if (dim > 4 || n >= layout::kClusterRows || epoch_end - epoch_begin < 4) return false;
+  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4) return false;
   const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
   layout::ClusterArgs c = {};
   const layout::Layout l = layout::carve(workspace, n, dim, e_cap);
