@@ -10,7 +10,7 @@
 //
 // Epoch (umap.py:359-387): every gather reads the epoch-start Y; the moves of
 // all pairs are accumulated into dY with float atomics and applied by a second
-// kernel, which reproduces the reference's synchronous scatter-add semantics.
+// kernel (few rows: after a barrier of one kernel), which reproduces the reference's synchronous scatter-add semantics.
 // Per active edge (i, j): attractive move clip(-2ab d^{2(b-1)}/(1+a d^{2b}) diff,
 // +-4) * alpha added to i and subtracted from j; neg_rate negatives (i, t) each
 // add clip(2b/((0.001+d^2)(1+a d^{2b})) diff, +-4) * alpha to i only.  The moves
@@ -54,7 +54,12 @@ constexpr int kEpochBlocksPerSM = UMAPB_LAYOUT_BLOCKS_PER_SM;
 #endif
 // the same for the kernel specialised to 5 negatives per edge (the default rate)
 constexpr int kEpochBlocksPerSM5 = UMAPB_LAYOUT_BLOCKS_PER_SM5;
-constexpr int kPre = 8;  // epoch kernel: chunks of 32 edges whose schedule words load together
+// epoch kernel: chunks of 32 edges whose schedule words load together.  5 negatives: a short pass
+// lets a block's gathers begin while its neighbours scan (B200, per epoch at 30,000, 70,000 and
+// 200,000 points, k = 15: 4 chunks 9.8, 19.8, 50.4 us; 8 11.4, 20.6, 50.9; 12 11.6, 20.7, 49.7).  Any
+// number: fuller batches count for more (30,092 points, k = 30, 10 negatives, dim 2: 4 chunks
+// 22.2, 8 19.6; 70,000 points, k = 15, 3 negatives: 18.2, 17.7).
+constexpr int pass_chunks(int neg) { return neg == 5 ? 4 : 8; }
 
 // ---- reference pair math (float32, evaluation order of umap.py:361-383) ----
 struct Params {
@@ -103,22 +108,32 @@ __device__ __forceinline__ void repel_add(const float (&yi)[DIM], const float (&
     acc[c] = __fadd_rn(acc[c], __fmul_rn(fminf(fmaxf(__fmul_rn(coeff, diff[c]), -4.0f), 4.0f), p.alpha));
 }
 
+// coherent loads: Y may have been written by a grid that this one has waited for
 template <int DIM>
-__device__ __forceinline__ void load_row(const float* __restrict__ Y, int i, float (&v)[DIM]) {
+__device__ __forceinline__ void load_row(const float* Y, int i, float (&v)[DIM]) {
   if constexpr (DIM == 2) {
-    const float2 t = __ldg(reinterpret_cast<const float2*>(Y) + i);
+    const float2 t = reinterpret_cast<const float2*>(Y)[i];
     v[0] = t.x;
     v[1] = t.y;
   } else if constexpr (DIM == 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(Y) + i);
+    const float4 t = reinterpret_cast<const float4*>(Y)[i];
     v[0] = t.x;
     v[1] = t.y;
     v[2] = t.z;
     v[3] = t.w;
   } else {
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) v[c] = __ldg(Y + (int64_t)i * DIM + c);
+    for (int c = 0; c < DIM; ++c) v[c] = Y[(int64_t)i * DIM + c];
   }
+}
+
+// Programmatic dependent launch: the next grid of the stream may start once every block of this
+// one has called next_may_start() or ended; await_previous() returns when the grid before has
+// ended and its writes are visible (no fence: one more per block costs 2 us an epoch).
+// Without the launch attribute neither does anything.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void await_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <int DIM>
@@ -162,12 +177,20 @@ __global__ void eps_kernel(const float* __restrict__ vals, const int64_t* __rest
 // Only the edges due in an epoch do work, about a third of them on average, so a
 // thread-per-edge loop leaves most lanes idle.  Each warp scans a contiguous
 // segment of edges, advances the schedule of the due ones and queues them in
-// shared memory; the warp works through the queue 32 edges at a time with every
-// lane busy (at most one partial batch per warp, at the end of its segment).
+// shared memory; the warps work through the queue 32 edges at a time with every
+// lane busy (at most one partial batch per block and pass).
+//
+// Two grids an epoch, this one and the apply.  Each is launched to overlap the one before:
+// the apply's blocks fill the SMs as the epoch's end, and the next epoch scans its first pass
+// while the apply runs, so that neither launch gap nor the scan's round trip is on the
+// chain.  What bounds it: the random 8-byte accesses (the two ends, five negatives, two sums
+// per due edge, 290 G/s measured), then the scan of the schedule.  B200, per epoch, k = 15,
+// 5 negatives, dim 2: 30,000 points 11.9 -> 9.8 us, 70,000 21.7 -> 19.8, 200,000 51.3 -> 50.4, of
+// which the overlap is 1.6 us at 70,000 and the short passes the rest at 30,000.
 // NEG > 0: compiled for exactly NEG (<= 8) negatives per edge (neg_rate == NEG), so
 // the registers of the unused sample slots are not held.
 template <int DIM, int NEG>
-__device__ __forceinline__ void edge_update(const float* __restrict__ Y, float* __restrict__ dY, int n, int i,
+__device__ __forceinline__ void edge_update(const float* Y, float* dY, int n, int i,
                                             int j, int64_t e, int epoch, const Params& p, int neg_rate, uint32_t k0,
                                             uint32_t k1) {
   static_assert(NEG >= 0 && NEG <= 8, "NEG is 0 (any rate) or a rate <= 8");
@@ -226,17 +249,19 @@ __device__ __forceinline__ void edge_update(const float* __restrict__ Y, float* 
 }
 
 template <int DIM, int NEG>
-__global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* __restrict__ Y, float* __restrict__ dY, int n,
+__global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* Y, float* dY, int n,
                                                            const int32_t* __restrict__ rows,
                                                            const int32_t* __restrict__ cols,
                                                            const float* __restrict__ eps, float* __restrict__ next,
                                                            const int64_t* __restrict__ n_edges, int epoch, Params p,
                                                            int neg_rate, uint32_t k0, uint32_t k1) {
-  // A pass: every warp loads the schedule words of kPre chunks of 32 edges of its
+  // A pass: every warp loads the schedule words of up to kPre chunks of 32 edges of its
   // segment at once (one round trip instead of kPre), advances the due edges and
   // appends them to the block's queue; then the block's 8 warps take the queue 32
   // edges at a time, so only the block's last batch of the pass runs partly empty.
-  __shared__ int32_t bq[(kBlock / 32) * kPre * 32];
+  constexpr int kPre = pass_chunks(NEG);
+  static_assert(kPre * 32 <= 4096, "an edge of a warp's pass has 12 bits in the queue");
+  __shared__ uint16_t bq[(kBlock / 32) * kPre * 32];  // warp << 12 | edge of the warp's pass
   __shared__ int s_cnt;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t E = *n_edges;
@@ -247,20 +272,24 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
   const int64_t e0 = b0 + (int64_t)warp * seg;
   const int64_t e1 = e0 + seg < E ? e0 + seg : E;
   const unsigned below = (1u << lane) - 1u;
-  const int passes = (int)((seg + 32 * kPre - 1) / (32 * kPre));  // the same for every warp of the grid
+  // passes of equal length, the same for every warp of the grid
+  const int passes = (int)((seg + 32 * kPre - 1) / (32 * kPre));
+  const int chunks = passes > 0 ? (int)((seg / 32 + passes - 1) / passes) : 0;
+  next_may_start();
   for (int ps = 0; ps < passes; ++ps) {
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
-    const int64_t sb = e0 + (int64_t)ps * 32 * kPre;
+    const int64_t done = (int64_t)ps * 32 * chunks, sb = e0 + done;
     float nx[kPre], ex[kPre];
 #pragma unroll
     for (int u = 0; u < kPre; ++u) {
-      const int64_t e = sb + 32 * u + lane;
-      nx[u] = e < e1 ? next[e] : INFINITY;
+      const int64_t e = u < chunks ? sb + 32 * u + lane : e1;
+      nx[u] = e < e1 ? __ldcg(next + e) : INFINITY;  // through L2: the epoch before wrote it
       ex[u] = e < e1 ? eps[e] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < kPre; ++u) {
+      if (u >= chunks) break;
       const int64_t e = sb + 32 * u + lane;
       const bool due = nx[u] <= ep;
       if (due) next[e] = __fadd_rn(nx[u], ex[u]);
@@ -268,26 +297,28 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
       int slot = 0;
       if (lane == 0 && b) slot = atomicAdd(&s_cnt, __popc(b));
       slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (due) bq[slot + __popc(b & below)] = (int32_t)(e - b0);
+      if (due) bq[slot + __popc(b & below)] = (uint16_t)(warp << 12 | 32 * u | lane);
     }
     __syncthreads();
     // the warp's batches: the head and tail ids of the next batch load while this
     // batch's rows of Y are gathered, one round trip per batch instead of two
     const int total = s_cnt;
     int base = warp * 32;
+    auto edge = [&](int q) { return b0 + done + (int64_t)(bq[q] >> 12) * seg + (bq[q] & 4095); };
     int64_t e = 0;
     int i = 0, j = 0;
     if (base + lane < total) {
-      e = b0 + bq[base + lane];
+      e = edge(base + lane);
       i = rows[e];
       j = cols[e];
     }
+    if (ps == 0) await_previous();  // from here on Y and dY
     for (; base < total; base += kBlock) {
       const int nb = base + kBlock;
       int64_t e2 = 0;
       int i2 = 0, j2 = 0;
       if (nb + lane < total) {
-        e2 = b0 + bq[nb + lane];
+        e2 = edge(nb + lane);
         i2 = rows[e2];
         j2 = cols[e2];
       }
@@ -298,11 +329,28 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
     }
     __syncthreads();
   }
+  if (passes == 0) await_previous();  // a grid ends after the one before it
 }
 
-__global__ void apply_kernel(float* __restrict__ Y, float* __restrict__ dY, int64_t m) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
-    Y[t] = __fadd_rn(Y[t], dY[t]);
+// The next epoch's grid starts while this one runs: the epoch whose schedule it reads has ended.
+__global__ void apply_kernel(float* Y, float* dY, int64_t m) {
+  await_previous();
+  next_may_start();
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t m4 = (reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(dY)) % 16 == 0 ? m / 4 : 0;
+  float4 *Y4 = reinterpret_cast<float4*>(Y), *dY4 = reinterpret_cast<float4*>(dY);
+  for (int64_t t = first; t < m4; t += step) {
+    float4 y = __ldcg(Y4 + t);
+    const float4 d = __ldcg(dY4 + t);
+    y.x = __fadd_rn(y.x, d.x);
+    y.y = __fadd_rn(y.y, d.y);
+    y.z = __fadd_rn(y.z, d.z);
+    y.w = __fadd_rn(y.w, d.w);
+    Y4[t] = y;
+    dY4[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int64_t t = 4 * m4 + first; t < m; t += step) {
+    Y[t] = __fadd_rn(__ldcg(Y + t), __ldcg(dY + t));
     dY[t] = 0.f;
   }
 }
@@ -778,21 +826,34 @@ static bool neg5_kernel_enabled() {
   return !(e && e[0] == '0' && e[1] == 0);
 }
 
+// A launch that may start before the grid before it has ended (overlap), or not.
+template <typename... P, typename... A>
+static void launch_overlapping(void (*kernel)(P...), unsigned grid, bool overlap, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // an error is seen by the launch check
+}
+
+// first: the grid before is not an epoch's apply
 template <int DIM>
 static void launch_epoch(const Layout& l, float* Y, int64_t n, const int32_t* rows, const int32_t* cols,
                          const float* eps, float* next, const int64_t* n_edges, int64_t e_cap, int epoch,
-                         const Params& p, int neg_rate, uint64_t seed, bool neg5, cudaStream_t stream) {
-  if (neg_rate == 5 && neg5)
-    sgd_epoch_kernel<DIM, 5><<<epoch_grid(e_cap, kEpochBlocksPerSM5), kBlock, 0, stream>>>(
-        Y, l.dY, (int)n, rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
-  else
-    sgd_epoch_kernel<DIM, 0><<<epoch_grid(e_cap, kEpochBlocksPerSM), kBlock, 0, stream>>>(
-        Y, l.dY, (int)n, rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
+                         const Params& p, int neg_rate, uint64_t seed, bool neg5, bool first, cudaStream_t stream) {
+  const bool five = neg_rate == 5 && neg5;
+  launch_overlapping(five ? sgd_epoch_kernel<DIM, 5> : sgd_epoch_kernel<DIM, 0>,
+                     epoch_grid(e_cap, five ? kEpochBlocksPerSM5 : kEpochBlocksPerSM), !first, stream, Y, l.dY, n,
+                     rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
   const int64_t m = n * DIM;
-  const unsigned gb = (unsigned)(ceil_div(m, kBlock) < num_sms() * 8 ? ceil_div(m, kBlock) : num_sms() * 8);
-  apply_kernel<<<gb, kBlock, 0, stream>>>(Y, l.dY, m);
+  const unsigned gb = (unsigned)(ceil_div(m, 4 * kBlock) < num_sms() * 8 ? ceil_div(m, 4 * kBlock) : num_sms() * 8);
+  launch_overlapping(apply_kernel, gb, true, stream, Y, l.dY, m);
 }
-
 static void launch_epoch_wide(const Layout& l, float* Y, int64_t n, int dim, const int32_t* rows,
                               const int32_t* cols, const float* eps, float* next, const int64_t* n_edges,
                               int64_t e_cap, int epoch, const Params& p, int neg_rate, uint64_t seed,
@@ -1028,10 +1089,10 @@ static int enqueue_epochs(float* Y, int64_t n, int32_t dim, const int32_t* rows,
   for (int ep = epoch_begin; ep < epoch_end; ++ep) {
     const layout::Params p = layout::make_params(a, b, learning_rate, ep, n_epochs);
     switch (dim) {
-      case 1: layout::launch_epoch<1>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, stream); break;
-      case 2: layout::launch_epoch<2>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, stream); break;
-      case 3: layout::launch_epoch<3>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, stream); break;
-      case 4: layout::launch_epoch<4>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, stream); break;
+      case 1: layout::launch_epoch<1>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, ep == epoch_begin, stream); break;
+      case 2: layout::launch_epoch<2>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, ep == epoch_begin, stream); break;
+      case 3: layout::launch_epoch<3>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, ep == epoch_begin, stream); break;
+      case 4: layout::launch_epoch<4>(l, Y, n, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, neg5, ep == epoch_begin, stream); break;
       default:
         layout::launch_epoch_wide(l, Y, n, dim, rows, cols, eps, next, n_edges, e_cap, ep, p, neg_rate, seed, stream);
         break;
