@@ -10,8 +10,9 @@ and after every epoch that has active edges (umap.py:420-442).
 Pipeline, all on the GPU through libumap_b200:
   kNN (brute tcgen05 / NNDescent) -> fuzzy set (FP64 sigma bisection)
   -> spectral init (CSR SpMV + Cholesky-QR power iteration)
-  -> layout epochs (exact float32 schedule, synchronous SGD), two launches per
-     epoch, run as one CUDA graph that the library records and updates per fit.
+  -> layout epochs (exact float32 schedule, synchronous SGD): few rows in one
+     launch; else two overlapping launches per epoch, run as one CUDA graph that the
+     library records and updates per fit.
 Host work left: the a/b curve fit (float64, microseconds); the NumPy streams the
 reference draws from are seeded on the host and drawn on the device.
 

@@ -54,12 +54,14 @@ constexpr int kEpochBlocksPerSM = UMAPB_LAYOUT_BLOCKS_PER_SM;
 #endif
 // the same for the kernel specialised to 5 negatives per edge (the default rate)
 constexpr int kEpochBlocksPerSM5 = UMAPB_LAYOUT_BLOCKS_PER_SM5;
-// epoch kernel: chunks of 32 edges whose schedule words load together.  5 negatives: a short pass
-// lets a block's gathers begin while its neighbours scan (B200, per epoch at 30,000, 70,000 and
-// 200,000 points, k = 15: 4 chunks 9.8, 19.8, 50.4 us; 8 11.4, 20.6, 50.9; 12 11.6, 20.7, 49.7).  Any
-// number: fuller batches count for more (30,092 points, k = 30, 10 negatives, dim 2: 4 chunks
-// 22.2, 8 19.6; 70,000 points, k = 15, 3 negatives: 18.2, 17.7).
-constexpr int pass_chunks(int neg) { return neg == 5 ? 4 : 8; }
+// Epoch kernel: chunks of 32 edges whose schedule words load together.  A short pass lets a
+// block's gathers begin while its neighbours scan; with many edges per warp the passes' round
+// trips and partly empty batches count for more.  B200, per epoch, k = 15, 5 negatives, dim 2,
+// 4 and 10 chunks: 30,000 points 9.8 and 11.5 us, 70,000 19.8 and 20.7, 100,000 27.1 and 26.9,
+// 200,000 50.3 and 49.6, 300,000 76.5 and 73.3, 1,000,000 253.6 and 243.4.  Other rates: 8 (30,092
+// points, k = 30, 10 negatives: 4 chunks 22.2, 8 19.6; 70,000 points, 3 negatives: 18.2, 17.7).
+constexpr int kShortPass = 4, kLongPass = 10, kAnyPass = 8;
+constexpr int64_t kLongPassEdges = 288;  // per warp: 91,000 points at k = 15
 
 // ---- reference pair math (float32, evaluation order of umap.py:361-383) ----
 struct Params {
@@ -185,7 +187,7 @@ __global__ void eps_kernel(const float* __restrict__ vals, const int64_t* __rest
 // while the apply runs, so that neither launch gap nor the scan's round trip is on the
 // chain.  What bounds it: the random 8-byte accesses (the two ends, five negatives, two sums
 // per due edge, 290 G/s measured), then the scan of the schedule.  B200, per epoch, k = 15,
-// 5 negatives, dim 2: 30,000 points 11.9 -> 9.8 us, 70,000 21.7 -> 19.8, 200,000 51.3 -> 50.4, of
+// 5 negatives, dim 2: 30,000 points 11.9 -> 9.8 us, 70,000 21.7 -> 19.8, 200,000 51.3 -> 49.6, of
 // which the overlap is 1.6 us at 70,000 and the short passes the rest at 30,000.
 // NEG > 0: compiled for exactly NEG (<= 8) negatives per edge (neg_rate == NEG), so
 // the registers of the unused sample slots are not held.
@@ -248,7 +250,7 @@ __device__ __forceinline__ void edge_update(const float* Y, float* dY, int n, in
   atomic_add_row<DIM>(dY, i, acc);
 }
 
-template <int DIM, int NEG>
+template <int DIM, int NEG, int kPre>
 __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* Y, float* dY, int n,
                                                            const int32_t* __restrict__ rows,
                                                            const int32_t* __restrict__ cols,
@@ -259,7 +261,6 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
   // segment at once (one round trip instead of kPre), advances the due edges and
   // appends them to the block's queue; then the block's 8 warps take the queue 32
   // edges at a time, so only the block's last batch of the pass runs partly empty.
-  constexpr int kPre = pass_chunks(NEG);
   static_assert(kPre * 32 <= 4096, "an edge of a warp's pass has 12 bits in the queue");
   __shared__ uint16_t bq[(kBlock / 32) * kPre * 32];  // warp << 12 | edge of the warp's pass
   __shared__ int s_cnt;
@@ -847,9 +848,13 @@ static void launch_epoch(const Layout& l, float* Y, int64_t n, const int32_t* ro
                          const float* eps, float* next, const int64_t* n_edges, int64_t e_cap, int epoch,
                          const Params& p, int neg_rate, uint64_t seed, bool neg5, bool first, cudaStream_t stream) {
   const bool five = neg_rate == 5 && neg5;
-  launch_overlapping(five ? sgd_epoch_kernel<DIM, 5> : sgd_epoch_kernel<DIM, 0>,
-                     epoch_grid(e_cap, five ? kEpochBlocksPerSM5 : kEpochBlocksPerSM), !first, stream, Y, l.dY, n,
-                     rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
+  const unsigned grid = epoch_grid(e_cap, five ? kEpochBlocksPerSM5 : kEpochBlocksPerSM);
+  const bool longer = e_cap > kLongPassEdges * (kBlock / 32) * (int64_t)grid;
+  launch_overlapping(!five    ? sgd_epoch_kernel<DIM, 0, kAnyPass>
+                     : longer ? sgd_epoch_kernel<DIM, 5, kLongPass>
+                              : sgd_epoch_kernel<DIM, 5, kShortPass>,
+                     grid, !first, stream, Y, l.dY, n, rows, cols, eps, next, n_edges, epoch, p, neg_rate,
+                     (uint32_t)seed, (uint32_t)(seed >> 32));
   const int64_t m = n * DIM;
   const unsigned gb = (unsigned)(ceil_div(m, 4 * kBlock) < num_sms() * 8 ? ceil_div(m, 4 * kBlock) : num_sms() * 8);
   launch_overlapping(apply_kernel, gb, true, stream, Y, l.dY, m);
