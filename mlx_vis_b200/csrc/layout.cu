@@ -54,14 +54,7 @@ constexpr int kEpochBlocksPerSM = UMAPB_LAYOUT_BLOCKS_PER_SM;
 #endif
 // the same for the kernel specialised to 5 negatives per edge (the default rate)
 constexpr int kEpochBlocksPerSM5 = UMAPB_LAYOUT_BLOCKS_PER_SM5;
-// Epoch kernel: chunks of 32 edges whose schedule words load together.  A short pass lets a
-// block's gathers begin while its neighbours scan; with many edges per warp the passes' round
-// trips and partly empty batches count for more.  B200, per epoch, k = 15, 5 negatives, dim 2,
-// 4 and 10 chunks: 30,000 points 9.8 and 11.5 us, 70,000 19.8 and 20.7, 100,000 27.1 and 26.9,
-// 200,000 50.3 and 49.6, 300,000 76.5 and 73.3, 1,000,000 253.6 and 243.4.  Other rates: 8 (30,092
-// points, k = 30, 10 negatives: 4 chunks 22.2, 8 19.6; 70,000 points, 3 negatives: 18.2, 17.7).
-constexpr int kShortPass = 4, kLongPass = 10, kAnyPass = 8;
-constexpr int64_t kLongPassEdges = 288;  // per warp: 91,000 points at k = 15
+constexpr int kPre = 8;  // epoch kernel: chunks of 32 edges whose schedule words load together
 
 // ---- reference pair math (float32, evaluation order of umap.py:361-383) ----
 struct Params {
@@ -183,16 +176,17 @@ __global__ void eps_kernel(const float* __restrict__ vals, const int64_t* __rest
 // lane busy (at most one partial batch per block and pass).
 //
 // Two grids an epoch, this one and the apply.  Each is launched to overlap the one before:
-// the apply's blocks fill the SMs as the epoch's end, and the next epoch scans its first pass
+// the apply's blocks start as the epoch's end, and the next epoch scans its first pass
 // while the apply runs, so that neither launch gap nor the scan's round trip is on the
 // chain.  What bounds it: the random 8-byte accesses (the two ends, five negatives, two sums
 // per due edge, 290 G/s measured), then the scan of the schedule.  B200, per epoch, k = 15,
-// 5 negatives, dim 2: 30,000 points 11.9 -> 9.8 us, 70,000 21.7 -> 19.8, 200,000 51.3 -> 49.6, of
-// which the overlap is 1.6 us at 70,000 and the short passes the rest at 30,000.
+// 5 negatives, dim 2: 30,000 points 11.1 -> 10.2 us, 70,000 20.6 -> 19.8, 200,000 51.4 -> 50.0; the
+// graph of 70,000 images over 500 epochs 16.8 -> 16.2.  (The apply let in from the epoch's start:
+// 0.6 to 1.3 us more.  Passes of 4 chunks gain 0.4 us at most and lose 0.8 on the images' graph.)
 // NEG > 0: compiled for exactly NEG (<= 8) negatives per edge (neg_rate == NEG), so
 // the registers of the unused sample slots are not held.
 template <int DIM, int NEG>
-__device__ __forceinline__ void edge_update(const float* Y, float* dY, int n, int i,
+__device__ __forceinline__ void edge_update(const float* Y, float* __restrict__ dY, int n, int i,
                                             int j, int64_t e, int epoch, const Params& p, int neg_rate, uint32_t k0,
                                             uint32_t k1) {
   static_assert(NEG >= 0 && NEG <= 8, "NEG is 0 (any rate) or a rate <= 8");
@@ -250,8 +244,8 @@ __device__ __forceinline__ void edge_update(const float* Y, float* dY, int n, in
   atomic_add_row<DIM>(dY, i, acc);
 }
 
-template <int DIM, int NEG, int kPre>
-__global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* Y, float* dY, int n,
+template <int DIM, int NEG>
+__global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* Y, float* __restrict__ dY, int n,
                                                            const int32_t* __restrict__ rows,
                                                            const int32_t* __restrict__ cols,
                                                            const float* __restrict__ eps, float* __restrict__ next,
@@ -276,7 +270,6 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
   // passes of equal length, the same for every warp of the grid
   const int passes = (int)((seg + 32 * kPre - 1) / (32 * kPre));
   const int chunks = passes > 0 ? (int)((seg / 32 + passes - 1) / passes) : 0;
-  next_may_start();
   for (int ps = 0; ps < passes; ++ps) {
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
@@ -331,6 +324,7 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
     __syncthreads();
   }
   if (passes == 0) await_previous();  // a grid ends after the one before it
+  next_may_start();  // here and not at the start: the apply's waiting blocks would take issue slots
 }
 
 // The next epoch's grid starts while this one runs: the epoch whose schedule it reads has ended.
@@ -849,12 +843,8 @@ static void launch_epoch(const Layout& l, float* Y, int64_t n, const int32_t* ro
                          const Params& p, int neg_rate, uint64_t seed, bool neg5, bool first, cudaStream_t stream) {
   const bool five = neg_rate == 5 && neg5;
   const unsigned grid = epoch_grid(e_cap, five ? kEpochBlocksPerSM5 : kEpochBlocksPerSM);
-  const bool longer = e_cap > kLongPassEdges * (kBlock / 32) * (int64_t)grid;
-  launch_overlapping(!five    ? sgd_epoch_kernel<DIM, 0, kAnyPass>
-                     : longer ? sgd_epoch_kernel<DIM, 5, kLongPass>
-                              : sgd_epoch_kernel<DIM, 5, kShortPass>,
-                     grid, !first, stream, Y, l.dY, n, rows, cols, eps, next, n_edges, epoch, p, neg_rate,
-                     (uint32_t)seed, (uint32_t)(seed >> 32));
+  launch_overlapping(five ? sgd_epoch_kernel<DIM, 5> : sgd_epoch_kernel<DIM, 0>, grid, !first, stream, Y, l.dY, n,
+                     rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
   const int64_t m = n * DIM;
   const unsigned gb = (unsigned)(ceil_div(m, 4 * kBlock) < num_sms() * 8 ? ceil_div(m, 4 * kBlock) : num_sms() * 8);
   launch_overlapping(apply_kernel, gb, true, stream, Y, l.dY, m);
