@@ -1022,7 +1022,10 @@ extern "C" int umapb_spectral(const int32_t* rows, const int32_t* cols, const fl
     // the block's share of the edges, and half as many again for uneven rows
     int64_t cap = e_cap / grid + e_cap / grid / 2 + 64;
     const int64_t room = (int64_t)(spectral::kPowerSmem - off_bytes) / 8;
-    if (cap > room) cap = room;
+    // A share that does not fit stays in L2, all of it, and L1 keeps its size: staging the part that
+    // fits took the start of 1,000,000 rows from 10.3 to 16.6 ms; without, graph and start of
+    // 1,000,000 rows 11.9 -> 9.2 ms, 300,000 3.8 -> 2.9, against the form before.
+    if (cap > room) cap = e_cap / grid > room ? 0 : room;
     const size_t smem = off_bytes + (size_t)cap * 8;
     int edge_cap = (int)cap;
     int per_sm = 0;

@@ -263,7 +263,7 @@ def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim):
 
 
 @pytest.mark.parametrize("n,k,dim", [(17, 16, 2), (300, 5, 1), (300, 40, 4), (2560, 12, 4), (2561, 12, 4),
-                                     (5120, 9, 2), (5121, 9, 2), (9000, 24, 3)])
+                                     (5120, 9, 2), (5121, 9, 2), (9000, 24, 3), (6000, 140, 2)])
 def test_power_iteration_forms_match_float64(n, k, dim):
     """The cluster form (up to 5,120 rows of 16 bytes, 2,560 of 32) and the grid-wide one on
     either side of their border, uneven row counts per CTA and more edges than a CTA's
