@@ -45,11 +45,11 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
   const unsigned below = (1u << lane) - 1u;
 
   const int my_old = lane < k ? a.idx_old[row * k + lane] : -1;
-  const float my_d = lane < k ? (a.curd ? a.curd : a.dist_old)[row * k + lane] : 0.f;
-  float d[NCH];
+  const float my_d = lane < k ? to_key((a.curd ? a.curd : a.dist_old)[row * k + lane]) : 0.f;
+  float d[NCH];  // keys of the nn-of-nn candidates; INFINITY, above every key: absent or taken
   const float* nn = a.nnbuf + row * nn_cols;
 #pragma unroll
-  for (int u = 0; u < NCH; ++u) d[u] = u * 32 + lane < nn_cols ? nn[u * 32 + lane] : INFINITY;
+  for (int u = 0; u < NCH; ++u) d[u] = u * 32 + lane < nn_cols ? to_key(nn[u * 32 + lane]) : INFINITY;
 
   // reverse candidates, one per lane: id rid at distance rd
   int rid = -1, pads = 0;  // pads: empty slots
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
     if (cnt <= 32) {
       if (lane < cnt) {
         rid = a.entries[o + lane] >> 5;
-        rd = a.entd[o + lane];
+        rd = to_key(a.entd[o + lane]);
       }
       if (cnt > k) {  // the k smallest ids
         int rank = 0;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
         if (rank >= k) rid = -1, rd = INFINITY;
       } else if (lane == cnt && pads) {
         rid = 0;
-        rd = a.d0[row];
+        rd = to_key(a.d0[row]);
       }
     } else {  // a hub: the k-th smallest id by bisection over the ids
       int lo = 0, hi = (int)a.n - 1;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
       if (lane < k) {
         const int e = s_c[warp][lane];
         rid = a.entries[o + e] >> 5;
-        rd = a.entd[o + e];
+        rd = to_key(a.entd[o + e]);
       }
       __syncwarp();
     }
@@ -120,6 +120,8 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
   float tau = __shfl_sync(kAll, lv, k - 1);
   int tau_i = __shfl_sync(kAll, li, k - 1);
 
+  // tau is at most kSent, below INFINITY, so a turn counts untaken candidates only and takes at
+  // least one of them
   while (true) {
     int c = rd <= tau ? 1 : 0;
 #pragma unroll
@@ -226,34 +228,38 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
     tau_i = __shfl_sync(kAll, li, k - 1);
   }
 
-  if (tau >= kBig) {
-    // fewer than k distinct candidates (small n): every one of them is in the list, and
-    // the dropped columns (the row itself, later copies of an id) complete it by id
-    bool seen = false;  // the list entry of this lane has occurred in a column
-    for (int t = 0; t < k; ++t) {
-      const int current = __shfl_sync(kAll, my_old, t);
-      seen = seen || li == current;
-    }
+  if (key_lt(kBig, 0, tau, tau_i)) {
+    // Fewer than k candidates nearer than 1e30 (small n, or infinite distances): the dropped
+    // columns (the row itself, later copies of an id) count as 1e30, by id.  Those of the
+    // current list are in the list already.
     const int total = nn_cols + (a.off ? 32 + pads : 0);
-    for (int t0 = 0; t0 < total; t0 += 32) {
-      const int t = t0 + lane;
+    auto column = [&](int t) {  // the id in column t (behind the current list), -1: none; all lanes call
       const int p = (int)(((uint32_t)(t < nn_cols ? t : 0) * a.magic) >> 20);
       const int src = __shfl_sync(kAll, my_old, p & 31);
       const int r = __shfl_sync(kAll, rid, (t - nn_cols) & 31);
-      int id = -1;
-      if (t < nn_cols) id = a.idx_old[(int64_t)src * k + (t - p * a.j_nn)];
-      else if (t < nn_cols + 32 && a.off) id = r;      // the slots (the first empty one among them)
-      else if (t < total - 1) id = 0;                  // the other empty slots
-      for (unsigned todo = __ballot_sync(kAll, id >= 0); todo; todo &= todo - 1u) {
-        const int si = __shfl_sync(kAll, id, __ffs(todo) - 1);
-        const unsigned hit = __ballot_sync(kAll, lane < k && lv < kBig && li == si);
-        bool drop = si == (int)row;
-        if (hit) {
-          const int l = __ffs(hit) - 1;
-          drop = __shfl_sync(kAll, seen, l);
-          if (lane == l) seen = true;
+      if (t < nn_cols) return (int)a.idx_old[(int64_t)src * k + (t - p * a.j_nn)];
+      if (t < nn_cols + 32) return a.off ? r : -1;  // the slots (the first empty one among them)
+      return t < total - 1 ? 0 : -1;                // the other empty slots
+    };
+    for (int t0 = 0; t0 < total; t0 += 32) {
+      const int id = column(t0 + lane);
+      const unsigned same = __match_any_sync(kAll, id >= 0 ? id : -2 - lane);
+      bool drop = id >= 0 && (id == (int)row || __ffs(same) - 1 != lane);
+      for (int t = 0; t < k; ++t) {
+        const int other = __shfl_sync(kAll, my_old, t);
+        drop = drop || (id >= 0 && id == other);
+      }
+      for (int e0 = 0; e0 < t0; e0 += 32) {  // an earlier column with the same id
+        if (!__any_sync(kAll, id >= 0 && !drop && key_lt(kBig, id, tau, tau_i))) break;
+        const int before = column(e0 + lane);
+        for (int t = 0; t < 32; ++t) {
+          const int other = __shfl_sync(kAll, before, t);
+          drop = drop || (id >= 0 && id == other);
         }
-        if (drop && key_lt(kBig, si, tau, tau_i)) {
+      }
+      for (unsigned todo = __ballot_sync(kAll, drop); todo; todo &= todo - 1u) {
+        const int si = __shfl_sync(kAll, id, __ffs(todo) - 1);
+        if (key_lt(kBig, si, tau, tau_i)) {
           list_insert(lv, li, kBig, si, k, lane);
           tau = __shfl_sync(kAll, lv, k - 1);
           tau_i = __shfl_sync(kAll, li, k - 1);
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
 
   if (lane < k) {
     a.idx_new[row * k + lane] = li;
-    a.dist_new[row * k + lane] = lv;
+    a.dist_new[row * k + lane] = from_key(lv);
     a.flags_new[row * k + lane] = li != my_old ? 1 : 0;
   }
   const int nch = __popc(__ballot_sync(kAll, lane < k && li != my_old));

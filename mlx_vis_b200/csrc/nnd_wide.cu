@@ -10,7 +10,7 @@
 //               per candidate, the dot rounded to FP16 in the FP16 iterations; the
 //               stored distance of an old neighbour unless the iteration recomputes
 //   top-k       (distance bits << 32 | id) keys sorted by a block bitonic network;
-//               self and duplicates sort last
+//               self and duplicates count as 1e30, infinite distances come after them
 //
 // Shared memory per block: candidate ids and distances (8 B per column) + a
 // 64-bit area of next_pow2(1.5 T) entries that holds the hash table and then the
@@ -28,6 +28,7 @@ namespace nnd_wide {
 
 constexpr int kThreads = 512;
 constexpr int kMaxK = 100;
+constexpr float kBig = 1e30f;  // distance of a dropped column (the row itself, a repeated id)
 
 __host__ __device__ inline int next_pow2(int v) {
   int p = 1;
@@ -187,13 +188,13 @@ __global__ void __launch_bounds__(kThreads) iter_kernel(Args a) {
       }
     }
     __syncthreads();
-    // keep flags into cd: +inf for self / later duplicates, else to be computed
+    // keep flags into cd: -1 for columns to be computed, 1e30 for self / later duplicates
     for (int t = threadIdx.x; t < a.T; t += blockDim.x) {
       const int32_t id = cid[t];
       uint32_t h = hash_id(id) & hm;
       while (hkey[h] != id) h = (h + 1) & hm;
       const bool keep = hval[h] == t && id != (int32_t)row;
-      cd[t] = keep ? -1.0f : INFINITY;
+      cd[t] = keep ? -1.0f : kBig;
     }
     __syncthreads();
     // distances: stored ones for old neighbours unless recomputed, the rest by warps
@@ -215,11 +216,12 @@ __global__ void __launch_bounds__(kThreads) iter_kernel(Args a) {
     }
     if (lane == 0 && my_evals) atomicAdd(&s_evals, my_evals);
     __syncthreads();
-    // top-k of (distance, id): keys sorted ascending, padding and dropped columns last
+    // top-k of (distance, id): keys sorted ascending, the padding last; every column is a key, so
+    // the k smallest are ids whatever the distances are
     const int P = next_pow2(a.T);
     for (int t = threadIdx.x; t < P; t += blockDim.x) {
       unsigned long long key = ~0ull;
-      if (t < a.T && cd[t] != INFINITY)
+      if (t < a.T)
         key = ((unsigned long long)__float_as_uint(cd[t]) << 32) | (uint32_t)cid[t];
       area[t] = key;
     }

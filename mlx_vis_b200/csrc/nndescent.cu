@@ -153,7 +153,7 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, const float* __r
   for (int t = lane; t < dd; t += 32) xs[t] = X[row * dd + t];
   __syncwarp();
   const float sqi = sq[row];
-  float my_d = kBig;
+  float my_d = INFINITY;  // past k: above every (distance, id)
   int my_i = 0x7fffffff;
   for (int p0 = 0; p0 < k; p0 += 4) {
     int c[4];
@@ -221,7 +221,7 @@ __global__ void sort_rows_kernel(int32_t* __restrict__ idx, float* __restrict__ 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kWarps + warp;
   if (row >= n) return;
-  float d = lane < k ? dist[row * k + lane] : kBig;
+  float d = lane < k ? dist[row * k + lane] : INFINITY;
   int i = lane < k ? idx[row * k + lane] : 0x7fffffff;
   warp_sort_keys(d, i, lane);
   if (lane < k) {
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) iter_kernel(IterArgs a) {
   int tau_i = li;
   for (int t0 = 0; t0 < a.tcap; t0 += 32) {
     const int t = t0 + lane;
-    float d = t < T_total ? cd[t] : kSent;
+    float d = t < T_total ? to_key(cd[t]) : kSent;
     int id = t < T_total ? cid[t] : 0x7fffffff;
     unsigned b = __ballot_sync(0xffffffffu, t < T_total && key_lt(d, id, tau, tau_i));
     if (__popc(b) > 10) {
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) iter_kernel(IterArgs a) {
   }
   if (lane < k) {
     a.idx_new[row * k + lane] = li;
-    a.dist_new[row * k + lane] = lv;
+    a.dist_new[row * k + lane] = from_key(lv);
     const bool ch = li != my_old;
     a.flags_new[row * k + lane] = ch ? 1 : 0;
   }

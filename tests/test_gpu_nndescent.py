@@ -444,3 +444,98 @@ def test_rows_that_are_not_whole_float4s(d):
     # d > 100: the first iteration runs on the rounded products with the random projection
     assert np.mean(idx != idx0) <= (0.002 if d > 100 else 0.0)
     np.testing.assert_allclose(dist, dist0, rtol=1e-5 if d > 100 else 0.0)
+
+
+def _opposite_rows(n, d, kind, rng):
+    """Integer rows whose FP16 dot products leave the FP16 range: near +50 in every column, one
+    row or half of them negated, or (mixed) a third of them small."""
+    X = rng.integers(45, 56, size=(n, d)).astype(np.float32)
+    if kind == "one":
+        X[7] *= -1
+    else:
+        X[rng.random(n) < 0.5] *= -1
+    if kind == "mixed":
+        small = rng.random(n) < 0.33
+        X[small] = rng.integers(-3, 4, size=(int(small.sum()), d))
+    return X
+
+
+@pytest.mark.parametrize("use_rev", [False, True])
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("kind", ["one", "half", "mixed"])
+@pytest.mark.parametrize("k", [15, 17, 20, 32])
+def test_select_with_infinite_distances(k, kind, recompute, use_rev):
+    """A dot product below -65,504 makes an FP16 iteration's distance infinite.  The row
+    update ends, keeps ids in range and equals the general one (all values are integers, so every
+    distance is exact): on either side of k = 16, up to which the sentinels behind a list of
+    k used to hide it."""
+    from mlx_vis_b200 import _lib
+
+    n, d, ld, j_nn = 300, 50, 56, k
+    rng = np.random.default_rng(k)
+    X = _opposite_rows(n, d, kind, rng)
+    idx = rng.integers(0, n, size=(n, k)).astype(np.int32)
+    sq = (X ** 2).sum(1).astype(np.float32)
+    with np.errstate(over="ignore"):
+        dot = (X @ X.T).astype(np.float16).astype(np.float32)
+    d2 = np.maximum(sq[:, None] + sq - 2 * dot, 0)
+    assert np.isinf(d2).any()
+    s = _lib.stream_handle()
+    Xh = np.zeros((n, ld), dtype=np.float16)
+    Xh[:, :d] = X
+
+    def dev(a):
+        return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+    Xd, sqd, idx_d, dist = dev(Xh), dev(sq), dev(idx), dev(np.take_along_axis(d2, idx, axis=1))
+    order = dev(rng.permutation(n).astype(np.int32))
+    nnbuf, curd, d0 = (torch.empty(m, device="cuda") for m in (n * k * j_nn, n * k, n))
+    rev = torch.empty((n, k), dtype=torch.int32, device="cuda")
+    ws = _lib.workspace(_lib.query("umapb_nnd_join_workspace", n, k, k), Xd.device)
+    _lib.call("umapb_nnd_join", _lib.ptr(Xd), _lib.ptr(sqd), d, ld, 1, _lib.ptr(idx_d), _lib.ptr(order), n, k, k, j_nn,
+              _lib.ptr(nnbuf), _lib.ptr(curd), _lib.ptr(rev), _lib.ptr(None), _lib.ptr(ws), ws.numel(), s)
+    _lib.call("umapb_nnd_dist_row0", _lib.ptr(Xd), _lib.ptr(sqd), n, d, ld, 1, _lib.ptr(d0), s)
+    got = []
+    for general in (True, False):
+        out = (torch.empty_like(idx_d), torch.empty_like(dist), torch.empty((n, k), dtype=torch.uint8, device="cuda"),
+               torch.zeros(1, dtype=torch.int64, device="cuda"))
+        if general:
+            _lib.call("umapb_nnd_iteration", _lib.ptr(Xd), _lib.ptr(sqd), d, ld, 1, _lib.ptr(idx_d), _lib.ptr(dist),
+                      _lib.ptr(None), _lib.ptr(rev if use_rev else None), _lib.ptr(order), _lib.ptr(nnbuf),
+                      _lib.ptr(curd), n, k, k, j_nn, 0, int(recompute), *(_lib.ptr(t) for t in out), _lib.ptr(None), s)
+        else:
+            _lib.call("umapb_nnd_select", _lib.ptr(idx_d), _lib.ptr(dist), _lib.ptr(order), _lib.ptr(nnbuf),
+                      _lib.ptr(curd), _lib.ptr(d0), n, k, j_nn, int(recompute), _lib.ptr(ws if use_rev else None),
+                      ws.numel(), *(_lib.ptr(t) for t in out), s)
+        got.append([t.cpu().numpy() for t in out])
+    assert got[0][0].min() >= 0 and got[0][0].max() < n
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["one", "half", "mixed"])
+@pytest.mark.parametrize("k", [15, 30, 50])
+def test_build_with_infinite_distances_equals_the_oracle(k, kind):
+    """Whole builds on such rows, with the join's row update (k = 15 and 30) and the block-per-row
+    one (k = 50): every distance is exact, so the graph equals the oracle's."""
+    from mlx_vis_b200 import NNDescent
+
+    X = _opposite_rows(400, 50, kind, np.random.default_rng(k))
+    idx, dist = NNDescent(k=k, random_state=3).build(X)
+    with np.errstate(over="ignore", invalid="ignore"):
+        oi, od = onnd.build(X, k=k, random_state=3)
+    assert np.array_equal(idx, oi)
+    np.testing.assert_allclose(dist, od, rtol=1e-6)
+
+
+@pytest.mark.parametrize("k", [10, 30, 50])
+def test_build_with_overflowing_rows_keeps_ids_in_range(k):
+    """Squared norms beyond FP32 make distances infinite in every iteration; fewer distinct
+    candidates than k among 60 rows as well.  No sentinel becomes an id."""
+    from mlx_vis_b200 import NNDescent
+
+    X = np.random.default_rng(k).normal(size=(60, 20)).astype(np.float32)
+    X[::3] *= 1e20
+    X[1::3] *= 1e15
+    idx, dist = NNDescent(k=k, random_state=1).build(X)
+    assert idx.min() >= 0 and idx.max() < 60 and not np.isnan(dist).any()
