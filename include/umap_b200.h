@@ -47,8 +47,9 @@ unsigned long long umapb_kernel_launches(void);
 /* Synchronises `stream`, reads the device status word at `workspace` and
  * returns UMAPB_OK or UMAPB_ERR_DEVICE (with a message). */
 int umapb_read_status(const void* workspace, umapb_stream_t stream);
-/* Time limit in nanoseconds of the spectral power iteration's grid barrier, for
- * launches made after the call (process-wide; 0 restores the default of 2 s).
+/* Time limit in nanoseconds of the grid barriers of the spectral power iteration and of
+ * the layout's single launch, for launches made after the call (process-wide; 0
+ * restores the default of 2 s).
  * No counterpart in the reference, which has no device-side waits. */
 int umapb_set_wait_limit_ns(unsigned long long ns);
 
@@ -316,7 +317,8 @@ int umapb_spectral_fallback(const void* workspace, float* Y, int64_t n, int32_t 
  *   stream keyed by (seed, epoch, edge, sample).  Four or more epochs whose Y and
  *   edge shares fit the SMs' shared memory run in one launch; the first 32-bit word
  *   of the workspace (zeroed by umapb_layout_prepare) is then 3 after a grid barrier
- *   that waited more than 2 s, and Y is not valid.
+ *   that waited longer than umapb_set_wait_limit_ns allows, and Y and next are as they
+ *   were before the call; calls of at most three epochs have no such wait.
  * umapb_layout_epoch_injected: one epoch whose negative tails are given in the
  *   reference's order (sample j pairs head ef[j % A] with neg_to[j], A = number
  *   of active edges, umap.py:433-436); neg_count must equal neg_rate * A.

@@ -285,7 +285,8 @@ def mt_jump_poly(b: int):
 
 
 def set_wait_limit_ns(ns: int) -> None:
-    """Time limit of the spectral power iteration's grid barrier (0: the 2 s default)."""
+    """Time limit of the grid barriers of the spectral power iteration and of the layout's
+    single launch (0: the 2 s default)."""
     call("umapb_set_wait_limit_ns", int(ns))
 
 
@@ -334,12 +335,29 @@ class Layout:
 
     def epochs(self, Y: torch.Tensor, begin: int, end: int, a: float, b: float, learning_rate: float,
                neg_rate: int, seed: int, graph: bool = False):
-        """Runs epochs [begin, end); with ``graph`` as one cached, updated CUDA graph."""
+        """Runs epochs [begin, end); with ``graph`` as one cached, updated CUDA graph.
+
+        Four or more epochs of few rows are one launch whose grid barrier is bounded
+        (set_wait_limit_ns).  A launch that gave up leaves Y and the schedule as they were;
+        ``check`` tells, and ``epochs_by_launches`` runs the same epochs without such a wait."""
         call("umapb_layout_epochs_graph" if graph else "umapb_layout_epochs", ptr(Y), self.n, self.dim,
              ptr(self.rows), ptr(self.cols), ptr(self.eps),
              ptr(self.next), ptr(self.n_edges), self.e_cap, int(begin), int(end), self.n_epochs, float(a), float(b),
              float(learning_rate), int(neg_rate), int(seed) & 0xFFFFFFFFFFFFFFFF, ptr(self.ws), self.ws.numel(),
              stream_handle())
+
+    def epochs_by_launches(self, Y: torch.Tensor, begin: int, end: int, *args):
+        """Epochs [begin, end) in calls too short for the single launch; ``args`` as for ``epochs``."""
+        for e in range(int(begin), int(end), 3):
+            self.epochs(Y, e, min(e + 3, int(end)), *args)
+
+    def check(self) -> None:
+        """Raises if a launch since the last check gave up at its barrier (synchronises)."""
+        try:
+            read_status(self.ws)
+        except UmapB200Error:
+            self.ws[:4].zero_()
+            raise
 
     def count_active(self, epoch: int) -> int:
         """Active edges in ``epoch`` for the current schedule state (synchronises)."""

@@ -190,15 +190,22 @@ class UMAP:
             st_h = torch.empty(1, dtype=torch.int32, pin_memory=True)
             st_h.copy_(self._spectral_ws[:4].view(torch.int32), non_blocking=True)
         ls_h = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        ls_h.copy_(self._layout_ws[:4].view(torch.int32), non_blocking=True)
-        self._layout_ws = None
+        lay, layout_args = self._layout
+        self._layout = None
+        ls_h.copy_(lay.ws[:4].view(torch.int32), non_blocking=True)
         Y_h = None
         if host_out:
             Y_h = torch.empty(Y.shape, dtype=Y.dtype, pin_memory=True)
             Y_h.copy_(Y, non_blocking=True)
         self.timings_ = ev.finish()  # synchronises the device
         if int(ls_h[0]) != 0:
-            raise _lib.UmapB200Error("umapb_layout_epochs", 5, "device-side wait expired in the layout")
+            # the grid barrier of the layout's single launch gave up, which left Y as it was
+            if self.verbose:
+                print("Layout's grid barrier timed out, running its epochs by launches")
+            lay.epochs_by_launches(Y, 0, int(self.n_epochs), *layout_args)
+            if Y_h is not None:
+                Y_h.copy_(Y, non_blocking=True)
+            torch.cuda.current_stream(dev).synchronize()
         self.graph_info_ = {"n_edges": int(ne_h[0])}
         if Y_h is not None:
             self.embedding_ = Y_h.numpy()
@@ -279,9 +286,9 @@ class UMAP:
     def _optimize(self, rows, cols, vals, n_edges, Y, a, b, n, seed, epoch_callback):
         ne = int(self.n_epochs)
         lay = _lib.Layout(rows, cols, vals, n_edges, n, self.n_components, ne)
-        self._layout_ws = lay.ws
         layout_seed = (seed * 0x9E3779B97F4A7C15 + 1) & 0xFFFFFFFFFFFFFFFF
         args = (a, b, self.learning_rate, self.negative_sample_rate, layout_seed)
+        self._layout = (lay, args)
         if epoch_callback is not None:
             epoch_callback(0, to_host(Y))
             for e in range(ne):

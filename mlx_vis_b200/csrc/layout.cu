@@ -360,9 +360,11 @@ __global__ void apply_kernel(float* Y, float* dY, int64_t m) {
 // next one, which every CTA has read before the last barrier, is cleared.  The draws and
 // the pair math are those of the launches.
 // Up to kClusterEdges edges the CTAs are one cluster of 16 and the barrier is the
-// cluster's; beyond, a resident grid with a barrier in L2 (bounded: 2 s, then the
-// status word), since the pair math of more edges wants more SMs.  Either form needs Y
+// cluster's; beyond, a resident grid with a barrier in L2 (bounded by umapb_set_wait_limit_ns,
+// then the status word), since the pair math of more edges wants more SMs.  Either form needs Y
 // and the share in one SM's shared memory (about 22,000 rows of two components).
+// Y and the schedule are written at the end only, and a barrier that gives up gives up for every
+// CTA, so after an expired wait both are as they were before the launch.
 // B200, per epoch, k = 15 where not said: 600 points, k = 5 8.0 -> 3.4 us (3.9 as a grid);
 // 1,000 points 4.0 either way; 2,000 points 6.7 -> 4.1 us (5.3 as a cluster); 4,000 points
 // 6.9 -> 4.8; 9,999 points, k = 10 8.4 -> 5.9; 20,000 points 9.8 -> 8.8.
@@ -384,11 +386,12 @@ struct ClusterArgs {
   int cap;       // edges per CTA
   float a, b, m2ab, two_b, lr;
   uint32_t k0, k1;
-  unsigned* bar;  // grid form: barrier counter, zero at launch
-  int* abort_g;
+  unsigned* bar;  // grid form: barrier counter, zero at launch; kGaveUp once a wait has expired
   int32_t* status;
   unsigned long long limit_ns;
 };
+
+constexpr unsigned kGaveUp = 1u << 31;
 
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
@@ -396,30 +399,34 @@ __device__ __forceinline__ unsigned long long gtimer() {
   return t;
 }
 
-// Barrier of the resident grid; false once it has waited limit_ns or another block has.
+// Barrier of the resident grid; false once a wait at it has lasted limit_ns.  The counter itself
+// carries the failure: a CTA whose time is up sets kGaveUp by compare-and-swap while
+// the count is short of the target, and a CTA passes on a count without it.  So either every CTA
+// passes a barrier or none does.
 __device__ __forceinline__ bool grid_barrier(const ClusterArgs& a, unsigned target) {
   __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    int ok = 1;
     // the block's writes are ordered before this by the block barrier
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
     const unsigned long long t0 = gtimer();
-    for (unsigned i = 1;; ++i) {
-      unsigned v;
+    unsigned v;
+    while (true) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-      if (v >= target) break;
-      if ((i & 255) == 0 && *(volatile int*)a.abort_g) {
-        ok = 0;
-        break;
-      }
+      if (v >= target) break;  // kGaveUp is above every target
       if (gtimer() - t0 > a.limit_ns) {
-        atomicExch(a.abort_g, 1);
-        ok = 0;
+        while (v < target) {  // ends: the count has moved on whenever the swap fails
+          unsigned was;
+          asm volatile("atom.acquire.gpu.global.cas.b32 %0, [%1], %2, %3;"
+                       : "=r"(was)
+                       : "l"(a.bar), "r"(v), "r"(v | kGaveUp)
+                       : "memory");
+          v = was == v ? v | kGaveUp : was;
+        }
         break;
       }
     }
-    s_ok = ok;
+    s_ok = (v & kGaveUp) == 0;
   }
   __syncthreads();
   return s_ok != 0;
@@ -482,7 +489,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(Clus
   p.m2ab = a.m2ab;
   p.two_b = a.two_b;
   int turn = 0;
-  for (int ep = a.epoch_begin; ep < a.epoch_end; ++ep) {
+  for (int ep = a.epoch_begin; ok && ep < a.epoch_end; ++ep) {
     float* dY = a.dY + (size_t)turn * values;
     const int then = turn == 2 ? 0 : turn + 1;
     float* next_dY = a.dY + (size_t)then * values;
@@ -543,7 +550,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1) layout_cluster_kernel(Clus
     turn = then;
     __syncthreads();
   }
-  if (!ok && tid == 0) atomicExch(a.status, (int32_t)kDevTimeoutEpilogue);
+  if (!ok) {  // every CTA is here: Y and the schedule stay as they were
+    if (tid == 0) atomicExch(a.status, (int32_t)kDevTimeoutEpilogue);
+    return;
+  }
   for (int t = tid; t < m; t += kClusterThreads) a.next[e0 + t] = s_next[t];
   for (int t = tid; t < own * DIM; t += kClusterThreads) a.Y[r0 * DIM + t] = sy[r0 * DIM + t];
 }
@@ -905,8 +915,7 @@ static bool launch_grid(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
   a.cap = (int)ceil_div(e_cap, ctas);
   const size_t smem = cluster_smem(a.n, DIM, a.cap);
   if (smem > kClusterSmem || a.cap > 65535) return false;
-  if (cudaMemsetAsync(a.abort_g, 0, reinterpret_cast<char*>(a.bar + 1) - reinterpret_cast<char*>(a.abort_g), stream) !=
-      cudaSuccess) {  // the status word is cleared by umapb_layout_prepare
+  if (cudaMemsetAsync(a.bar, 0, sizeof(unsigned), stream) != cudaSuccess) {  // umapb_layout_prepare clears the status
     cudaGetLastError();
     return false;
   }
@@ -1031,16 +1040,16 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
                             int32_t neg_rate, uint64_t seed, void* workspace, cudaStream_t stream) {
   // below four epochs the load of the edges and the store of their schedule cost more than the
   // launches (a callback after every epoch runs them one by one)
-  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4) return false;
+  // (above a million epochs the barrier's count would run into its top bit)
+  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4 || epoch_end - epoch_begin > 1000000) return false;
   const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
   layout::ClusterArgs c = {};
   const layout::Layout l = layout::carve(workspace, n, dim, e_cap);
   c.Y = Y;
   c.dY = l.dY;
   c.status = l.status;
-  c.abort_g = l.status + 32;
-  c.bar = reinterpret_cast<unsigned*>(l.status + 48);
-  c.limit_ns = 2000000000ull;
+  c.bar = reinterpret_cast<unsigned*>(l.status + 32);
+  c.limit_ns = wait_limit_ns();
   c.rows = rows;
   c.cols = cols;
   c.eps = eps;

@@ -345,3 +345,63 @@ def test_layout_many_epochs_match_single_epochs(n, k, dim, neg, graph):
     # float32 sums of up to (1 + neg) k clipped moves of at most 0.04 per epoch, in another order
     scale = np.abs(Y0.cpu().numpy()).max()
     assert np.abs(out[0][0] - out[1][0]).max() < 2e-5 * scale
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_layout_barrier_that_gives_up_changes_nothing(graph):
+    """The resident grid's barrier with a limit of 1 ns: the launch ends with the status word set, Y
+    and the schedule as they were, and the same epochs run by launches from there."""
+    from mlx_vis_b200 import _lib
+
+    n, k = 4000, 9  # 36,000 edges: a grid, not a cluster
+    rng = np.random.default_rng(5)
+    rows = np.sort(rng.integers(0, n, size=n * k)).astype(np.int32)
+    cols = rng.integers(0, n, size=n * k).astype(np.int32)
+    vals = rng.uniform(0.05, 1.0, size=n * k).astype(np.float32)
+    ne = torch.tensor([n * k], dtype=torch.int64, device="cuda")
+    Y0 = cuda((10 * rng.normal(size=(n, 2))).astype(np.float32))
+    args = (1.577, 0.895, 0.01, 5, 12345)
+    lay, want = (_lib.Layout(cuda(rows), cuda(cols), cuda(vals), ne, n, 2, 200) for _ in range(2))
+    Y, Yw, next0 = Y0.clone(), Y0.clone(), lay.next.clone()
+    try:
+        _lib.set_wait_limit_ns(1)
+        lay.epochs(Y, 0, 12, *args, graph=graph)
+        torch.cuda.synchronize()
+    finally:
+        _lib.set_wait_limit_ns(0)
+    assert _lib.status_word(lay.ws) == 3
+    assert torch.equal(Y, Y0) and torch.equal(lay.next, next0)
+    with pytest.raises(_lib.UmapB200Error):
+        lay.check()
+    lay.check()  # told once
+    lay.epochs_by_launches(Y, 0, 12, *args)
+    want.epochs(Yw, 0, 12, *args)  # one launch
+    want.check()
+    assert torch.equal(lay.next, want.next)
+    assert float((Yw - Y0).abs().max()) > 1e-3
+    assert float((Y - Yw).abs().max()) < 2e-5 * float(Y0.abs().max())  # float32 sums in another order
+
+
+def test_fit_goes_on_by_launches_when_the_layout_gives_up(gauss2000):
+    """fit_transform with a layout whose barrier expires: the same embedding by launches.  Even at a
+    limit of 1 ns every CTA of a fit can find the others there, so some fits may be needed."""
+    from mlx_vis_b200 import UMAP, _lib
+
+    def fit(limit):
+        try:
+            _lib.set_wait_limit_ns(limit)
+            before = _lib.kernel_launches()
+            # a random start: the spectral one has a barrier with the same limit
+            Y = UMAP(n_epochs=20, learning_rate=0.05, init="random", knn_method="brute",
+                     random_state=4).fit_transform(gauss2000)
+            return Y, _lib.kernel_launches() - before
+        finally:
+            _lib.set_wait_limit_ns(0)
+
+    want, launches = fit(0)
+    for _ in range(40):
+        Y, took = fit(1)
+        assert np.linalg.norm(Y - want) < 1e-3 * np.linalg.norm(want)  # sums in another order over 20 epochs
+        if took != launches:
+            break
+    assert took == launches + 40  # two launches an epoch besides the one that gave up
