@@ -25,6 +25,7 @@
 // for the r-th active edge.
 #include <math.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include <mutex>
 
@@ -909,7 +910,7 @@ static bool launch_grid(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
     }
     if (known[dev] < 0) return false;
   }
-  int64_t ctas = ceil_div(e_cap, 256);
+  int64_t ctas = ceil_div(e_cap > 0 ? e_cap : 1, 256);
   if (ctas > num_sms()) ctas = num_sms();
   a.rows_per = (int)ceil_div(a.n, ctas);
   a.cap = (int)ceil_div(e_cap, ctas);
@@ -978,9 +979,16 @@ static bool launch_cluster(ClusterArgs a, int64_t e_cap, cudaStream_t stream) {
   return true;
 }
 
+// UMAPB_LAYOUT_ONE_LAUNCH in the environment (read per call): 0 runs few rows by launches as well,
+// grid runs few edges on the grid that devices without such clusters use.
+static bool one_launch_is(const char* what) {
+  const char* e = getenv("UMAPB_LAYOUT_ONE_LAUNCH");
+  return e && strcmp(e, what) == 0;
+}
+
 template <int DIM, int NEG>
 static bool launch_resident(const ClusterArgs& a, int64_t e_cap, cudaStream_t stream) {
-  return (e_cap <= kClusterEdges && launch_cluster<DIM, NEG>(a, e_cap, stream)) ||
+  return (e_cap <= kClusterEdges && !one_launch_is("grid") && launch_cluster<DIM, NEG>(a, e_cap, stream)) ||
          launch_grid<DIM, NEG>(a, e_cap, stream);
 }
 
@@ -1041,7 +1049,9 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
   // below four epochs the load of the edges and the store of their schedule cost more than the
   // launches (a callback after every epoch runs them one by one)
   // (above a million epochs the barrier's count would run into its top bit)
-  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4 || epoch_end - epoch_begin > 1000000) return false;
+  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4 || epoch_end - epoch_begin > 1000000 ||
+      layout::one_launch_is("0"))
+    return false;
   const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
   layout::ClusterArgs c = {};
   const layout::Layout l = layout::carve(workspace, n, dim, e_cap);

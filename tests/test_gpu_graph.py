@@ -405,3 +405,20 @@ def test_fit_goes_on_by_launches_when_the_layout_gives_up(gauss2000):
         if took != launches:
             break
     assert took == launches + 40  # two launches an epoch besides the one that gave up
+
+
+@pytest.mark.parametrize("form", ["", "grid", "0"])
+def test_layout_without_edges(monkeypatch, form):
+    """No edge and no room for one, in every form of the epochs: Y stays."""
+    from mlx_vis_b200 import _lib
+
+    monkeypatch.setenv("UMAPB_LAYOUT_ONE_LAUNCH", form)
+    one = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ne = torch.zeros(1, dtype=torch.int64, device="cuda")
+    lay = _lib.Layout(one, one, torch.zeros(1, device="cuda"), ne, 50, 2, 20)
+    lay.e_cap = 0
+    Y0 = cuda(np.random.default_rng(0).normal(size=(50, 2)).astype(np.float32))
+    Y = Y0.clone()
+    lay.epochs(Y, 0, 6, 1.577, 0.895, 1.0, 5, 3)
+    lay.check()
+    assert torch.equal(Y, Y0)
