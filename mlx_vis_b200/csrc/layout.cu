@@ -825,8 +825,8 @@ static unsigned epoch_grid(int64_t e_cap, int blocks_per_sm) {
   return (unsigned)(want < cap ? want : cap);
 }
 
-// The kernel compiled for 5 negatives runs at that rate unless the environment sets
-// UMAPB_LAYOUT_NEG5=0 (read per call): both kernels make the same draws and sums.
+// The kernels compiled for 5 negatives (of the launches and of the single launch) run at that rate
+// unless the environment sets UMAPB_LAYOUT_NEG5=0 (read per call): the same draws and sums.
 static bool neg5_kernel_enabled() {
   const char* e = getenv("UMAPB_LAYOUT_NEG5");
   return !(e && e[0] == '0' && e[1] == 0);
@@ -1077,7 +1077,7 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
   c.lr = learning_rate;
   c.k0 = (uint32_t)seed;
   c.k1 = (uint32_t)(seed >> 32);
-  const bool five = neg_rate == 5;
+  const bool five = neg_rate == 5 && layout::neg5_kernel_enabled();
   bool ok = false;
   switch (dim) {
     case 1: ok = layout::launch_resident<1, 0>(c, e_cap, stream); break;

@@ -220,30 +220,36 @@ def test_device_legacy_normal_equals_numpy(seed, shape, parallel):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
-def test_graph_epochs_match_launched_epochs(golden, manifest):
+def test_graph_epochs_match_launched_epochs(golden, manifest, monkeypatch):
     """umapb_layout_epochs_graph (recorded once, then updated in place for a new
-    layout) reaches the same coordinates as the launch-by-launch loop; float atomics
-    may add the moves of one point in another order, hence the tolerance."""
+    layout, and for another rate and seed) reaches the same coordinates as the
+    launch-by-launch loop; float atomics may add the moves of one point in another order, hence the
+    tolerance.  So few rows would otherwise be one launch, which records no graph."""
+    monkeypatch.setenv("UMAPB_LAYOUT_ONE_LAUNCH", "0")
     fz, opt = golden("fuzzy_gauss"), golden("optimize_gauss")
     m = manifest["optimize_gauss"]
-    outs = []
-    for graph in (False, True, True):  # the second graph call updates the cached executable
-        lay = _layout(fz)
-        Y = cuda(opt["Y_ep0"].copy())
-        lay.epochs(Y, 0, 6, m["a"], m["b"], 1.0, 5, 7, graph=graph)
-        outs.append(Y.cpu().numpy())
-    scale = float(np.abs(outs[0]).max())
-    assert np.abs(outs[0] - opt["Y_ep0"]).max() > 1e-3 * scale  # the epochs moved the points
-    for o in outs[1:]:
-        assert np.median(np.abs(o - outs[0])) < 1e-5 * scale
-        assert np.abs(o - outs[0]).max() < 1e-2 * scale
+    for rate, seed in ((1.0, 7), (0.5, 8)):
+        outs = []
+        for graph in (False, True, True):  # the second graph call updates the cached executable
+            lay = _layout(fz)
+            Y = cuda(opt["Y_ep0"].copy())
+            lay.epochs(Y, 0, 6, m["a"], m["b"], rate, 5, seed, graph=graph)
+            outs.append(Y.cpu().numpy())
+        scale = float(np.abs(outs[0]).max())
+        assert np.abs(outs[0] - opt["Y_ep0"]).max() > 1e-3 * scale  # the epochs moved the points
+        for o in outs[1:]:
+            assert np.median(np.abs(o - outs[0])) < 1e-5 * scale
+            assert np.abs(o - outs[0]).max() < 1e-2 * scale
 
 
+@pytest.mark.parametrize("form", ["", "0"])
 @pytest.mark.parametrize("dim", [2, 3])
-def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim):
+def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim, form):
     """At the default 5 negatives per edge the epochs run on a kernel compiled for that
-    rate (UMAPB_LAYOUT_NEG5=0 selects the general kernel): both draw the same tails and
-    make the same sums, so only the order of the float atomics may differ."""
+    rate (UMAPB_LAYOUT_NEG5=0 selects the general kernel), in one launch and by launches:
+    both draw the same tails and make the same sums, so only the order of the float atomics
+    may differ."""
+    monkeypatch.setenv("UMAPB_LAYOUT_ONE_LAUNCH", form)
     fz, opt = golden("fuzzy_gauss"), golden("optimize_gauss")
     m = manifest["optimize_gauss"]
     Y0 = opt["Y_ep0"]
