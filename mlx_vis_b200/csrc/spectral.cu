@@ -570,11 +570,17 @@ __global__ void __launch_bounds__(kPowerThreads, 1)
 // cluster's hardware barrier.  The CTAs' Gram matrices are exchanged the same way and
 // added in rank order, without atomics.  B200, 2,000 rows, k = 15: 613 -> 325 us against 16
 // blocks over L2, where every iteration pays a round trip each for V and the barrier.
+// Eight SMs gather an edge a cycle each, the chip 148, so the form is for the rows that one pass of
+// the CTAs takes (2,048) as long as shared memory holds their edges, and for few edges in two
+// passes.  100 iterations, cluster and grid (its blocks by edges as below), 2 components: 2,048
+// rows, k = 15 363 and 486 us, k = 75 814 and 875, k = 90 (not all staged) 1062 and 980; 3,000 rows,
+// k = 12 470 and 480; 4,000 rows, k = 10 493 and 499, k = 15 525 and 490; 5,000 rows, k = 50 2166 and 749.
 constexpr int kClusterCtas = 8;
 constexpr int kClusterThreads = 544;  // 16 warps with rows and the factor warp
 constexpr int kClusterRowThreads = kClusterThreads - 32;
 constexpr size_t kClusterSmem = 216 * 1024;
-constexpr size_t kClusterVBytes = 160 * 1024;  // both buffers of V: up to 5,120 rows of 16 bytes
+constexpr int kClusterPass = kClusterCtas * kClusterRowThreads / kLanes;  // rows of one pass
+constexpr int64_t kClusterTwoPassEdges = 40000;  // rows of 16 bytes (up to 3 components) only
 
 template <int KK>
 __global__ void __launch_bounds__(kClusterThreads, 1)
@@ -720,18 +726,20 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   for (int t = threadIdx.x; t < rows * (vp / 4); t += kClusterThreads) out[t] = mine[t];
 }
 
-// Enqueues the cluster form when V and the edge offsets fit; false: use another form.
+// Enqueues the cluster form where it is the faster one; false: use another form.
 template <int KK>
 static bool launch_power_cluster(const int64_t* row_ptr, const int32_t* cols, const float* wn, int64_t e_cap,
                                  int64_t n, int n_iter, float* V0, float* V1, double* Rinv, cudaStream_t stream) {
   constexpr int vp = KK <= 4 ? 4 : 8;
-  const size_t v_bytes = 2 * (size_t)n * vp * sizeof(float);
-  if (v_bytes > kClusterVBytes) return false;
+  const bool one_pass = n <= kClusterPass;
+  if (!one_pass && (KK > 4 || n > 2 * kClusterPass || e_cap > kClusterTwoPassEdges)) return false;
+  const size_t v_bytes = 2 * (size_t)n * vp * sizeof(float);  // at most 128 KB
   const int per = (int)ceil_div(n, kClusterCtas);
   const size_t fixed = v_bytes + ((size_t)per + 1) * 4;
   // a CTA's share of the edges, and half as many again for uneven rows; the rest from L2
   int64_t cap = e_cap / kClusterCtas + e_cap / kClusterCtas / 2 + 64;
   const int64_t room = (int64_t)(kClusterSmem - fixed) / 8;
+  if (one_pass && ceil_div(e_cap, kClusterCtas) > room) return false;
   if (cap > room) cap = room;
   const size_t smem = fixed + (size_t)cap * 8;
   {
@@ -987,7 +995,7 @@ extern "C" int umapb_spectral(const int32_t* rows, const int32_t* cols, const fl
   UMAPB_LAUNCH_CHECK("spectral: setup kernels");
   const unsigned pb = (unsigned)ceil_div(n * spectral::kLanes, spectral::kBlock);
   // one cooperative launch for all iterations, one resident block per SM, fewer when that
-  // would leave a block less than a row per lane pair (a smaller barrier); the
+  // would leave a block little to do (a smaller barrier); the
   // per-iteration launches remain for devices that refuse it and behind
   // UMAPB_SPECTRAL_COOP=0
   int coop = 0, dev = 0;
@@ -1012,8 +1020,15 @@ extern "C" int umapb_spectral(const int32_t* rows, const int32_t* cols, const fl
                      : kk == 3 ? (const void*)spectral::power_kernel<3>
                      : kk == 4 ? (const void*)spectral::power_kernel<4>
                                : (const void*)spectral::power_kernel<5>;
-    const int64_t min_rows = spectral::kPowerRowThreads / spectral::kLanes / 2;
+    // A block for every 248 rows (half a pass; 124 of the wider rows, whose FP64 arithmetic is
+    // longer) and for every 2,048 edges, which an SM gathers in about a microsecond: by rows alone a
+    // few SMs had all edges of a wide neighbourhood.  100 iterations, 2 components, by
+    // rows alone and now: 5,121 rows, k = 50 1007 -> 744 us, k = 100 2610 -> 1084; 20,000 rows, k = 50
+    // 1039 -> 853; 10,000 rows, k = 15 554 -> 503; 4 components, 10,000 rows, k = 10 898 -> 760.
+    const int64_t min_rows = spectral::kPowerRowThreads / spectral::kLanes / (kk > 4 ? 4 : 2);
     int64_t grid = ceil_div(n, min_rows);
+    if (ceil_div(e_cap, 2048) > grid) grid = ceil_div(e_cap, 2048);
+    if (grid > ceil_div(n, 16)) grid = ceil_div(n, 16);  // a warp's rows at least
     if (grid > num_sms()) grid = num_sms();
     int per = (int)ceil_div(n, grid);
     grid = ceil_div(n, per);

@@ -269,10 +269,13 @@ def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim, 
 
 
 @pytest.mark.parametrize("n,k,dim", [(17, 16, 2), (300, 5, 1), (300, 40, 4), (2560, 12, 4), (2561, 12, 4),
-                                     (5120, 9, 2), (5121, 9, 2), (9000, 24, 3), (6000, 140, 2)])
+                                     (5120, 9, 2), (5121, 9, 2), (9000, 24, 3), (6000, 140, 2), (2048, 40, 2), (2048, 60, 4),
+                                     (2049, 9, 4), (2049, 60, 3), (4096, 16, 3), (4097, 16, 2), (2000, 100, 2),
+                                     (2000, 200, 2), (33, 300, 2)])
 def test_power_iteration_forms_match_float64(n, k, dim):
-    """The cluster form (up to 5,120 rows of 16 bytes, 2,560 of 32) and the grid-wide one on
-    either side of their border, uneven row counts per CTA and more edges than a CTA's
+    """The cluster form (one pass of 2,048 rows whose edges fit shared memory; up to 4,096 rows of
+    16 bytes with 40,000 edges) and the grid-wide one (blocks by rows, by edges and by
+    warps) on either side of their borders, uneven row counts per CTA and more edges than a CTA's
     shared memory was sized for, against float64 torch.  FP32 storage of V leaves 100
     rounded steps: 1e-5 of the 0..10 range."""
     from mlx_vis_b200 import _lib
