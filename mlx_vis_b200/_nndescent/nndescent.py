@@ -56,6 +56,21 @@ def iteration_params(update_frac: float, k: int, mc: int):
     return min(mc_nn, k), j_nn, min(mc_conv, k)
 
 
+def pads_rows(n: int, d: int, k: int, mc: int) -> bool:
+    """Whether rows whose length is no multiple of four are padded for the FP32 joins.
+
+    The joins store every distance and read it back; the row kernel computes its candidates' and
+    keeps them.  The joins win by the distances they share, k^2 d a row, once there are
+    rows enough for their launches; with fewer sources than neighbours (mc < k) only for long
+    rows.  B200, builds with the row kernel alone and with the joins: 21,000 rows, k = 3, d = 17
+    1.43 and 1.61 ms, k = 5, d = 51 1.73 and 1.86, k = 8, d = 51 1.76 and 1.65, k = 16, d = 51 2.68
+    and 1.80, k = 5, d = 301 2.49 and 2.40; 3,000 rows, k = 8, d = 51 0.92 and 0.93; mc = 5 of
+    k = 16: 21,000 x 51 2.39 and 2.76, 21,000 x 301 3.63 and 3.65, 100,000 x 301 16.5 and 14.0."""
+    if mc >= k:
+        return n * k >= 40000 and (k >= 8 or (k >= 4 and k * k * d >= 7000))
+    return d >= 256 and n * d >= 6000000
+
+
 def state_words(state) -> np.ndarray:
     """np.random.get_state() as the uint32[628] buffer umapb_nnd_random_start reads."""
     name, key, pos, has_gauss, gauss = state[:5]
@@ -245,9 +260,9 @@ class NNDescent:
         join_on = os.environ.get("UMAPB_NND_JOIN", "1") != "0"
         nnbuf = curd = join_ws = None
         # FP32 rows for the joins, which read whole float4s: rows of another length are
-        # copied once to zero-padded ones
+        # copied once to zero-padded ones where that pays
         Xi, di = X, d
-        if join_on and k <= JOIN_MAX_K and d % 4 != 0:
+        if join_on and k <= JOIN_MAX_K and d % 4 != 0 and pads_rows(n, d, k, mc):
             di = (d + 3) // 4 * 4
             Xi = torch.empty((n, di), dtype=torch.float32, device=dev)
             call("umapb_nnd_pad_cols", ptr(X), n, d, di, ptr(Xi), s)
@@ -295,7 +310,7 @@ class NNDescent:
                 if use_rev:
                     call("umapb_nnd_reverse", P(idx), n, k, P(rev), P(rev_ws), rev_ws.numel(), s)
                 # the nn-of-nn distances of the NEW-first sources from the blocked join
-                join = join_on and k <= JOIN_MAX_K and mc_conv > 0 and j_nn > 0
+                join = join_on and k <= JOIN_MAX_K and mc_conv > 0 and j_nn > 0 and di % 4 == 0
                 if join and nnbuf is None:
                     nnbuf = torch.empty(n * k * k, dtype=torch.float32, device=dev)
                     curd = torch.empty((n, k), dtype=torch.float32, device=dev)
@@ -319,7 +334,7 @@ class NNDescent:
                     Xd, sqd = Xi, sq
                 use_half = it in (1, 2, 3, 4)
                 recompute = (it == 0) or use_half
-                join = join_on and k <= JOIN_MAX_K and mc_nn > 0
+                join = join_on and k <= JOIN_MAX_K and mc_nn > 0 and (use_half or Xd.shape[1] % 4 == 0)
                 if fp32_due:
                     if not (Xd is Xi and not use_half and join and mc_nn == k):
                         call("umapb_nnd_gather", P(X), P(sq), n, d, P(idx), P(dist), k, 0, s)
@@ -369,8 +384,9 @@ class NNDescent:
                 info = dict(path="full", mc_new=mc_nn, j_nn=j_nn, use_rev=use_rev, use_half=use_half, space=dd,
                             elem=2 if use_half else 4, join=join)
             # the buckets of the next full iteration's join follow from the new lists alone: made
-            # while the host reads the count, unless the search is about to leave the full path
-            if select and update_frac >= 0.6 and it + 1 < self.n_iters:
+            # while the host reads the count, unless the search is about to leave the full path or the
+            # next iteration (FP32 after the fourth) has no join
+            if select and update_frac >= 0.6 and it + 1 < self.n_iters and (it < 4 or di % 4 == 0):
                 call("umapb_nnd_join_prepare", P(idx2), P(order), n, k, k, P(join_ws), join_ws.numel(), s)
                 prepared = True
             if it == 0 and while_first_iteration is not None:

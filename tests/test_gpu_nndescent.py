@@ -426,24 +426,43 @@ def test_select_matches_the_general_row_update(n, k, j_nn, recompute, use_rev):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("n,k,padded", [(1500, 12, False), (4000, 12, True)])
 @pytest.mark.parametrize("d", [5, 50, 102])
-def test_rows_that_are_not_whole_float4s(d):
-    """Row lengths that are not a multiple of four go through the joins on zero-padded
-    copies: the same graph as without the join, but for ties in the FP32 sums."""
+def test_rows_that_are_not_whole_float4s(d, n, k, padded):
+    """Row lengths that are not a multiple of four go through the FP32 joins on zero-padded
+    copies where that pays and without those joins elsewhere: the same graph as without any
+    join, but for ties in the FP32 sums."""
     import os
 
     from mlx_vis_b200 import NNDescent
+    from mlx_vis_b200._nndescent.nndescent import pads_rows
 
-    X = np.random.default_rng(d).integers(-40, 41, size=(1500, d)).astype(np.float32)  # exact FP32 distances
-    idx, dist = NNDescent(k=12, random_state=3, n_iters=1).build(X)
+    assert pads_rows(n, d, k, k) == padded
+    X = np.random.default_rng(d).integers(-40, 41, size=(n, d)).astype(np.float32)  # exact FP32 distances
+    nn = NNDescent(k=k, random_state=3, n_iters=1)
+    idx, dist = nn.build(X)
+    assert nn.history_[0]["join"] == (padded or d > 100)  # d > 100: in 100 projected columns
     os.environ["UMAPB_NND_JOIN"] = "0"
     try:
-        idx0, dist0 = NNDescent(k=12, random_state=3, n_iters=1).build(X)
+        idx0, dist0 = NNDescent(k=k, random_state=3, n_iters=1).build(X)
     finally:
         del os.environ["UMAPB_NND_JOIN"]
     # d > 100: the first iteration runs on the rounded products with the random projection
     assert np.mean(idx != idx0) <= (0.002 if d > 100 else 0.0)
     np.testing.assert_allclose(dist, dist0, rtol=1e-5 if d > 100 else 0.0)
+
+
+@pytest.mark.parametrize("d", [17, 50])
+@pytest.mark.parametrize("k,mc", [(5, None), (12, None), (12, 5), (30, None)])
+def test_short_rows_track_the_oracle(d, k, mc):
+    """Whole builds of rows that are not whole float4s, with padded FP32 joins (k = 30) and without
+    (FP16 iterations on joins, FP32 ones in the row kernel), against the oracle."""
+    from mlx_vis_b200 import NNDescent, datasets
+
+    X = datasets.gaussian_mixture(2500, d, seed=k)
+    idx, _ = NNDescent(k=k, max_candidates=mc, random_state=5).build(X)
+    oi, _ = onnd.build(X, k=k, max_candidates=mc, random_state=5)
+    assert recall(idx, oi) > 0.98
 
 
 def _opposite_rows(n, d, kind, rng):
