@@ -18,8 +18,8 @@
 // What bounds it: instructions (a few hundred per row); ids of rejected candidates are
 // never read.  Against collecting every id and removing duplicates through a hash table
 // first (and a separate kernel for the reverse slots), B200, row updates of the full
-// path: 70000 x 784, k = 15 7 x 415 -> 7 x 139 us; 1000000 x 128, k = 15 7 x 5.2 -> 7 x
-// 2.0 ms; 30001 x 50, k = 30 4 x 1500 -> 4 x 351 us.
+// path: 70000 x 784, k = 15 7 x 415 -> 7 x 125 us; 1000000 x 128, k = 15 7 x 5.2 -> 7 x
+// 1.73 ms; 30001 x 50, k = 30 4 x 1500 -> 4 x 340 us.
 #include <math.h>
 
 #include "common.cuh"
@@ -31,6 +31,8 @@ namespace nnd {
 
 constexpr int kSelWarps = 4;
 constexpr unsigned kAll = 0xffffffffu;
+// mark of a candidate that is absent or taken: a NaN, neither below nor at any distance
+__device__ __forceinline__ float gone() { return __int_as_float(0x7fffffff); }
 
 // NCH: registers of 32 nn-of-nn candidates (k * j_nn <= 32 NCH)
 template <int NCH>
@@ -45,22 +47,22 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
   const unsigned below = (1u << lane) - 1u;
 
   const int my_old = lane < k ? a.idx_old[row * k + lane] : -1;
-  const float my_d = lane < k ? to_key((a.curd ? a.curd : a.dist_old)[row * k + lane]) : 0.f;
-  float d[NCH];  // keys of the nn-of-nn candidates; INFINITY, above every key: absent or taken
+  const float my_d = lane < k ? (a.curd ? a.curd : a.dist_old)[row * k + lane] : 0.f;
+  float d[NCH];  // nn-of-nn candidates; gone(): absent or taken
   const float* nn = a.nnbuf + row * nn_cols;
 #pragma unroll
-  for (int u = 0; u < NCH; ++u) d[u] = u * 32 + lane < nn_cols ? to_key(nn[u * 32 + lane]) : INFINITY;
+  for (int u = 0; u < NCH; ++u) d[u] = u * 32 + lane < nn_cols ? nn[u * 32 + lane] : gone();
 
   // reverse candidates, one per lane: id rid at distance rd
   int rid = -1, pads = 0;  // pads: empty slots
-  float rd = INFINITY;
+  float rd = gone();
   if (a.off) {
     const int o = a.off[row], cnt = a.off[row + 1] - o;
     pads = cnt < k ? k - cnt : 0;
     if (cnt <= 32) {
       if (lane < cnt) {
         rid = a.entries[o + lane] >> 5;
-        rd = to_key(a.entd[o + lane]);
+        rd = a.entd[o + lane];
       }
       if (cnt > k) {  // the k smallest ids
         int rank = 0;
@@ -68,39 +70,46 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
           const int id = __shfl_sync(kAll, rid, t);
           rank += id < rid || (id == rid && t < lane) ? 1 : 0;
         }
-        if (rank >= k) rid = -1, rd = INFINITY;
+        if (rank >= k) rid = -1, rd = gone();
       } else if (lane == cnt && pads) {
         rid = 0;
-        rd = to_key(a.d0[row]);
+        rd = a.d0[row];
       }
-    } else {  // a hub: the k-th smallest id by bisection over the ids
-      int lo = 0, hi = (int)a.n - 1;
-      while (lo < hi) {
-        const int mid = lo + (hi - lo) / 2;
-        int c = 0;
-        for (int e = lane; e < cnt; e += 32) c += (a.entries[o + e] >> 5) <= mid ? 1 : 0;
-        if ((int)__reduce_add_sync(kAll, (unsigned)c) >= k) hi = mid;
-        else lo = mid + 1;
-      }
-      int base = 0;
-      for (int eq = 0; eq < 2; ++eq) {  // the smaller ids, then copies of the k-th
-        for (int e0 = 0; e0 < cnt && base < k; e0 += 32) {
-          const int e = e0 + lane;
-          const int id = e < cnt ? a.entries[o + e] >> 5 : 0x7fffffff;
-          const bool take = eq ? id == hi : id < hi;
-          const unsigned b = __ballot_sync(kAll, take);
-          const int p = base + __popc(b & below);
-          if (take && p < k) s_c[warp][p] = e;
-          base += __popc(b);
+    } else {
+      // a hub: its k smallest ids in one pass, as a list of (id, entry) over the lanes in which
+      // earlier copies of an id come first; the ids arrive nearly ascending, so few enter
+      // (bisecting the ids took 17 passes, and one row listed by thousands held up the grid: 100,000 x
+      // 51, k = 2 420 -> 142 us)
+      int hid = 0x7fffffff, he = 0, worst = 0x7fffffff;
+      for (int e0 = 0; e0 < cnt; e0 += 128) {
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int e = e0 + 32 * u + lane;
+          v[u] = e < cnt ? a.entries[o + e] >> 5 : 0x7fffffff;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          unsigned b = __ballot_sync(kAll, v[u] < worst);
+          while (b) {
+            const int s = __ffs(b) - 1;
+            const int id = __shfl_sync(kAll, v[u], s);
+            const int at = __popc(__ballot_sync(kAll, lane < k && hid <= id));
+            const int up_id = __shfl_up_sync(kAll, hid, 1), up_e = __shfl_up_sync(kAll, he, 1);
+            if (lane < k && lane >= at) {
+              hid = lane == at ? id : up_id;
+              he = lane == at ? e0 + 32 * u + s : up_e;
+            }
+            worst = __shfl_sync(kAll, hid, k - 1);
+            b &= b - 1u;
+            b &= __ballot_sync(kAll, v[u] < worst);
+          }
         }
       }
-      __syncwarp();
-      if (lane < k) {
-        const int e = s_c[warp][lane];
-        rid = a.entries[o + e] >> 5;
-        rd = to_key(a.entd[o + e]);
+      if (lane < k) {  // more entries than k, so the list is full
+        rid = hid;
+        rd = a.entd[o + he];
       }
-      __syncwarp();
     }
   }
 
@@ -120,8 +129,8 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
   float tau = __shfl_sync(kAll, lv, k - 1);
   int tau_i = __shfl_sync(kAll, li, k - 1);
 
-  // tau is at most kSent, below INFINITY, so a turn counts untaken candidates only and takes at
-  // least one of them
+  // gone() is not <= tau, whatever tau is: a turn counts untaken candidates only and takes at least
+  // one of them
   while (true) {
     int c = rd <= tau ? 1 : 0;
 #pragma unroll
@@ -130,10 +139,10 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
     if (c == 0) break;
     float T = tau;
     // a band of at least kBandMin candidates where possible: a step costs NCH compares, a short
-    // band may leave the list to be settled by another one (B200, 1,000,000 rows, k = 15: 1.96 ms
-    // at 12, 1.85 at 20, 1.86 at 26; 30,000 rows, k = 30: 351 us at 12, 362 at 20, 432 at 26)
+    // band may leave the list to be settled by another one (B200, earlier form, 1,000,000 rows, k = 15:
+    // 1.96 ms at 12, 1.85 at 20, 1.86 at 26; 30,000 rows, k = 30: 351 us at 12, 362 at 20, 432 at 26)
     constexpr int kBandMin = NCH <= 8 ? 20 : 12;
-    if (c > 32) {  // the bits of non-negative floats order like the values
+    if (c > 32) {  // the bits of non-negative floats (and of gone()) order like the values
       uint32_t mn = __float_as_uint(rd);
 #pragma unroll
       for (int u = 0; u < NCH; ++u) mn = min(mn, __float_as_uint(d[u]));
@@ -166,7 +175,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
       if (take && p < 32) {
         s_d[warp][p] = d[u];
         s_c[warp][p] = u * 32 + lane;
-        d[u] = INFINITY;
+        d[u] = gone();
       }
       base += __popc(b);
     }
@@ -177,7 +186,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
       if (take && p < 32) {
         s_d[warp][p] = rd;
         s_c[warp][p] = NCH * 32 + lane;
-        rd = INFINITY;
+        rd = gone();
       }
       base += __popc(b);
     }
@@ -270,7 +279,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_kernel(SelectArgs 
 
   if (lane < k) {
     a.idx_new[row * k + lane] = li;
-    a.dist_new[row * k + lane] = from_key(lv);
+    a.dist_new[row * k + lane] = lv;
     a.flags_new[row * k + lane] = li != my_old ? 1 : 0;
   }
   const int nch = __popc(__ballot_sync(kAll, lane < k && li != my_old));

@@ -9,15 +9,10 @@ namespace umapb {
 namespace nnd {
 
 constexpr float kBig = 1e30f;         // distance of a dropped column (the row itself, a repeated id)
-constexpr float kSent = kBig * 4.0f;  // above every real key, including 1e30 entries
-// The largest key of a real candidate.  Distances can be infinite (an FP16 dot product below
-// -65,504, an FP32 overflow); as keys they are held below the sentinels, so that a list of
-// k candidates never ends in one, and become infinite again in the stored lists.
-constexpr float kMaxKey = 0x1.93e592p+101f;  // the float below kSent
-static_assert(kMaxKey < kSent && kMaxKey > 3.9e30f, "the float below kSent");
-
-__device__ __forceinline__ float to_key(float d) { return fminf(d, kMaxKey); }
-__device__ __forceinline__ float from_key(float key) { return key < kMaxKey ? key : INFINITY; }
+// Behind a list of fewer than 32 keys: (INFINITY, 0x7fffffff), above every key.  Distances can be
+// infinite themselves (an FP16 dot product below -65,504, an FP32 overflow), so a mark that
+// a kernel compares with them has to be a NaN.
+constexpr float kSent = INFINITY;
 
 __device__ __forceinline__ bool key_lt(float a, int ia, float b, int ib) {
   return a < b || (a == b && ia < ib);

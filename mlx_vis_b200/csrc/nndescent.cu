@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) iter_kernel(IterArgs a) {
   int tau_i = li;
   for (int t0 = 0; t0 < a.tcap; t0 += 32) {
     const int t = t0 + lane;
-    float d = t < T_total ? to_key(cd[t]) : kSent;
+    float d = t < T_total ? cd[t] : kSent;
     int id = t < T_total ? cid[t] : 0x7fffffff;
     unsigned b = __ballot_sync(0xffffffffu, t < T_total && key_lt(d, id, tau, tau_i));
     if (__popc(b) > 10) {
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kWarps * 32, 10) iter_kernel(IterArgs a) {
   }
   if (lane < k) {
     a.idx_new[row * k + lane] = li;
-    a.dist_new[row * k + lane] = from_key(lv);
+    a.dist_new[row * k + lane] = lv;
     const bool ch = li != my_old;
     a.flags_new[row * k + lane] = ch ? 1 : 0;
   }
