@@ -1,6 +1,6 @@
 // Fuzzy simplicial set — replaces UMAP._fuzzy_simplicial_set, mlx_vis/_umap/umap.py:199-270.
 //
-// K1 weights:   2 or 8 lanes per row.  rho = max(min positive distance, 1e-8)
+// K1 weights:   1 to 8 lanes per row.  rho = max(min positive distance, 1e-8)
 //               (umap.py:211-214); sigma by the reference's bisection
 //               (umap.py:217-236: lo 1e-20, hi 1e3, sigma 1, 64 steps, target
 //               log2 k over columns 1..k-1, converged when |sum - target| < 1e-5;
@@ -35,9 +35,9 @@ __device__ __forceinline__ float dev_exp<float>(float x) { return expf(x); }
 // A row's bisection is a serial chain of up to 64 steps, each a sum of k - 1
 // exponentials.  LANES lanes share a step's exponentials; their gaps d - rho stay in
 // registers (the first 8 of a lane) and one reciprocal of sigma serves them all.  Many rows
-// are bound by the FP64 units, so 2 lanes (the bisection's own arithmetic is
-// repeated in every lane); few rows by the chain, so 8.  B200, k = 15: 70,000 rows 82 -> 67
-// us (2 lanes), 2,000 rows 58 -> 18 us (8 lanes) against one thread per row.
+// are bound by the FP64 units, and the bisection's own arithmetic is repeated in every lane, so they
+// take one lane; few rows are bound by the chain.  B200, k = 15: 2,000 rows 61 -> 18 us (8
+// lanes), 70,000 rows 82 -> 57 us (1 lane) against one thread that divides at every neighbour.
 template <class T, int LANES>
 __global__ void weights_kernel(const float* __restrict__ knn_dist, int64_t n, int k, float* __restrict__ w,
                                float* __restrict__ rho_out, float* __restrict__ sigma_out) {
@@ -111,12 +111,23 @@ __global__ void weights_kernel(const float* __restrict__ knn_dist, int64_t n, in
 template <class T>
 static void launch_weights(const float* knn_dist, int64_t n, int k, float* w, float* rho_out, float* sigma_out,
                            cudaStream_t stream) {
-  const bool few = n * 8 < (int64_t)num_sms() * 2048;  // 8 lanes a row still fit the chip at once
-  const unsigned blocks = (unsigned)ceil_div(n * (few ? 8 : 2), kBlock);
-  if (few)
-    weights_kernel<T, 8><<<blocks, kBlock, 0, stream>>>(knn_dist, n, k, w, rho_out, sigma_out);
+  // Kernel times in us at 1 / 2 / 4 / 8 lanes.  k = 3: 2,000 rows 12.6 / 13.6 / 14.3 / 14.7, 70,000 15.8 /
+  // 29 / 46 / 79.  k = 15: 10,000 rows 45 / 29 / 25 / 24, 20,000 46 / 34 / 34 / 41, 37,000 46 / 36 / 50 /
+  // 62, 70,000 57 / 66 / 84 / 112.  k = 30: 20,000 rows 99 / 68 / 54 / 55, 70,000 121 / 134 / 131 / 155.
+  // k = 50: 20,000 rows 170 / 112 / 85 / 77, 200,000 540 / 521 / 536 / 587.  k = 100: 70,000 rows 503 / 450 /
+  // 389 / 371.
+  int lanes = 1;
+  if (n < 16384)
+    lanes = k < 5 ? 1 : 8;
+  else if (n < 40000)
+    lanes = k < 5 ? 1 : k < 20 ? 2 : k < 40 ? 4 : 8;
   else
-    weights_kernel<T, 2><<<blocks, kBlock, 0, stream>>>(knn_dist, n, k, w, rho_out, sigma_out);
+    lanes = k < 40 ? 1 : k < 64 ? 2 : 8;
+  const auto kernel = lanes == 1   ? weights_kernel<T, 1>
+                      : lanes == 2 ? weights_kernel<T, 2>
+                      : lanes == 4 ? weights_kernel<T, 4>
+                                   : weights_kernel<T, 8>;
+  kernel<<<(unsigned)ceil_div(n * lanes, kBlock), kBlock, 0, stream>>>(knn_dist, n, k, w, rho_out, sigma_out);
 }
 
 __device__ __forceinline__ void atomic_max_nonneg(float* addr, float v) {

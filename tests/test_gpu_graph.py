@@ -305,10 +305,12 @@ def test_power_iteration_forms_match_float64(n, k, dim):
     assert np.abs(Y - want).max() < 1e-4
 
 
-@pytest.mark.parametrize("n,k", [(40, 2), (333, 9), (333, 10), (1000, 66), (40000, 17), (40000, 18)])
+@pytest.mark.parametrize("n,k", [(40, 2), (333, 9), (333, 10), (1000, 66), (40000, 17), (40000, 18), (1000, 4),
+                                 (40001, 9), (40001, 10), (16384, 16), (16385, 18), (20001, 20), (20001, 34), (20001, 40),
+                                 (40001, 41), (40001, 64)])
 def test_fuzzy_lanes_match_float64(n, k):
-    """The bisection with 8 lanes per row (few rows) and 2 (many): neighbours on either side
-    of the gaps a lane keeps in registers, rows with equal and with zero distances."""
+    """The bisection with 1, 2, 4 and 8 lanes per row, by rows and neighbours: neighbours on either
+    side of the gaps a lane keeps in registers, rows with equal and with zero distances."""
     rng = np.random.default_rng(n + k)
     dist = np.sort(rng.uniform(0.5, 3.0, size=(n, k)), axis=1).astype(np.float32)
     dist[::7, : k // 2] = 0.0
