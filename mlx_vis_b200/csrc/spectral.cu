@@ -430,7 +430,11 @@ __device__ __forceinline__ double block_gram(const double (&part)[KK * KK], doub
 
 constexpr int kPowerThreads = 1024;  // two lanes for each of 496 rows (one pass up to 73,408 rows) and the factor warp
 constexpr int kPowerRowThreads = kPowerThreads - 32;
-constexpr size_t kPowerSmem = 200 * 1024;  // dynamic shared memory at most
+// Dynamic shared memory at most: with the static part within the 196 KB setting of an SM, which
+// leaves L1 60 KB.  The next setting leaves 28, too little for the gathers in flight: 100 iterations
+// of 150,000 rows, k = 20, 2 components, 200 KB and 188 KB 2628 and 1765 us; 300,000 rows, k = 10, 4
+// components 5764 and 3895.
+constexpr size_t kPowerSmem = 188 * 1024;
 
 template <int KK>  // columns of V: n_components + 1
 __global__ void __launch_bounds__(kPowerThreads, 1)

@@ -271,7 +271,7 @@ def test_neg5_kernel_matches_general_kernel(golden, manifest, monkeypatch, dim, 
 @pytest.mark.parametrize("n,k,dim", [(17, 16, 2), (300, 5, 1), (300, 40, 4), (2560, 12, 4), (2561, 12, 4),
                                      (5120, 9, 2), (5121, 9, 2), (9000, 24, 3), (6000, 140, 2), (2048, 40, 2), (2048, 60, 4),
                                      (2049, 9, 4), (2049, 60, 3), (4096, 16, 3), (4097, 16, 2), (2000, 100, 2),
-                                     (2000, 200, 2), (33, 300, 2)])
+                                     (2000, 200, 2), (33, 300, 2), (60000, 130, 1)])
 def test_power_iteration_forms_match_float64(n, k, dim):
     """The cluster form (one pass of 2,048 rows whose edges fit shared memory; up to 4,096 rows of
     16 bytes with 40,000 edges) and the grid-wide one (blocks by rows, by edges and by
