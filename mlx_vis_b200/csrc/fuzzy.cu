@@ -144,7 +144,8 @@ __global__ void symmetrize_kernel(const int32_t* __restrict__ knn_idx, const flo
     const int32_t j = knn_idx[e];
     const float we = w[e];
     float wr = 0.f;
-    if (j >= 0 && j < n) {
+    const bool known = j >= 0 && j < n;  // the kNN search marks a missing neighbour by an id beyond the rows
+    if (known) {
       // eight entries at a time, their loads in flight together; the first match counts
       const int32_t* rj = knn_idx + (int64_t)j * k;
       int pos = -1;
@@ -155,8 +156,8 @@ __global__ void symmetrize_kernel(const int32_t* __restrict__ knn_idx, const flo
       }
       if (pos >= 0) wr = w[(int64_t)j * k + pos];
     }
-    v = __fsub_rn(__fadd_rn(we, wr), __fmul_rn(we, wr));
-    w_sym[e] = v;
+    v = known ? __fsub_rn(__fadd_rn(we, wr), __fmul_rn(we, wr)) : 0.f;
+    w_sym[e] = known ? v : -1.f;  // below every threshold: no edge to a row that does not exist
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));

@@ -433,3 +433,34 @@ def test_layout_without_edges(monkeypatch, form):
     lay.epochs(Y, 0, 6, 1.577, 0.895, 1.0, 5, 3)
     lay.check()
     assert torch.equal(Y, Y0)
+
+
+def test_fuzzy_drops_missing_neighbours():
+    """Where scores overflow, the exact search fills a row with the id 0x7fffffff at an infinite distance:
+    no edge points there, and the others keep their weights."""
+    n, k = 300, 6
+    rng = np.random.default_rng(1)
+    idx = ((np.arange(n)[:, None] + 1 + np.arange(k)) % n).astype(np.int32)
+    dist = np.sort(rng.uniform(0.5, 3.0, size=(n, k)), axis=1).astype(np.float32)
+    idx[:20], dist[:20] = 0x7FFFFFFF, np.inf  # rows without any neighbour
+    idx[20:40, -1], dist[20:40, -1] = 0x7FFFFFFF, np.inf  # and with one less
+    idx[40, -1] = -1
+    (r, c, v), _ = gpu_fuzzy(idx, dist, 200, fp64=True)
+    assert c.min() >= 0 and c.max() < n and r.min() >= 20 and not np.isnan(v).any()
+    whole = ((np.arange(n)[:, None] + 1 + np.arange(k)) % n).astype(np.int32)
+    (ro, co, vo), _ = ofz.fuzzy_simplicial_set(whole, np.where(np.isinf(dist), np.float32(1e6), dist), 200,
+                                               dtype=np.float64)
+    # rows at a distance from the altered ones, whose neighbours are as they were
+    a, b = (r >= 60) & (r < n - 10), (ro >= 60) & (ro < n - 10)
+    assert np.array_equal(r[a], ro[b]) and np.array_equal(c[a], co[b])
+    np.testing.assert_allclose(v[a], vo[b], rtol=1e-6)
+
+
+def test_fit_of_rows_that_overflow():
+    """Squared norms beyond FP32 leave rows without neighbours: the fit ends with every other row embedded."""
+    from mlx_vis_b200 import UMAP
+
+    X = np.random.default_rng(0).normal(size=(400, 12)).astype(np.float32)
+    X[::40] *= 1e25
+    Y = UMAP(n_epochs=20, knn_method="brute", random_state=0).fit_transform(X)
+    assert Y.shape == (400, 2)
