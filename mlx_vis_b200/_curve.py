@@ -6,7 +6,7 @@ Gauss-Newton in float64 on 300 points of [0, 3 spread], starting at a = b = 1,
 each step the least-squares solution of J step = -residual (numpy.linalg.lstsq),
 at most 100 steps, stopping once |step|^2 < 1e-12.  Like the reference, a fit
 that diverges surfaces numpy.linalg.LinAlgError from lstsq.  Host-side scalar
-work: it runs once per fit and costs microseconds.
+work: it runs once per fit and costs about 0.4 ms, while the device works on the start.
 """
 
 from __future__ import annotations

@@ -13,7 +13,7 @@ Pipeline, all on the GPU through libumap_b200:
   -> layout epochs (exact float32 schedule, synchronous SGD): few rows in one
      launch; else two overlapping launches per epoch, run as one CUDA graph that the
      library records and updates per fit.
-Host work left: the a/b curve fit (float64, microseconds); the NumPy streams the
+Host work left: the a/b curve fit (float64, 0.4 ms); the NumPy streams the
 reference draws from are seeded on the host and drawn on the device.
 
 New keyword arguments (defaults keep the reference behaviour):

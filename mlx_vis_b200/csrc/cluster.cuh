@@ -37,9 +37,5 @@ __device__ __forceinline__ uint32_t peer(uint32_t smem, uint32_t rank) {
   return r;
 }
 
-__device__ __forceinline__ void store(uint32_t at, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
-}
-
 }  // namespace cluster
 }  // namespace umapb

@@ -366,9 +366,11 @@ __global__ void apply_kernel(float* Y, float* dY, int64_t m) {
 // and the share in one SM's shared memory (about 22,000 rows of two components).
 // Y and the schedule are written at the end only, and a barrier that gives up gives up for every
 // CTA, so after an expired wait both are as they were before the launch.
-// B200, per epoch, k = 15 where not said: 600 points, k = 5 8.0 -> 3.4 us (3.9 as a grid);
-// 1,000 points 4.0 either way; 2,000 points 6.7 -> 4.1 us (5.3 as a cluster); 4,000 points
-// 6.9 -> 4.8; 9,999 points, k = 10 8.4 -> 5.9; 20,000 points 9.8 -> 8.8.
+// B200, per epoch, overlapping launches and one: 600 points, k = 5 8.3 and 3.7 us (4.1 as a grid);
+// 1,000, k = 12 7.5 and 4.2 (either way); 2,000, k = 15 6.6 and 4.3 (5.3 as a cluster); 9,999, k = 10 8.5
+// and 6.0; 10,000, k = 100 10.8 and 8.7; 20,000, k = 5 9.6 and 7.6, k = 15 9.0 either way, k = 28 at 0 / 5 /
+// 10 negatives 8.5 / 11.3 / 16.6 and 9.1 / 10.7 / 13.6; 12,500, k = 24, 3 components 13.0 and 10.7; 9,500, k =
+// 40, 4 components 9.3 and 8.9: what fits is at worst a few percent slower than the launches.
 // (Moves added in the owners' shared memory took 23 us an epoch: float adds there are
 // compare-and-swap loops, remote ones a round trip a try.  Owners that apply their rows and
 // store them into all copies need a second barrier: 6.3 us.)
@@ -1049,8 +1051,8 @@ static bool enqueue_cluster(float* Y, int64_t n, int32_t dim, const int32_t* row
   // below four epochs the load of the edges and the store of their schedule cost more than the
   // launches (a callback after every epoch runs them one by one)
   // (above a million epochs the barrier's count would run into its top bit)
-  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4 || epoch_end - epoch_begin > 1000000 ||
-      layout::one_launch_is("0"))
+  if (!layout::resident_rows(n, dim) || epoch_end - epoch_begin < 4 ||
+      epoch_end - epoch_begin > 1000000 || layout::one_launch_is("0"))
     return false;
   const layout::Params p = layout::make_params(a, b, learning_rate, 0, n_epochs);
   layout::ClusterArgs c = {};

@@ -75,10 +75,11 @@ __global__ void convert_rows_kernel(const float* __restrict__ X, const int64_t* 
   }
 }
 
-// Y[b] = H[b] . W^T + bias for Hd a multiple of 256 up to 1024 (WORDS 16-byte words of a row per
-// lane) and 16-byte aligned rows: a lane keeps its columns of W in registers for all
-// the rows its warp takes, so a row costs its own bytes and one butterfly.  16384 rows x
-// 512, c = 2: 8 us against 15 when every 8 rows staged W in shared memory again.
+// Y[b] = H[b] . W^T + bias for Hd = 256 WORDS (WORDS 16-byte words of a row per lane) and 16-byte
+// aligned rows: a lane keeps its columns of W in registers for all the rows its warp takes, so
+// a row costs its own bytes and one butterfly.  Built for the default width, 512,
+// alone; other widths take the kernel below.  16384 rows, c = 2: 8 us against 15 when every 8 rows
+// staged W in shared memory again.
 template <int C, int WORDS>
 __global__ void __launch_bounds__(256) head_rows_kernel(const __nv_bfloat16* __restrict__ H, int ldh, int B, int Hd,
                                                         const float* __restrict__ W, const float* __restrict__ bias,
