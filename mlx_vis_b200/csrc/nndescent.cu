@@ -556,7 +556,7 @@ struct JoinArgs {
   int half_round;
   float* nnbuf;  // (n, mc * j_nn)
   float* curd;   // (n, k), nullable: current-neighbour distances not wanted
-  float* entd;   // the same distances in bucket order (one per entry)
+  float* entd;   // nullable: the same distances in bucket order (one per entry)
   unsigned long long* evals;  // nullable
 };
 
@@ -570,10 +570,8 @@ __device__ __forceinline__ void join_store(const JoinArgs& a, int64_t s, int e, 
   const int cid = join_col_id(a, s, col);
   const float d = d2_from_dot(a.sqd[i], a.sqd[cid], dot, a.half_round != 0);
   if (col == 0) {
-    if (a.curd) {
-      a.curd[i * a.k + p] = d;
-      a.entd[e] = d;
-    }
+    if (a.curd) a.curd[i * a.k + p] = d;
+    if (a.entd) a.entd[e] = d;
   } else {
     a.nnbuf[i * (int64_t)(a.mc * a.j_nn) + p * a.j_nn + (col - 1)] = d;
   }
@@ -1328,7 +1326,7 @@ static int join_impl(const void* Xd, const float* sqd, int32_t dd, int32_t ldx, 
   a.half_round = half;
   a.nnbuf = nnbuf;
   a.curd = curd;
-  a.entd = w.entd;
+  a.entd = flags ? nullptr : w.entd;  // the row update's reverse candidates
   a.evals = evals;
   const unsigned jb = (unsigned)ceil_div(w.max_chunks, nnd::kWarps);  // warps past the chunk count exit
   if (half) {

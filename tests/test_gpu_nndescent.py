@@ -426,6 +426,35 @@ def test_select_matches_the_general_row_update(n, k, j_nn, recompute, use_rev):
         assert np.array_equal(a, b)
 
 
+def test_select_after_a_join_without_current_distances():
+    """umapb_nnd_join's curd is optional: the reverse candidates' distances are in its workspace
+    either way."""
+    from mlx_vis_b200 import _lib
+
+    n, k = 400, 12
+    rng = np.random.default_rng(9)
+    X = torch.from_numpy(rng.integers(-3, 4, size=(n, 8)).astype(np.float32)).cuda()
+    idx = torch.from_numpy(rng.integers(0, n, size=(n, k)).astype(np.int32)).cuda()
+    dist = ((X[:, None, :] - X[idx.long()]) ** 2).sum(-1).contiguous()
+    sq = (X ** 2).sum(1).contiguous()
+    s = _lib.stream_handle()
+    d0, nnbuf, curd = (torch.empty(m, device="cuda") for m in (n, n * k * k, n * k))
+    ws = _lib.workspace(_lib.query("umapb_nnd_join_workspace", n, k, k), X.device)
+    _lib.call("umapb_nnd_dist_row0", _lib.ptr(X), _lib.ptr(sq), n, 8, 8, 0, _lib.ptr(d0), s)
+    got = []
+    for cur in (curd, None):
+        out = (torch.empty_like(idx), torch.empty_like(dist), torch.empty((n, k), dtype=torch.uint8, device="cuda"),
+               torch.zeros(1, dtype=torch.int64, device="cuda"))
+        ws.zero_()
+        _lib.call("umapb_nnd_join", _lib.ptr(X), _lib.ptr(sq), 8, 8, 0, _lib.ptr(idx), _lib.ptr(None), n, k, k, k,
+                  _lib.ptr(nnbuf), _lib.ptr(cur), _lib.ptr(None), _lib.ptr(None), _lib.ptr(ws), ws.numel(), s)
+        _lib.call("umapb_nnd_select", _lib.ptr(idx), _lib.ptr(dist), _lib.ptr(None), _lib.ptr(nnbuf), _lib.ptr(None),
+                  _lib.ptr(d0), n, k, k, 0, _lib.ptr(ws), ws.numel(), *(_lib.ptr(t) for t in out), s)
+        got.append([t.cpu().numpy() for t in out])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("n,k,padded", [(1500, 12, False), (4000, 12, True)])
 @pytest.mark.parametrize("d", [5, 50, 102])
 def test_rows_that_are_not_whole_float4s(d, n, k, padded):
