@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(256) head_backward_kernel(
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       pb[u] += dz[u];
-      tile[rr][lane * 4 + u] = dz[u];
+      if (dZT) tile[rr][lane * 4 + u] = dz[u];
     }
   }
 #pragma unroll
