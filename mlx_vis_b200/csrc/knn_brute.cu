@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(Cfg<NL, PAIR>::kThreads, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int col = col0 + j;
-            const float x = (col != self_col && col < n) ? v[j] : INFINITY;
+            const float x = (col != self_col && col < n) ? fminf(v[j], INFINITY) : INFINITY;  // NaN: not valid
 #pragma unroll
             for (int d = D - 1; d > 0; --d) a[d] = fminf(a[d], fmaxf(a[d - 1], x));
             a[0] = fminf(a[0], x);

@@ -100,6 +100,25 @@ def test_brute_list_edges(n, k, pair, monkeypatch):
     assert_exact_knn(X, idx, d2, k, squared=True)
 
 
+@pytest.mark.parametrize("pair", ["1", "0"])
+@pytest.mark.parametrize("n,k", [(900, 10), (900, 110), (250, 15), (250, 45), (250, 80), (250, 100)])
+@pytest.mark.parametrize("bad", [np.nan, 1e25])
+def test_brute_beside_rows_without_scores(bad, n, k, pair, monkeypatch):
+    """Half of the rows are NaN or overflow in their squared norm: nobody's neighbours, and the other
+    rows' results equal the exact search among themselves, one list of candidates or several, also where one
+    tile holds most neighbours (its admission cap counts scores)."""
+    monkeypatch.setenv("UMAPB_KNN_PAIR", pair)
+    rng = np.random.default_rng(n + k)
+    X = rng.normal(size=(n, 20)).astype(np.float32)
+    good = rng.permutation(n) >= n // 2
+    X[~good] *= np.float32(bad)
+    idx, dist = run_knn(X, k)
+    new_id = np.full(n, -1)
+    new_id[good] = np.arange(int(good.sum()))
+    assert good[idx[good]].all()
+    assert_exact_knn(X[good], new_id[idx[good]], dist[good], k)
+
+
 @pytest.mark.parametrize("d", [33, 36, 50, 62, 66, 130, 132, 194, 390])
 def test_brute_rerank_loads_and_alignment(d):
     """The rerank's load widths and lanes per candidate: row lengths that are multiples of
