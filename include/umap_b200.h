@@ -322,7 +322,7 @@ int umapb_spectral_fallback(const void* workspace, float* Y, int64_t n, int32_t 
  * umapb_layout_epoch_injected: one epoch whose negative tails are given in the
  *   reference's order (sample j pairs head ef[j % A] with neg_to[j], A = number
  *   of active edges, umap.py:433-436); neg_count must equal neg_rate * A.
- * Y (n, dim) float32 is updated in place; dim in {1, 2, 3, 4}.
+ * Y (n, dim) float32 is updated in place; 1 <= dim <= 32.
  * ------------------------------------------------------------------------- */
 int umapb_layout_workspace(int64_t n, int32_t dim, int64_t e_cap, size_t* bytes);
 int umapb_layout_prepare(const float* vals, const int64_t* n_edges, int64_t e_cap, int32_t n_epochs, float* eps,
