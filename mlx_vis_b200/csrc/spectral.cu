@@ -1028,10 +1028,17 @@ extern "C" int umapb_spectral(const int32_t* rows, const int32_t* cols, const fl
     // longer) and for every 2,048 edges, which an SM gathers in about a microsecond: by rows alone a
     // few SMs had all edges of a wide neighbourhood.  100 iterations, 2 components, by
     // rows alone and now: 5,121 rows, k = 50 1007 -> 744 us, k = 100 2610 -> 1084; 20,000 rows, k = 50
-    // 1039 -> 853; 10,000 rows, k = 15 554 -> 503; 4 components, 10,000 rows, k = 10 898 -> 760.
+    // 1039 -> 853; 10,000 rows, k = 15 554 -> 503; 4 components, 10,000 rows, k = 10 898 -> 760.  The last
+    // third of the SMs is for 4,096 edges a block: 20,000 rows, k = 15, 3 components 638 us at 81 blocks,
+    // 628 at 98, 663 at 147; k = 30 841, 806 at 147.
     const int64_t min_rows = spectral::kPowerRowThreads / spectral::kLanes / (kk > 4 ? 4 : 2);
     int64_t grid = ceil_div(n, min_rows);
-    if (ceil_div(e_cap, 2048) > grid) grid = ceil_div(e_cap, 2048);
+    int64_t by_edges = ceil_div(e_cap, 2048);
+    if (by_edges > num_sms() * 2 / 3) {
+      by_edges = num_sms() * 2 / 3;
+      if (ceil_div(e_cap, 4096) > by_edges) by_edges = ceil_div(e_cap, 4096);
+    }
+    if (by_edges > grid) grid = by_edges;
     if (grid > ceil_div(n, 16)) grid = ceil_div(n, 16);  // a warp's rows at least
     if (grid > num_sms()) grid = num_sms();
     int per = (int)ceil_div(n, grid);
