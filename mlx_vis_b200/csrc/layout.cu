@@ -55,7 +55,7 @@ constexpr int kEpochBlocksPerSM = UMAPB_LAYOUT_BLOCKS_PER_SM;
 #endif
 // the same for the kernel specialised to 5 negatives per edge (the default rate)
 constexpr int kEpochBlocksPerSM5 = UMAPB_LAYOUT_BLOCKS_PER_SM5;
-constexpr int kPre = 8;  // epoch kernel: chunks of 32 edges whose schedule words load together
+constexpr int kPreMin = 5, kPreMax = 8;  // epoch kernel: chunks of 32 edges whose schedule words load together
 
 // ---- reference pair math (float32, evaluation order of umap.py:361-383) ----
 struct Params {
@@ -245,7 +245,7 @@ __device__ __forceinline__ void edge_update(const float* Y, float* __restrict__ 
   atomic_add_row<DIM>(dY, i, acc);
 }
 
-template <int DIM, int NEG>
+template <int DIM, int NEG, int kPre>
 __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpochBlocksPerSM) sgd_epoch_kernel(const float* Y, float* __restrict__ dY, int n,
                                                            const int32_t* __restrict__ rows,
                                                            const int32_t* __restrict__ cols,
@@ -268,9 +268,7 @@ __global__ void __launch_bounds__(kBlock, NEG == 5 ? kEpochBlocksPerSM5 : kEpoch
   const int64_t e0 = b0 + (int64_t)warp * seg;
   const int64_t e1 = e0 + seg < E ? e0 + seg : E;
   const unsigned below = (1u << lane) - 1u;
-  // The same for every warp of the grid.  (Passes of equal length, so that the last one is not short,
-  // put a branch in front of every chunk: 70,000 points, k = 100 43.3 -> 45.9 us an epoch, 200,000, k =
-  // 15 47.7 -> 48.8, 1,000,000 229 -> 233; at best, 85,000 in three components, 40.6 -> 40.1.)
+  // the same for every warp of the grid
   const int passes = (int)((seg + 32 * kPre - 1) / (32 * kPre));
   for (int ps = 0; ps < passes; ++ps) {
     if (threadIdx.x == 0) s_cnt = 0;
@@ -849,6 +847,27 @@ static void launch_overlapping(void (*kernel)(P...), unsigned grid, bool overlap
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // an error is seen by the launch check
 }
 
+// Chunks in a pass of the epoch kernel, so that a warp's segment is cut into passes of equal length: a
+// short last pass leaves most of a block's batches out.  The length is compiled in: a branch in front
+// of every chunk cost more than it gave.  B200, per epoch, passes of 8 chunks / equal ones by a
+// branch / by the kernel: 70,000 points, k = 15 (7 chunks a warp) 20.0 / 20.0 / 19.2 us, 85,000, 3
+// components (9) 40.6 / 40.1 / 39.3, 170,000, 1 component (17) 39.9 / 39.4 / 38.1, 40,000, k = 100 (27)
+// 26.7 / 27.2 / 25.1; 1,000,000 (99) 229.4 / 233.2 / 229.5.
+static int pass_chunks(int64_t e_cap, unsigned grid) {
+  const int64_t chunks = ceil_div(ceil_div(e_cap > 0 ? e_cap : 1, 32), (int64_t)grid * (kBlock / 32));
+  const int64_t passes = ceil_div(chunks, kPreMax);
+  const int64_t c = ceil_div(chunks, passes);
+  return (int)(c < kPreMin ? kPreMin : c);
+}
+
+template <int DIM, int NEG>
+static auto epoch_kernel(int chunks) -> decltype(&sgd_epoch_kernel<DIM, NEG, kPreMax>) {
+  return chunks == 5   ? sgd_epoch_kernel<DIM, NEG, 5>
+         : chunks == 6 ? sgd_epoch_kernel<DIM, NEG, 6>
+         : chunks == 7 ? sgd_epoch_kernel<DIM, NEG, 7>
+                       : sgd_epoch_kernel<DIM, NEG, 8>;
+}
+
 // first: the grid before is not an epoch's apply
 template <int DIM>
 static void launch_epoch(const Layout& l, float* Y, int64_t n, const int32_t* rows, const int32_t* cols,
@@ -856,7 +875,8 @@ static void launch_epoch(const Layout& l, float* Y, int64_t n, const int32_t* ro
                          const Params& p, int neg_rate, uint64_t seed, bool neg5, bool first, cudaStream_t stream) {
   const bool five = neg_rate == 5 && neg5;
   const unsigned grid = epoch_grid(e_cap, five ? kEpochBlocksPerSM5 : kEpochBlocksPerSM);
-  launch_overlapping(five ? sgd_epoch_kernel<DIM, 5> : sgd_epoch_kernel<DIM, 0>, grid, !first, stream, Y, l.dY, n,
+  const int chunks = pass_chunks(e_cap, grid);
+  launch_overlapping(five ? epoch_kernel<DIM, 5>(chunks) : epoch_kernel<DIM, 0>(chunks), grid, !first, stream, Y, l.dY, n,
                      rows, cols, eps, next, n_edges, epoch, p, neg_rate, (uint32_t)seed, (uint32_t)(seed >> 32));
   const int64_t m = n * DIM;
   const unsigned gb = (unsigned)(ceil_div(m, 4 * kBlock) < num_sms() * 8 ? ceil_div(m, 4 * kBlock) : num_sms() * 8);

@@ -325,7 +325,7 @@ def test_fuzzy_lanes_match_float64(n, k):
 @pytest.mark.parametrize("n,k,dim,neg", [(2, 1, 2, 5), (17, 3, 1, 5), (513, 7, 2, 5), (700, 9, 3, 5), (300, 5, 4, 2),
                                          (2000, 15, 2, 0), (1025, 11, 2, 11), (1228, 10, 2, 5), (1229, 10, 2, 5), (4000, 9, 1, 5),
                                          (20, 1600, 2, 5), (3000, 20, 4, 3), (20000, 15, 2, 5), (13001, 15, 3, 5),
-                                         (30001, 5, 2, 5), (18501, 21, 3, 10), (56001, 3, 1, 0), (70003, 15, 2, 5), (70003, 24, 2, 5)])
+                                         (30001, 5, 2, 5), (18501, 21, 3, 10), (56001, 3, 1, 0), (70003, 15, 2, 5), (70003, 24, 2, 5), (80003, 15, 3, 5), (70003, 15, 2, 3)])
 @pytest.mark.parametrize("graph", [False, True])
 def test_layout_many_epochs_match_single_epochs(n, k, dim, neg, graph):
     """Epochs 3 to 12 in one call (one launch up to 12,288 edges on a cluster, beyond on a resident
